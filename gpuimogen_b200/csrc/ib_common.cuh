@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/imogen_b200.h"
+#include "ib_fast.cuh"
 
 namespace ib {
 
@@ -40,6 +41,7 @@ template <typename FT>
 struct FluidConsts {
     FT gamma, gm1, govergm1;
     FT isotemp, isotempsq;
+    FT hgm1, rgm1;            // (gamma - 1) / 2 and 1 / (gamma - 1), product build
     double minmass, mintemp;  // floors stay FP64
 };
 
@@ -52,6 +54,8 @@ inline FluidConsts<FT> make_consts(double gamma, double rho_min, double c_iso)
     c.govergm1 = (FT)(gamma / (gamma - 1.0));
     c.isotemp = (FT)c_iso;
     c.isotempsq = (FT)(c_iso * c_iso);
+    c.hgm1 = (FT)(.5 * (gamma - 1.0));
+    c.rgm1 = (FT)(1.0 / (gamma - 1.0));
     c.minmass = rho_min;
     c.mintemp = 1e-5 / (gamma - 1);  // cudaFluidStep.cu:298
     return c;
@@ -68,39 +72,57 @@ __device__ __forceinline__ FT flux_minmod(FT A, FT B)
     return A;
 }
 
+__device__ __forceinline__ bool signs_differ(double a, double b)
+{
+    return (__double2hiint(a) ^ __double2hiint(b)) < 0;
+}
+__device__ __forceinline__ bool signs_differ(float a, float b)
+{
+    return (__float_as_int(a) ^ __float_as_int(b)) < 0;
+}
+
 template <int SLOPE, typename FT>
 __device__ __forceinline__ FT slope_limit(FT A, FT B)
 {
     if constexpr (SLOPE == IB_SLOPE_OSPRE) {  // limiter_functions.h:87-95
         FT R = A * B;
+#ifdef IB_STRICT_ARITH
         if (R > 0) {
             FT S = A + B;
             return (FT).75 * R * S / (S * S - R);
         }
         return (FT)0.0;
+#else
+        const FT S = A + B;  // the denominator is A^2 + A B + B^2 > 0 where R > 0
+        const FT s = (FT).75 * R * S * rcp_fast_pos(S * S - R);
+        return (R > 0) ? s : (FT)0;
+#endif
     } else if constexpr (SLOPE == IB_SLOPE_MC) {  // limiter_functions.h:105-115
-        if (A * B <= 0) return (FT)0;
 #ifdef IB_STRICT_ARITH
+        if (A * B <= 0) return (FT)0;
         FT R = B / A;
         FT S = (FT).25 + (FT).25 * R;
         S = (S < R) ? S : R;
         S = (S < 1) ? S : (FT)1.0;
         return S * A;
 #else
-        // min(.25(1+R), R, 1) * A with R = B/A, without the division: for A and B of one sign
-        // it is the smaller in magnitude of .25(A+B), B and A
-        FT S = (FT).25 * (A + B);
-        if (A > 0) {
-            S = (S < B) ? S : B;
-            return (S < A) ? S : A;
-        }
-        S = (S > B) ? S : B;
-        return (S > A) ? S : A;
+        // min(.25(1+R), R, 1) * A with R = B/A, without the division: for A and B of one sign it is
+        // the smallest in magnitude of .25(A+B), B and A (of opposite sign: 0; by their sign bits,
+        // so that slopes below 1e-162, whose product underflows to zero, are limited like any other)
+        const FT S = (FT).25 * (A + B);
+        const FT m = (fabs(A) < fabs(B)) ? A : B;
+        const FT r = (fabs(m) <= fabs(S)) ? m : S;
+        return signs_differ(A, B) ? (FT)0 : r;
 #endif
     } else if constexpr (SLOPE == IB_SLOPE_VANLEER) {  // limiter_functions.h:54-61
         FT r = A * B;
+#ifdef IB_STRICT_ARITH
         if (r > (FT)0.0) return r / (A + B);
         return (FT)0;
+#else
+        const FT s = r * rcp_fast(A + B);
+        return (r > (FT)0.0) ? s : (FT)0;
+#endif
     } else if constexpr (SLOPE == IB_SLOPE_MINMOD) {  // limiter_functions.h:71-77
         // the FP64 reference returns this limiter through a float
         if (A * B < 0) return (FT)0.0;
@@ -149,24 +171,14 @@ __device__ __forceinline__ float dsqrt<float>(float x) { return sqrtf(x); }
 // ------------------------------------------------------------------------------------------
 // Einfeldt wave-speed bounds (cudaFluidStep.cu:1728-1755, isothermal 1780-1799)
 // ------------------------------------------------------------------------------------------
-// irL, irR: 1/rhoL and 1/rhoR as the product build forms them (the HLLC star flux reuses them)
-template <typename FT>
-__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR,
-                                         FT vR, FT PR, FT dvsq, FT &sl, FT &sr, FT &irL, FT &irR)
-{
 #ifdef IB_STRICT_ARITH
+template <typename FT>
+__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR, FT vR, FT PR,
+                                         FT dvsq, FT &sl, FT &sr)
+{
     FT csql = c.gamma * PL / rhoL;
     FT csqr = c.gamma * PR / rhoR;
     FT Fa = dsqrt<FT>(rhoR / rhoL);
-    irL = (FT)1.0 / rhoL;  // unused by the strict star flux, which divides as the reference does
-    irR = (FT)1.0 / rhoR;
-#else
-    irL = (FT)1.0 / rhoL;
-    irR = (FT)1.0 / rhoR;
-    FT csql = c.gamma * PL * irL;
-    FT csqr = c.gamma * PR * irR;
-    FT Fa = dsqrt<FT>(rhoR * irL);
-#endif
     FT Fb = (FT)1.0 / ((FT)1.0 + Fa);
     FT Croe = ((csql + Fa * csqr) + (FT).5 * c.gm1 * dvsq * Fa * Fb) * Fb;
     FT Vroe = (vL + Fa * vR) * Fb;
@@ -177,20 +189,47 @@ __device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT v
     Croe = 2 * Vroe - Croe;
     sr = (Croe > sr) ? Croe : sr;
 }
+#else
+// with the Roe weights wl = 1 / (1 + Fa) and wr = Fa wl, Fa = sqrt(rhoR / rhoL); irL, irR: the density
+// reciprocals, which the HLLC star flux takes over
+template <typename FT>
+__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR, FT vR, FT PR,
+                                         FT dvsq, FT &sl, FT &sr, FT &irL, FT &irR)
+{
+    irL = rcp_fast(rhoL);
+    irR = rcp_fast(rhoR);
+    const FT csql = c.gamma * PL * irL, csqr = c.gamma * PR * irR;
+    const FT Fa = sqrt_fast(rhoR * irL);
+    const FT wl = rcp_fast((FT)1.0 + Fa);
+    const FT wr = Fa * wl;
+    const FT vroe = wl * vL + wr * vR;
+    const FT croe = sqrt_fast(wl * csql + wr * csqr + c.hgm1 * dvsq * (wl * wr));
+    sl = vL - sqrt_fast(csql);
+    sr = vR + sqrt_fast(csqr);
+    const FT s1 = vroe - croe, s2 = vroe + croe;
+    sl = (s1 < sl) ? s1 : sl;
+    sr = (s2 > sr) ? s2 : sr;
+}
 
 template <typename FT>
-__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR,
-                                         FT vR, FT PR, FT dvsq, FT &sl, FT &sr)
+__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR, FT vR, FT PR,
+                                         FT dvsq, FT &sl, FT &sr)
 {
     FT irL, irR;
     einfeldt<FT>(c, rhoL, vL, PL, rhoR, vR, PR, dvsq, sl, sr, irL, irR);
 }
+#endif
 
 template <typename FT>
 __device__ __forceinline__ void einfeldt_iso(FT rhoL, FT vL, FT rhoR, FT vR, FT cs, FT &sl, FT &sr)
 {
+#ifdef IB_STRICT_ARITH
     FT Fa = dsqrt<FT>(rhoR / rhoL);
     FT Fb = (FT)1.0 / ((FT)1.0 + Fa);
+#else
+    FT Fa = sqrt_fast(rhoR * rcp_fast(rhoL));
+    FT Fb = rcp_fast((FT)1.0 + Fa);
+#endif
     FT Vroe = (vL + Fa * vR) * Fb;
     cs = Vroe - cs;
     sl = vL - cs;
@@ -211,7 +250,11 @@ struct V5 {
 template <typename FT>
 __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 {
+#ifdef IB_STRICT_ARITH
     FT F = (FT)1.0 / A;
+#else
+    FT F = rcp_fast(A);
+#endif
     B -= (FT).5 * (C * C + D * D + E * E) * F;
     C *= F;
     D *= F;
@@ -242,6 +285,7 @@ __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT
 
 // HLLC flux through the face between the right face state of the left cell (l) and the left
 // face state of the right cell (r).  (cudaFluidStep.cu:1318-1432)
+#ifdef IB_STRICT_ARITH
 template <typename FT>
 __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
@@ -252,8 +296,8 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     D = vyL - vyR;
     E = vzL - vzR;
     C = C * C + D * D + E * E;
-    FT sl, sr, irL, irR;
-    einfeldt<FT>(c, rhoL, vxL, PL, rhoR, vxR, PR, C, sl, sr, irL, irR);
+    FT sl, sr;
+    einfeldt<FT>(c, rhoL, vxL, PL, rhoR, vxR, PR, C, sl, sr);
     C = sl;
     D = sr;
     A = rhoL * (C - vxL);
@@ -282,11 +326,7 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
             H *= A;
             C *= (E - B);
             B = PL + D * (C + E * B);
-#ifdef IB_STRICT_ARITH
             G = D * E * (c.govergm1 * PL / rhoL + G + C);
-#else
-            G = D * E * (c.govergm1 * PL * irL + G + C);
-#endif
             f.a[0] = A; f.a[1] = G; f.a[2] = B; f.a[3] = F; f.a[4] = H;
         }
     } else {
@@ -300,11 +340,7 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
             H *= A;
             D *= (E - B);
             B = PR + C * (D + E * B);
-#ifdef IB_STRICT_ARITH
             G = C * E * (c.govergm1 * PR / rhoR + G + D);
-#else
-            G = C * E * (c.govergm1 * PR * irR + G + D);
-#endif
             f.a[0] = A; f.a[1] = G; f.a[2] = B; f.a[3] = F; f.a[4] = H;
         } else {  // right state
             A = rhoR; B = vxR; C = vyR; D = vzR;
@@ -320,6 +356,47 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     }
     return f;
 }
+#else
+// The same flux with fewer and shorter dependent chains: reciprocals and roots of ib_fast.cuh, and the
+// star (or outer) state computed once, for the side that the contact speed selects, instead of in
+// divergent branches.
+template <typename FT>
+__device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
+{
+    const FT rhoL = l.a[0], PL = l.a[1], vL = l.a[2];
+    const FT rhoR = r.a[0], PR = r.a[1], vR = r.a[2];
+    const FT dn = vL - vR, d1 = l.a[3] - r.a[3], d2 = l.a[4] - r.a[4];
+    FT sl, sr, irL, irR;
+    einfeldt<FT>(c, rhoL, vL, PL, rhoR, vR, PR, dn * dn + d1 * d1 + d2 * d2, sl, sr, irL, irR);
+    const FT A = rhoL * (sl - vL), B = rhoR * (sr - vR);
+    const FT sm = (B * vR - PR - A * vL + PL) * rcp_fast(B - A);  // Batten et al. eq. 34
+    const bool left = sm > 0;
+    const FT rho = left ? rhoL : rhoR, P = left ? PL : PR, v = left ? vL : vR;
+    const FT t1 = left ? l.a[3] : r.a[3], t2 = left ? l.a[4] : r.a[4];
+    const FT ke = (FT).5 * (v * v + t1 * t1 + t2 * t2);
+    const FT h = c.govergm1 * P;
+    V5<FT> f;
+    if (left ? sl > 0 : !(sr > 0)) {  // the outer state: no wave crosses the face
+        const FT m = rho * v;
+        f.a[0] = m;
+        f.a[1] = v * (ke * rho + h);
+        f.a[2] = m * v + P;
+        f.a[3] = m * t1;
+        f.a[4] = m * t2;
+    } else {
+        const FT S = left ? sl : sr;
+        const FT D = (left ? A : B) * rcp_fast(S - sm);
+        const FT m = D * sm;
+        const FT q = S * (sm - v);
+        f.a[0] = m;
+        f.a[1] = m * (h * (left ? irL : irR) + ke + q);
+        f.a[2] = P + D * (q + sm * v);
+        f.a[3] = m * t1;
+        f.a[4] = m * t2;
+    }
+    return f;
+}
+#endif
 
 // Slab offsets (in slabs) of the local components [rho, E, p_n, p_t1, p_t2] for a sweep along
 // direction dir; HLLC (cudaFluidStep.cu:1200-1219) and HLL (1864-1882) differ for z.

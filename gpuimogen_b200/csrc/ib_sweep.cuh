@@ -38,16 +38,23 @@ __device__ __forceinline__ V5<FT> v5_sub(const V5<FT> &a, const V5<FT> &b)
 }
 
 // HLL primitives: [rho, v_n, P, v_t1, v_t2] with P taken from the floored pressure
-// (cudaFluidStep.cu:1864-1888)
+// (cudaFluidStep.cu:1864-1888).  irho: 1 / rho, product build (one reciprocal for the five quotients of
+// the pressure solver and the velocities; the strict build divides as the reference does)
 template <typename FT>
-__device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2)
+__device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2, FT irho)
 {
     V5<FT> w;
     w.a[0] = rho;
-    w.a[1] = pn / rho;
     w.a[2] = P;
+#ifdef IB_STRICT_ARITH
+    w.a[1] = pn / rho;
     w.a[3] = pt1 / rho;
     w.a[4] = pt2 / rho;
+#else
+    w.a[1] = pn * irho;
+    w.a[3] = pt1 * irho;
+    w.a[4] = pt2 * irho;
+#endif
     return w;
 }
 
@@ -81,7 +88,11 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
     }
     Sleft = sl;
     Sright = sr;
+#ifdef IB_STRICT_ARITH
     FT Atilde = 1 / (Sright - Sleft);
+#else
+    FT Atilde = rcp_fast(Sright - Sleft);
+#endif
     FT Fa = Ale * Ble;
     FT Fb = Are * Bre;
     V5<FT> f;
@@ -113,7 +124,12 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
             Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele);
             Fb = (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere);
             FT e = (Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb);
-            f.a[1] = (e + (c.govergm1 * (Sright * Cle * Ble - Sleft * Cre * Bre) + Sleft * Sright * (Cre - Cle) / c.gm1)) * Atilde;
+#ifdef IB_STRICT_ARITH
+            const FT dp = Sleft * Sright * (Cre - Cle) / c.gm1;
+#else
+            const FT dp = Sleft * Sright * (Cre - Cle) * c.rgm1;
+#endif
+            f.a[1] = (e + (c.govergm1 * (Sright * Cle * Ble - Sleft * Cre * Bre) + dp)) * Atilde;
         } else {
             // isothermal energy flux lacks the 1/(S_R-S_L) factor (cudaFluidStep.cu:2178-2182)
             Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele) + Cle;
@@ -137,9 +153,9 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
 
 // HLL pressure solver with floors (cukern_PressureSolverHydro, cudaFluidStep.cu:2813-2864) on a
 // conserved state in local order u = [rho, E, p_n, p_t1, p_t2]; mom[m] = local index of memory
-// slab 2+m (the reference sums px, py, pz in slab order).  Returns P, modifies u.
+// slab 2+m (the reference sums px, py, pz in slab order).  Returns P and 1 / rho, modifies u.
 template <int DIR>
-__device__ __forceinline__ double hll_pressure(double u[5], double minmass, double mintemp, double gm1)
+__device__ __forceinline__ double hll_pressure(double u[5], double minmass, double mintemp, double gm1, double &irho)
 {
     // local index of memory slabs 2,3,4 under HllSlots<DIR>
     constexpr int m2 = (HllSlots<DIR>::n == 2) ? 2 : ((HllSlots<DIR>::t1 == 2) ? 3 : 4);
@@ -165,11 +181,22 @@ __device__ __forceinline__ double hll_pressure(double u[5], double minmass, doub
         z = u[m4];
         momsq += z * z;
     }
+#ifdef IB_STRICT_ARITH
+    irho = 0.0;
     P = E - .5 * momsq / rho;
     if (P < rho * mintemp) {
         P = mintemp * rho;
         u[1] = (.5 * momsq / rho) + P;
     }
+#else
+    irho = rcp_fast(rho);
+    const double ke = .5 * momsq * irho;
+    P = E - ke;
+    if (P < rho * mintemp) {
+        P = mintemp * rho;
+        u[1] = ke + P;
+    }
+#endif
     return P * gm1;
 }
 
@@ -192,8 +219,9 @@ __device__ __forceinline__ V5<FT> stage_prims(double u[5], const FluidConsts<FT>
     if constexpr (METHOD == IB_METHOD_HLLC) {
         return hllc_prims<FT>((FT)u[0], (FT)u[1], (FT)u[2], (FT)u[3], (FT)u[4]);
     } else {
-        double P = hll_pressure<DIR>(u, c.minmass, c.mintemp, (double)c.gm1);
-        return hll_prims<FT>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4]);
+        double irho;
+        double P = hll_pressure<DIR>(u, c.minmass, c.mintemp, (double)c.gm1, irho);
+        return hll_prims<FT>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4], (FT)irho);
     }
 }
 
