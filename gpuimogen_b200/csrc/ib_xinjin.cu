@@ -12,20 +12,36 @@
 
 namespace ib {
 
-// Maximum over the pencil of column `col` (W interleaved pencils per block), ignoring NaN
-// candidates as the reference's `(a > b) ? a : b` tree does.
+// Maximum of non-negative doubles over a warp: their bit patterns order as unsigned integers, so the
+// maximum of the high words, then of the low words that go with it (two warp reductions instead of
+// five rounds of two shuffles, a comparison and a select).
+__device__ __forceinline__ double warp_max_pos(double v)
+{
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+
+// Maximum over the pencil of column `col` (W interleaved pencils per block) of v >= 0, which the
+// caller has taken so that NaN never wins, as in the reference's `(a > b) ? a : b` tree.
 template <int W>
 __device__ __forceinline__ double block_max_keep(double v, double *red, int col)
 {
-#pragma unroll
-    for (int o = 16; o >= W; o >>= 1) {
-        double w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = (w > v) ? w : v;
-    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    if constexpr (W == 1) {
+        v = warp_max_pos(v);
+    } else {
+#pragma unroll
+        for (int o = 16; o >= W; o >>= 1) {
+            double w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = (w > v) ? w : v;
+        }
+    }
     __syncthreads();
     if (lane < W) red[wid * W + lane] = v;
     __syncthreads();
+    if constexpr (W == 1) return warp_max_pos(lane < nw ? red[lane] : 0.0);
     double m = 0.0;
     for (int w = 0; w < nw; w++) m = (red[w * W + col] > m) ? red[w * W + col] : m;
     return m;
@@ -41,51 +57,34 @@ __device__ __forceinline__ double freeze_cell(const double (&X)[5], double invrh
     px = X[2];
     psq += px * px;
     double P = (X[1] - .5 * psq * invrho) * gm1;
+#ifdef IB_STRICT_ARITH
     return fabs(px) * invrho + sqrt(gamma * P * invrho);
+#else
+    return fabs(px) * invrho + sqrt_fast(gamma * P * invrho);
+#endif
 }
 
 // The left- and right-going limited fluxes of one component, flux_limit<FLIM>(A1, B1) and
-// flux_limit<FLIM>(A2, B2).  Product build, Ospre and van Leer: their two divisions share one
-// (1/(d1 d2) times d2 and d1) when d1, d2 and d1 d2 are all normal numbers, so that neither
-// reciprocal can overflow; otherwise (subnormal denominators of momenta near 1e-154, where a
-// reciprocal of infinity times an underflowed zero numerator would give NaN) each divides on
-// its own, as the strict build always does.
+// flux_limit<FLIM>(A2, B2).  Product build, Ospre and van Leer: selects instead of branches and the
+// reciprocals of ib_fast.cuh.  Ospre's denominator A^2 + A B + B^2 can underflow (momenta near 1e-154):
+// its reciprocal then stays finite and the numerator is zero.  Van Leer's A + B is a normal number
+// wherever 2 A B > 0.
 template <int FLIM>
 __device__ __forceinline__ void flux_limit_pair(double A1, double B1, double A2, double B2, double &o1, double &o2)
 {
 #ifndef IB_STRICT_ARITH
-    if constexpr (FLIM == IB_FLUX_OSPRE || FLIM == IB_FLUX_VANLEER) {
-        double n1, d1, n2, d2;
-        bool p1, p2;
-        if constexpr (FLIM == IB_FLUX_OSPRE) {  // 1.5 r (A + B) / (A^2 + r + B^2), 0 where r <= 0
-            const double r1 = A1 * B1, r2 = A2 * B2;
-            p1 = !(r1 <= 0.0);
-            p2 = !(r2 <= 0.0);
-            n1 = 1.5 * r1 * (A1 + B1);
-            d1 = A1 * A1 + r1 + B1 * B1;
-            n2 = 1.5 * r2 * (A2 + B2);
-            d2 = A2 * A2 + r2 + B2 * B2;
-        } else {  // 2AB / (A + B) where 2AB > 0
-            const double r1 = 2.0 * A1 * B1, r2 = 2.0 * A2 * B2;
-            p1 = r1 > 0.0;
-            p2 = r2 > 0.0;
-            n1 = r1;
-            d1 = A1 + B1;
-            n2 = r2;
-            d2 = A2 + B2;
-        }
-        d1 = p1 ? d1 : 1.0;
-        d2 = p2 ? d2 : 1.0;
-        const double pd = d1 * d2;
-        constexpr double kMinNormal = 2.2250738585072014e-308, kMax = 1.7976931348623157e308;
-        if (fabs(d1) >= kMinNormal && fabs(d2) >= kMinNormal && fabs(pd) >= kMinNormal && fabs(pd) <= kMax) {
-            const double rr = 1.0 / pd;
-            o1 = p1 ? n1 * (d2 * rr) : 0.0;
-            o2 = p2 ? n2 * (d1 * rr) : 0.0;
-        } else {
-            o1 = p1 ? n1 / d1 : 0.0;
-            o2 = p2 ? n2 / d2 : 0.0;
-        }
+    if constexpr (FLIM == IB_FLUX_OSPRE) {  // 1.5 r (A + B) / (A^2 + r + B^2), 0 where r <= 0
+        const double r1 = A1 * B1, r2 = A2 * B2;
+        const double l1 = 1.5 * r1 * (A1 + B1) * rcp_fast_pos(A1 * A1 + r1 + B1 * B1);
+        const double l2 = 1.5 * r2 * (A2 + B2) * rcp_fast_pos(A2 * A2 + r2 + B2 * B2);
+        o1 = (r1 <= 0.0) ? 0.0 : l1;
+        o2 = (r2 <= 0.0) ? 0.0 : l2;
+        return;
+    } else if constexpr (FLIM == IB_FLUX_VANLEER) {  // 2AB / (A + B) where 2AB > 0
+        const double r1 = 2.0 * A1 * B1, r2 = 2.0 * A2 * B2;
+        const double l1 = r1 * rcp_fast(A1 + B1), l2 = r2 * rcp_fast(A2 + B2);
+        o1 = (r1 > 0.0) ? l1 : 0.0;
+        o2 = (r2 > 0.0) ? l2 : 0.0;
         return;
     }
 #endif
@@ -162,7 +161,7 @@ __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab
 #ifdef IB_STRICT_ARITH
                 const double v = freeze_cell(X, 1.0 / X[0], gamma, gm1);
 #else
-                if (stage == 0) rinv[m] = 1.0 / X[0];
+                if (stage == 0) rinv[m] = rcp_fast(X[0]);
                 const double v = freeze_cell(X, rinv[m], gamma, gm1);
 #endif
                 cm = (v > cm) ? v : cm;
@@ -276,7 +275,7 @@ __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab
 #ifdef IB_STRICT_ARITH
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) / p0;
 #else
-                rinv[m] = 1.0 / p0;
+                rinv[m] = rcp_fast(p0);
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) * rinv[m];
 #endif
                 if ((p1 - w) < p0 * mintemp) p1 = w + p0 * mintemp;
@@ -366,7 +365,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #pragma unroll 1
     for (int col = 0; col < WC; col++) {
         auto TI = [&](int k) { return (k * n + i) * WC + col; };
-        double u0[5], u1[5];
+        double u0[5], u1[5], nl[5], nr[5];  // nl, nr: this cell's own relaxation fluxes
 #ifndef IB_STRICT_ARITH
         double rinv = 1.0;
 #endif
@@ -383,7 +382,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #ifdef IB_STRICT_ARITH
                 const double v = freeze_cell(X, 1.0 / X[0], a.gamma, gm1);
 #else
-                if (stage == 0) rinv = 1.0 / X[0];
+                if (stage == 0) rinv = rcp_fast(X[0]);
                 const double v = freeze_cell(X, rinv, a.gamma, gm1);
 #endif
                 cm = (v > cm) ? v : cm;
@@ -406,18 +405,17 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
                     else if (k == 1) w = Vx * (qk + Pv);
                     else if (k == nslot) w = Vx * qk + Pv;
                     else w = Vx * qk;
-                    Lb[k * NP + i] = (Cf * qk - w);
-                    Rb[k * NP + i] = (Cf * qk + w);
+                    Lb[k * NP + i] = nl[k] = (Cf * qk - w);
+                    Rb[k * NP + i] = nr[k] = (Cf * qk + w);
                 }
             }
             __syncthreads();
             if (stage == 1) {
-                double nl[5], nr[5];
                 if (act) {
 #pragma unroll
                     for (int k = 0; k < 5; k++) {
-                        const double Lm = Lb[k * NP + il], L0 = Lb[k * NP + i], Lp = Lb[k * NP + ir];
-                        const double Rm = Rb[k * NP + il], R0 = Rb[k * NP + i], Rp = Rb[k * NP + ir];
+                        const double Lm = Lb[k * NP + il], L0 = nl[k], Lp = Lb[k * NP + ir];
+                        const double Rm = Rb[k * NP + il], R0 = nr[k], Rp = Rb[k * NP + ir];
                         const double dL0 = 0.5 * (L0 - Lm), dLp = 0.5 * (Lp - L0);
                         const double dR0 = 0.5 * (R0 - Rm), dRp = 0.5 * (Rp - R0);
                         double limL, limR;
@@ -438,17 +436,17 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #pragma unroll
                 for (int k = 0; k < 5; k++) {
                     if constexpr (GEO == CYL_NONE) {
-                        pr[k] = u0[k] - lam * (Rb[k * NP + i] - Rb[k * NP + il] - Lb[k * NP + ir] + Lb[k * NP + i]);
+                        pr[k] = u0[k] - lam * (nr[k] - Rb[k * NP + il] - Lb[k * NP + ir] + nl[k]);
                     } else if constexpr (GEO == CYL_THETA_DIV) {
 #ifdef IB_STRICT_ARITH
-                        pr[k] = u0[k] - lam * (Rb[k * NP + i] - Rb[k * NP + il] - Lb[k * NP + ir] + Lb[k * NP + i]) / rpen;
+                        pr[k] = u0[k] - lam * (nr[k] - Rb[k * NP + il] - Lb[k * NP + ir] + nl[k]) / rpen;
 #else
-                        pr[k] = u0[k] - lam * (Rb[k * NP + i] - Rb[k * NP + il] - Lb[k * NP + ir] + Lb[k * NP + i]) *
+                        pr[k] = u0[k] - lam * (nr[k] - Rb[k * NP + il] - Lb[k * NP + ir] + nl[k]) *
                                             (1.0 / rpen);
 #endif
                     } else {
                         const double lr = lam / rpen;
-                        pr[k] = u0[k] - lr * (Rb[k * NP + i] - Rb[k * NP + il] - Lb[k * NP + ir] + Lb[k * NP + i]);
+                        pr[k] = u0[k] - lr * (nr[k] - Rb[k * NP + il] - Lb[k * NP + ir] + nl[k]);
                     }
                 }
                 double p0 = pr[0], p1 = pr[1];
@@ -457,7 +455,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #ifdef IB_STRICT_ARITH
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) / p0;
 #else
-                rinv = 1.0 / p0;
+                rinv = rcp_fast(p0);
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) * rinv;
 #endif
                 if ((p1 - w) < p0 * a.mintemp) p1 = w + p0 * a.mintemp;
