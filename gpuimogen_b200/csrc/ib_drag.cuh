@@ -36,8 +36,14 @@ __device__ __forceinline__ double pow_of(const PowBase &b, double y)
 // allregimeCdrag (cudaSource2FluidDrag.cu:819-833)
 __device__ __forceinline__ double allregime_cdrag(double Re, double Kn)
 {
+#ifdef IB_STRICT_ARITH
     double cunningham = 1 + Kn * (1.142 + 1 * 0.558 * exp(-0.999 / Kn));
     double C_drag = (3 / Re + .45 * pow_of(pow_base(Re), -.319) + .0509 * Re / (8710 + Re)) / cunningham;
+#else  // the reciprocals of ib_fast.cuh (Kn is zero in gas without internal energy)
+    double cunningham = 1 + Kn * (1.142 + 1 * 0.558 * exp(-0.999 * rcp_fast_pos(Kn)));
+    double C_drag = (3 * rcp_fast_pos(Re) + .45 * pow_of(pow_base(Re), -.319) + .0509 * Re * rcp_fast(8710 + Re)) *
+                    rcp_fast(cunningham);
+#endif
     return C_drag;
 }
 
@@ -49,7 +55,11 @@ __device__ __forceinline__ double drag_k(const DragParams &d, double rhoA, doubl
     double Tn = d.alpha * u;
     const PowBase bT = pow_base(Tn);
     double Re = d.delta * rhoA * magdv * pow_of(bT, d.viscpow);
+#ifdef IB_STRICT_ARITH
     double Kn = d.beta * pow_of(bT, d.lampow) / rhoA;
+#else
+    double Kn = d.beta * pow_of(bT, d.lampow) * rcp_fast(rhoA);
+#endif
     double Cd_hat = allregime_cdrag(Re, Kn);
     return Cd_hat * magdv * (rhoA + rhoB) * d.epsilon;
 }
@@ -62,7 +72,11 @@ __device__ __forceinline__ double logtrap_keff(const DragParams &d, double g0, d
 {
     double mu, k, dv_i, dv_t, dvsq, duint, t2;
     bool skip;
+#ifdef IB_STRICT_ARITH
     mu = d0 / (g0 + d0);
+#else
+    mu = d0 * rcp_fast(g0 + d0);
+#endif
     k = drag_k(d, g0, d0, t0, t1, skip);
     t2 = skip ? 0 : k;
     k = t2;
@@ -70,7 +84,11 @@ __device__ __forceinline__ double logtrap_keff(const DragParams &d, double g0, d
     dv_t = dv_i * exp(-t * k);
     dvsq = dv_t * dv_t;
     duint = -.5 * dv_i * dv_i * mu * expm1(-2 * k * t);
+#ifdef IB_STRICT_ARITH
     t0 = sqrt(dvsq);
+#else
+    t0 = fabs(dv_t);
+#endif
     t1 += duint;
     k = drag_k(d, g0, d0, t0, t1, skip);
     if (!skip) t2 += k;
@@ -108,7 +126,7 @@ __device__ __forceinline__ void drag_features(double g0, double gE, double g2, d
     magdv = sqrt(dvsq);
     u = press / g0;
 #else  // the two density reciprocals once instead of eight divisions
-    const double ig = 1.0 / g0, id = 1.0 / d0;
+    const double ig = rcp_fast(g0), id = rcp_fast(d0);
     dv = g2 * ig - d2 * id;
     dvsq = dv * dv;
     dv = g3 * ig - d3 * id;
@@ -116,7 +134,7 @@ __device__ __forceinline__ void drag_features(double g0, double gE, double g2, d
     dv = g4 * ig - d4 * id;
     dvsq += dv * dv;
     press = (gE - .5 * (g2 * g2 + g3 * g3 + g4 * g4) * ig);
-    magdv = sqrt(dvsq);
+    magdv = sqrt_fast(dvsq);
     u = press * ig;
 #endif
 }
@@ -136,10 +154,10 @@ __device__ __forceinline__ void drag_apply(double *g, double *ds, int64_t S, dou
     auto over_sum = [&](double x) { return x / (g0 + d0); };
     auto over_d0 = [&](double x) { return x / d0; };
 #else  // three reciprocals instead of nine divisions
-    const double isum = 1.0 / (g0 + d0), rhodinv = 1.0 / d0;
+    const double isum = rcp_fast(g0 + d0), rhodinv = rcp_fast(d0);
     mu = d0 * isum;
     mu = mu * g0;
-    rhoginv = 1.0 / g0;
+    rhoginv = rcp_fast(g0);
     auto over_sum = [&](double x) { return x * isum; };
     auto over_d0 = [&](double x) { return x * rhodinv; };
 #endif
