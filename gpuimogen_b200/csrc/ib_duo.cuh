@@ -1,0 +1,257 @@
+// ib_duo.cuh -- sweep kernels with two neighbouring cells a thread: x rows of up to 1024 cells, and y/z
+// pencils of up to 512 cells that TMA cannot fetch (odd nx, unaligned arrays).
+//
+// A thread owns the cells a = 2t and b = 2t + 1 and a CTA whole pencils, so that both SSPRK stages run on
+// chip (ib_sweep.cuh).  What bounds such a sweep, once its divisions and square roots are the short ones of
+// ib_fast.cuh, is the traffic between threads through shared memory: with one cell a thread the data pipe was
+// 70 % busy in the 256^3 x sweep.  Two cells a thread exchange only b's primitives with the thread after and
+// a's with the one before, one face and one flux: half the bytes per cell (data pipe 50 %), no exchange at all
+// for the face between a and b, and two independent chains of FP64 arithmetic (256^3 HLLC x 0.534 -> 0.461 ms
+// at five 128-thread CTAs of 96 registers per SM; 128 registers and four CTAs 0.483, 80 and six 0.565 with
+// spills).  The y/z boxes that TMA fetches stay with the one-cell kernels: there the wait for a box weighs more
+// than the exchange, and the fewer warps of this form hide it less (256^3 y: 0.552 against 0.580 ms).
+//
+// Per stage: primitives to shared memory, barrier, limited slopes, the flux through a|b and a's left
+// face to shared memory, barrier, the flux through b's right face to shared memory, barrier, update.
+// (Forming the right neighbour's face again instead of exchanging it saves a barrier but measured slower,
+// 0.461 -> 0.492 ms: more live registers.)  Three planes of 5 x TT values rotate through the roles
+// (primitives of a, later fluxes; primitives of b; left faces) so that no stage writes a plane which the one
+// before may still be reading.
+#pragma once
+
+#include "ib_sweep.cuh"
+
+namespace ib {
+
+// A thread's place: plane slots of its own cells, of the thread before and the one after (periodic).
+// Pencils of odd length: the last thread owns only a; its b stands for the pencil's first cell.
+struct DuoPos {
+    int own, left, right;
+    bool first, ghost;  // odd lengths only: the pencil's first thread, the last one
+};
+
+struct DuoGeo {
+    double ra, rb, dr;  // radial sweeps: the radii of the two cells' centres, the cell size
+    double rpen;        // theta sweeps: the pencil's radius
+};
+
+// NS sweeps of the cells (ua, ub) of this thread, in place.  planes: 15 TT values of FT; SS: 10 TT
+// doubles, where u1 + u0 of the SSPRK average waits through the second stage.  All threads of the CTA
+// call it.
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO>
+__device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], bool act, const DuoPos &p, FT *planes,
+                                           double *SS, double lambda, const FluidConsts<FT> &c, const DuoGeo &g)
+{
+    double va[5], vb[5];
+#pragma unroll
+    for (int s = 0; s < 2 * NS; s++) {
+        const bool second = s & 1;
+        FT *P = planes + (s % 3) * 5 * TT, *Q = planes + ((s + 1) % 3) * 5 * TT, *R = planes + ((s + 2) % 3) * 5 * TT;
+        V5<FT> wa, wb;
+        if (act) {
+            wa = stage_prims<METHOD, DIR, FT>(second ? va : ua, c);  // HLL floors its argument
+            wb = stage_prims<METHOD, DIR, FT>(second ? vb : ub, c);
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                P[k * TT + p.own] = wa.a[k];
+                Q[k * TT + p.own] = wb.a[k];
+                if (second) {  // after the prims: HLL floors the stage's input
+                    SS[k * TT + p.own] = va[k] + ua[k];
+                    SS[(5 + k) * TT + p.own] = vb[k] + ub[k];
+                }
+            }
+        }
+        __syncthreads();
+        V5<FT> fm, rb;  // the flux through a|b, b's right face
+        double pa = 0.0, pb = 0.0;  // radial sweeps: the cells' face pressure sums (HLLC) or input pressures (HLL)
+        if (act) {
+            V5<FT> lb, ra;
+            if (ODD && p.ghost) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) wb.a[k] = P[k * TT + p.right];
+            }
+            if (GEO == CYL_RADIAL && METHOD == IB_METHOD_HLL) { pa = (double)wa.a[2]; pb = (double)wb.a[2]; }
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const FT wl = (ODD && p.first) ? P[k * TT + p.left] : Q[k * TT + p.left];
+                const FT wr = (ODD && p.ghost) ? Q[k * TT + p.right] : P[k * TT + p.right];
+                const FT dl = wa.a[k] - wl, dm = wb.a[k] - wa.a[k], dr = wr - wb.a[k];
+                const FT ha = slope_limit<SLOPE, FT>(dl, dm), hb = slope_limit<SLOPE, FT>(dm, dr);
+                FT la;
+                if (METHOD == IB_METHOD_HLLC && k == 1) {  // internal energy to pressure
+                    la = c.gm1 * (wa.a[k] - ha);
+                    ra.a[k] = c.gm1 * (wa.a[k] + ha);
+                    lb.a[k] = c.gm1 * (wb.a[k] - hb);
+                    rb.a[k] = c.gm1 * (wb.a[k] + hb);
+                    if (GEO == CYL_RADIAL) {
+                        pa = (double)la + (double)ra.a[k];
+                        pb = (double)lb.a[k] + (double)rb.a[k];
+                    }
+                } else {
+                    la = wa.a[k] - ha;
+                    ra.a[k] = wa.a[k] + ha;
+                    lb.a[k] = wb.a[k] - hb;
+                    rb.a[k] = wb.a[k] + hb;
+                }
+                R[k * TT + p.own] = la;
+            }
+            fm = stage_flux<METHOD, FT>(c, ra, lb);
+        }
+        __syncthreads();
+        V5<FT> fb;
+        if (act) {
+            V5<FT> lr;
+#pragma unroll
+            for (int k = 0; k < 5; k++) lr.a[k] = R[k * TT + p.right];
+            fb = stage_flux<METHOD, FT>(c, rb, lr);
+#pragma unroll
+            for (int k = 0; k < 5; k++) P[k * TT + p.own] = (ODD && p.ghost) ? fm.a[k] : fb.a[k];
+        }
+        __syncthreads();
+        if (act) {
+            const double lam = (GEO == CYL_THETA_LAM) ? lambda / g.rpen : lambda;
+            // the isothermal HLL radial term's density: the new prediction (first stage), the stage's own
+            // floored input (second)
+            const double rho_a = va[0], rho_b = vb[0];
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const double fl = (double)P[k * TT + p.left], fc = (double)fm.a[k], fr = (double)fb.a[k];
+                const double ta = second ? SS[k * TT + p.own] : ua[k], tb = second ? SS[(5 + k) * TT + p.own] : ub[k];
+                double na, nb;
+                if constexpr (GEO == CYL_NONE) {
+                    na = ta - lambda * (fc - fl);
+                    nb = tb - lambda * (fr - fc);
+                } else {
+                    na = ta - cyl_dflux<METHOD, GEO>(k, fc, fl, lam, g.ra, g.dr, g.rpen, pa, pa,
+                                                     second ? rho_a : (k == 0 ? 0.0 : va[0]), c);
+                    nb = tb - cyl_dflux<METHOD, GEO>(k, fr, fc, lam, g.rb, g.dr, g.rpen, pb, pb,
+                                                     second ? rho_b : (k == 0 ? 0.0 : vb[0]), c);
+                }
+                if (second) {
+                    ua[k] = .5 * na;
+                    ub[k] = .5 * nb;
+                } else {
+                    va[k] = na;
+                    vb[k] = nb;
+                }
+            }
+        }
+    }
+}
+
+// Dynamic shared memory of a CTA of TT threads: the planes and the SSPRK sums.
+template <typename FT, int TT>
+__host__ __device__ constexpr size_t duo_smem_bytes() { return (size_t)15 * TT * sizeof(FT) + (size_t)80 * TT; }
+
+// CTAs per SM that the registers are held to: about 20 warps of 96 registers per SM for FP64, 24 of 80 for the
+// FP32 flux (256^3 x: 0.327 ms against 0.352 at 96); FP64 CTAs of 256 and 512 threads take 128 registers
+template <typename FT>
+constexpr int duo_min_blocks(int TT)
+{
+    if (sizeof(FT) == 4) return TT <= 128 ? 6 : (TT <= 160 ? 5 : (TT <= 192 ? 4 : (TT <= 256 ? 3 : 1)));
+    return TT <= 128 ? 5 : (TT <= 160 ? 4 : (TT <= 192 ? 3 : (TT <= 256 ? 2 : 1)));
+}
+
+// ------------------------------------------------------------------------------------------
+// x rows: rp rows per CTA (short rows share one), T = ceil(n / 2) threads each.  vec: 16-byte accesses.
+// ------------------------------------------------------------------------------------------
+template <int METHOD, int SLOPE, typename FT, int TT, int NS, bool ODD, int GEO>
+__global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT)) duo_row_kernel(SweepArgs a, FluidConsts<FT> c, int rp, int T, int vec)
+{
+    extern __shared__ __align__(16) unsigned char row_smem_raw[];
+    double *SS = reinterpret_cast<double *>(row_smem_raw);
+    FT *planes = reinterpret_cast<FT *>(SS + 10 * TT);
+    if (a.lambda.off()) return;  // a device timestep of 0: after the end time
+    const double lambda = a.lambda.get();
+    const int n = a.nx;
+    const int r = threadIdx.x / T, t = threadIdx.x - r * T;
+    const int64_t row = (int64_t)blockIdx.x * rp + r;
+    const bool act = r < rp && row < (int64_t)a.ny * a.nz;
+    DuoPos p;
+    p.own = threadIdx.x;
+    p.left = (t == 0) ? p.own + T - 1 : p.own - 1;
+    p.right = (t == T - 1) ? p.own - (T - 1) : p.own + 1;
+    p.first = ODD && t == 0;
+    p.ghost = ODD && t == T - 1;
+    double ua[5], ub[5];
+    double *q = a.q + row * n + 2 * t;
+#pragma unroll
+    for (int k = 0; k < 5; k++) ua[k] = ub[k] = 1.0;
+    if (act) {
+        if (!ODD && vec) {
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                const double2 v = *reinterpret_cast<const double2 *>(q + (int64_t)slot_of<METHOD, 1>(k) * a.slab);
+                ua[k] = v.x;
+                ub[k] = v.y;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                ua[k] = q[(int64_t)slot_of<METHOD, 1>(k) * a.slab];
+                if (!p.ghost) ub[k] = q[(int64_t)slot_of<METHOD, 1>(k) * a.slab + 1];
+            }
+        }
+    }
+    DuoGeo g;
+    if (GEO == CYL_RADIAL) { g.ra = a.crin + (2 * t) * a.cdr; g.rb = a.crin + (2 * t + 1) * a.cdr; g.dr = a.cdr; }
+    duo_sweeps<METHOD, SLOPE, FT, 1, TT, NS, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
+    if (act) {
+        if (!ODD && vec) {
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+                *reinterpret_cast<double2 *>(q + (int64_t)slot_of<METHOD, 1>(k) * a.slab) = make_double2(ua[k], ub[k]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 5; k++) {
+                q[(int64_t)slot_of<METHOD, 1>(k) * a.slab] = ua[k];
+                if (!p.ghost) q[(int64_t)slot_of<METHOD, 1>(k) * a.slab + 1] = ub[k];
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------
+// y and z pencils by plain loads and stores: COLS pencils per CTA, T = ceil(n / 2) threads each, the
+// pencil fastest, so that COLS lanes read neighbouring doubles.
+// ------------------------------------------------------------------------------------------
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int COLS, bool ODD, int GEO>
+__global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT))
+    duo_pencil_kernel(SweepArgs a, FluidConsts<FT> c, int64_t npencil, CylPencil cyl)
+{
+    extern __shared__ __align__(16) unsigned char row_smem_raw[];
+    double *SS = reinterpret_cast<double *>(row_smem_raw);
+    FT *planes = reinterpret_cast<FT *>(SS + 10 * TT);
+    if (a.lambda.off()) return;  // a device timestep of 0: after the end time
+    const double lambda = a.lambda.get();
+    const PencilMap pm{a.nx, a.ny, a.nz, DIR};
+    const int T = (pm.length() + 1) / 2;
+    const int t = threadIdx.x / COLS;
+    const int64_t pencil = (int64_t)blockIdx.x * COLS + threadIdx.x % COLS;
+    const bool act = t < T && pencil < npencil;
+    DuoPos p;
+    p.own = threadIdx.x;
+    p.left = (t == 0) ? p.own + (T - 1) * COLS : p.own - COLS;
+    p.right = (t == T - 1) ? p.own - (T - 1) * COLS : p.own + COLS;
+    p.first = ODD && t == 0;
+    p.ghost = ODD && t == T - 1;
+    double *q = a.q + pm.base(pencil) + 2 * t * pm.stride();
+    double ua[5], ub[5];
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        ua[k] = act ? q[(int64_t)slot_of<METHOD, DIR>(k) * a.slab] : 1.0;
+        ub[k] = (act && !p.ghost) ? q[(int64_t)slot_of<METHOD, DIR>(k) * a.slab + pm.stride()] : 1.0;
+    }
+    DuoGeo g;
+    if (GEO != CYL_NONE) g.rpen = theta_radius(cyl, (int)(pencil % a.nx), (int)(pencil / a.nx));
+    duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
+    if (act) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            q[(int64_t)slot_of<METHOD, DIR>(k) * a.slab] = ua[k];
+            if (!p.ghost) q[(int64_t)slot_of<METHOD, DIR>(k) * a.slab + pm.stride()] = ub[k];
+        }
+    }
+}
+
+}  // namespace ib

@@ -1,0 +1,111 @@
+// ib_duo_launch.cuh -- host launch logic of the two-cells-a-thread sweep kernels (ib_duo.cuh).
+#pragma once
+
+#include "ib_duo.cuh"
+#include "ib_internal.cuh"
+
+namespace ib {
+
+// Opts a kernel in to the dynamic shared memory it needs, when that grows.
+template <typename K>
+int duo_opt_in(K kern, int &have, size_t bytes)
+{
+    if ((int)bytes <= have) return IB_SUCCESSFUL;
+    const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (rc == IB_SUCCESSFUL) have = (int)bytes;
+    return rc;
+}
+
+template <int METHOD, int SLOPE, typename FT, int TT, int NS, bool ODD, int GEO>
+int launch_duo_row_t(const SweepArgs &a, const FluidConsts<FT> &c, cudaStream_t st)
+{
+    auto kern = duo_row_kernel<METHOD, SLOPE, FT, TT, NS, ODD, GEO>;
+    constexpr size_t shm = duo_smem_bytes<FT, TT>();
+    static int have = 48 * 1024;
+    const int rc = duo_opt_in(kern, have, shm);
+    if (rc) return rc;
+    const int T = (a.nx + 1) / 2, rp = TT / T;
+    const int64_t rows = (int64_t)a.ny * a.nz;
+    const int64_t nblk = (rows + rp - 1) / rp;
+    const int vec = !ODD && !((uintptr_t)a.q & 15) && !(a.slab & 1);
+    kern<<<(unsigned)nblk, (rp * T + 31) / 32 * 32, shm, st>>>(a, c, rp, T, vec);
+    return check_launch();
+}
+
+// x rows of up to 1024 cells.  The thread count is the one that leaves few lanes idle: rows of up to 128
+// cells share a CTA of 128 threads, two rows of 129-160 cells one of 160, longer rows have a CTA of their
+// own.  Against one thread per cell (HLLC FP64, x of 160^3 / 256^3 / 320 x 100 x 64 / 512 x 512 x 64 / 1000 x
+// 100 x 64): 0.142 / 0.535 / 0.078 / 0.607 / 0.312 -> 0.137 / 0.469 / 0.067 / 0.548 / 0.282 ms.
+template <int METHOD, int SLOPE, typename FT, int GEO = CYL_NONE>
+int launch_duo_row(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+                   cudaStream_t st, int nsweep, double crin = 0.0, double cdr = 0.0)
+{
+    const int nx = grid[0];
+    if (nx > 1024 || (int64_t)grid[1] * grid[2] >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
+    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, crin, cdr};
+    const int T = (nx + 1) / 2;
+    auto go = [&](auto ns, auto odd) {
+        auto t = [&](auto tt) {
+            return launch_duo_row_t<METHOD, SLOPE, FT, decltype(tt)::value, decltype(ns)::value, decltype(odd)::value, GEO>(
+                a, c, st);
+        };
+        using std::integral_constant;
+        if (T <= 64 || (T > 80 && T <= 128)) return t(integral_constant<int, 128>{});
+        if (T <= 160) return t(integral_constant<int, 160>{});
+        if (T <= 192) return t(integral_constant<int, 192>{});
+        if (T <= 256) return t(integral_constant<int, 256>{});
+        return t(integral_constant<int, 512>{});
+    };
+    std::integral_constant<int, 1> one;
+    if constexpr (GEO == CYL_NONE) {
+        if (nsweep == 2 && !(nx & 1)) return go(std::integral_constant<int, 2>{}, std::false_type{});
+    }
+    for (int k = 0; k < nsweep; k++) {
+        const int rc = (nx & 1) ? go(one, std::true_type{}) : go(one, std::false_type{});
+        if (rc) return rc;
+    }
+    return IB_SUCCESSFUL;
+}
+
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int COLS, bool ODD, int GEO>
+int launch_duo_pencil_t(const SweepArgs &a, const FluidConsts<FT> &c, int n, cudaStream_t st, const CylPencil &cyl)
+{
+    auto kern = duo_pencil_kernel<METHOD, SLOPE, FT, DIR, TT, COLS, ODD, GEO>;
+    constexpr size_t shm = duo_smem_bytes<FT, TT>();
+    static int have = 48 * 1024;
+    const int rc = duo_opt_in(kern, have, shm);
+    if (rc) return rc;
+    const int64_t np = (int64_t)a.nx * a.ny * a.nz / n;
+    kern<<<(unsigned)((np + COLS - 1) / COLS), ((n + 1) / 2 * COLS + 31) / 32 * 32, shm, st>>>(a, c, np, cyl);
+    return check_launch();
+}
+
+// y and z pencils of up to 512 cells, any nx and alignment: as many neighbouring pencils as 256 threads hold,
+// at most 8
+template <int METHOD, int SLOPE, typename FT, int DIR, int GEO = CYL_NONE>
+int launch_duo_pencil(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+                      cudaStream_t st, int nsweep, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
+{
+    const int n = grid[DIR - 1];
+    if (n > 512 || (int64_t)grid[0] * grid[1] * grid[2] / n >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
+    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, 0.0, 0.0};
+    using std::integral_constant;
+    auto go = [&](auto odd) {
+        auto t = [&](auto tt, auto cols) {
+            return launch_duo_pencil_t<METHOD, SLOPE, FT, DIR, decltype(tt)::value, decltype(cols)::value,
+                                       decltype(odd)::value, GEO>(a, c, n, st, cyl);
+        };
+        if (n > 256) return t(integral_constant<int, 256>{}, integral_constant<int, 1>{});
+        if (n > 128) return t(integral_constant<int, 256>{}, integral_constant<int, 2>{});
+        if (n > 64) return t(integral_constant<int, 256>{}, integral_constant<int, 4>{});
+        if (n > 32) return t(integral_constant<int, 256>{}, integral_constant<int, 8>{});
+        return t(integral_constant<int, 128>{}, integral_constant<int, 8>{});
+    };
+    for (int k = 0; k < nsweep; k++) {
+        const int rc = (n & 1) ? go(std::true_type{}) : go(std::false_type{});
+        if (rc) return rc;
+    }
+    return IB_SUCCESSFUL;
+}
+
+}  // namespace ib

@@ -6,14 +6,13 @@
 // only on cells i-2..i+2 of the row, periodically wrapped (cudaFluidStep.cu:1157-1162), so here
 // both stages run in one kernel straight on the XYZ arrays:
 //
-//  * row kernel (x sweeps, rows up to 1024 cells): one CTA holds one whole periodic row, one
-//    thread per cell (or two), neighbours exchanged through two shared-memory planes;
-//    coalesced loads and stores, no halo recomputation.
+//  * two-cell kernels (ib_duo.cuh: x rows up to 1024 cells, short pencils, pencils TMA cannot
+//    fetch): a CTA holds whole periodic rows or pencils, two neighbouring cells a thread.
 //  * pipeline kernels (y and z sweeps of pencils up to 512 cells): persistent CTAs walk blocks
 //    of adjacent whole pencils that arrive by TMA, double-buffered, and leave by TMA store.
 //  * chunked pipeline (pencils above 512 cells): chunks with 4 halo rows per side, the halos
 //    copied to a side buffer first so every chunk is an independent job.
-//  * tile kernel (whatever the TMA rules exclude: odd nx, long odd rows): a CTA walks four
+//  * tile kernel (long pencils that the TMA rules exclude: odd nx, long odd rows): a CTA walks four
 //    neighbouring pencils in chunks staged in shared memory.
 #pragma once
 
@@ -307,168 +306,6 @@ struct SweepArgs {
     DevScalar lambda;
     double crin, cdr;  // radial sweeps (GEO == CYL_RADIAL): radius of cell 0's centre, radial cell size
 };
-
-// ------------------------------------------------------------------------------------------
-// Row kernel: one CTA per x row (nx <= CPT*blockDim.x), periodic in shared memory.
-// Dynamic shared memory: 2 planes x 5 components x nx elements of FT; with row_ssum, 5 x nx
-// doubles more hold u1 + u0 of the SSPRK average through the second stage, so that neither state
-// stays in registers there (fewer spills at 64 registers; slower for the 512-cell rows and two
-// cells per thread, which keep them in registers).
-// ------------------------------------------------------------------------------------------
-#ifndef IB_ROW_MINB
-#define IB_ROW_MINB 2
-#endif
-template <int CPT, int NFIX>
-__host__ __device__ constexpr bool row_ssum() { return CPT == 1 && NFIX != 512; }
-
-// NS: sweeps applied in a row (1, or 2 for the two same-axis sweeps in the middle of an iteration).
-// GEO == CYL_RADIAL: the radial sweep of cylindrical geometry (x = r), whose update weights the
-// faces by their radii and adds the geometric pressure term to p_r (cyl_dflux); one cell per
-// thread, FP64, one sweep.
-// PADN (rows of a run-time length only): stride of the shared-memory planes fixed at PADN cells,
-// so that the phases address them at constant offsets; 0 = the row length.
-template <int METHOD, int SLOPE, typename FT, int CPT, int NFIX = 0, int NS = 1, int GEO = CYL_NONE, int PADN = 0>
-__global__ void __launch_bounds__(512, (CPT == 1) ? IB_ROW_MINB : 1) sweep_row_kernel(SweepArgs a, FluidConsts<FT> c)
-{
-    static_assert(PADN == 0 || (NFIX == 0 && CPT == 1), "a fixed plane stride for rows of a run-time length");
-    static_assert(GEO == CYL_NONE || (GEO == CYL_RADIAL && row_ssum<CPT, NFIX>() && NS == 1 &&
-                                      std::is_same<FT, double>::value),
-                  "radial rows: one cell per thread with the SSPRK sum in shared memory, one FP64 sweep");
-    // its own name: every declaration of one extern shared array must agree on the alignment, and
-    // the TMA kernels' smem_raw is 1024-byte aligned
-    extern __shared__ __align__(16) unsigned char row_smem_raw[];
-    const int n = NFIX ? NFIX : a.nx;  // NFIX: the row length fixed at compile time
-    const int NP = PADN ? PADN : n;    // stride of the planes
-    FT *SA = reinterpret_cast<FT *>(row_smem_raw);
-    FT *SB = SA + 5 * NP;
-    double *SS = reinterpret_cast<double *>(row_smem_raw + (size_t)10 * NP * sizeof(FT));
-    const int64_t row = blockIdx.x;
-    double *q = a.q + row * n;
-    const int64_t S = a.slab;
-    if (a.lambda.off()) return;  // a device timestep of 0: after the end time
-    const double lambda = a.lambda.get();
-
-    double u0[CPT][5], u1[CPT][5];
-    V5<FT> keep[CPT];  // right faces, later fluxes
-    bool act[CPT];
-    // radial rows: the stage's face pressure sum (HLLC) or its input's pressure (HLL)
-    double psum = 0.0, php = 0.0;
-#pragma unroll
-    for (int m = 0; m < CPT; m++) {
-        int i = threadIdx.x + m * blockDim.x;
-        act[m] = i < n;
-#pragma unroll
-        for (int k = 0; k < 5; k++) u0[m][k] = act[m] ? q[(int64_t)slot_of<METHOD, 1>(k) * S + i] : 1.0;
-    }
-
-#pragma unroll
-    for (int sw = 0; sw < NS; sw++) {
-    if (NS > 1 && sw > 0) {
-        // the next sweep starts from this one's result (the planes alternate: no barrier)
-#pragma unroll
-        for (int m = 0; m < CPT; m++)
-#pragma unroll
-            for (int k = 0; k < 5; k++) u0[m][k] = u1[m][k];
-    }
-#pragma unroll
-    for (int stage = 0; stage < 2; stage++) {
-        double (*u)[5] = (stage == 0) ? u0 : u1;
-        // the planes swap roles between the stages, so neither stage rewrites the plane the
-        // other's last phase reads and no barrier separates them
-        FT *PX = (stage == 0) ? SA : SB;  // primitives, then fluxes
-        FT *PY = (stage == 0) ? SB : SA;  // left faces
-        // (a) primitives -> PX
-#pragma unroll
-        for (int m = 0; m < CPT; m++) {
-            int i = threadIdx.x + m * blockDim.x;
-            if (act[m]) {
-                V5<FT> w = stage_prims<METHOD, 1, FT>(u[m], c);
-#pragma unroll
-                for (int k = 0; k < 5; k++) PX[k * NP + i] = w.a[k];
-                if (GEO == CYL_RADIAL && METHOD == IB_METHOD_HLL) php = (double)w.a[2];
-                if (row_ssum<CPT, NFIX>() && stage == 1) {  // after the prims: HLL floors u1 in place
-#pragma unroll
-                    for (int k = 0; k < 5; k++) SS[k * NP + i] = u1[m][k] + u0[m][k];
-                }
-            }
-        }
-        __syncthreads();
-        // (b) limited faces; left faces -> PY, right faces kept
-#pragma unroll
-        for (int m = 0; m < CPT; m++) {
-            int i = threadIdx.x + m * blockDim.x;
-            if (act[m]) {
-                int il = (i == 0) ? n - 1 : i - 1, ir = (i == n - 1) ? 0 : i + 1;
-                V5<FT> w, dl, dr, L;
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    w.a[k] = PX[k * NP + i];
-                    dl.a[k] = w.a[k] - PX[k * NP + il];
-                    dr.a[k] = PX[k * NP + ir] - w.a[k];
-                }
-                stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, keep[m]);
-#pragma unroll
-                for (int k = 0; k < 5; k++) PY[k * NP + i] = L.a[k];
-                if (GEO == CYL_RADIAL && METHOD == IB_METHOD_HLLC) psum = (double)L.a[1] + (double)keep[m].a[1];
-            }
-        }
-        __syncthreads();
-        // (c) flux through face i+1/2 -> PX
-#pragma unroll
-        for (int m = 0; m < CPT; m++) {
-            int i = threadIdx.x + m * blockDim.x;
-            if (act[m]) {
-                int ir = (i == n - 1) ? 0 : i + 1;
-                V5<FT> Lr;
-#pragma unroll
-                for (int k = 0; k < 5; k++) Lr.a[k] = PY[k * NP + ir];
-                keep[m] = stage_flux<METHOD, FT>(c, keep[m], Lr);
-#pragma unroll
-                for (int k = 0; k < 5; k++) PX[k * NP + i] = keep[m].a[k];
-            }
-        }
-        __syncthreads();
-        // (d) conservative update
-#pragma unroll
-        for (int m = 0; m < CPT; m++) {
-            int i = threadIdx.x + m * blockDim.x;
-            if (act[m]) {
-                int il = (i == 0) ? n - 1 : i - 1;
-                if constexpr (GEO == CYL_RADIAL) {
-                    const double rc = a.crin + i * a.cdr;
-                    // the isothermal HLL term's density: the new prediction (stage 0), the stage's
-                    // own floored input (stage 1)
-                    const double rho_in = u1[m][0];
-#pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        const double rho1 = (stage == 0) ? (k == 0 ? 0.0 : u1[m][0]) : rho_in;
-                        const double d = cyl_dflux<METHOD, GEO>(k, (double)keep[m].a[k], (double)PX[k * NP + il], lambda,
-                                                                rc, a.cdr, 0.0, psum, php, rho1, c);
-                        if (stage == 0) u1[m][k] = u0[m][k] - d;
-                        else u1[m][k] = .5 * (SS[k * NP + i] - d);
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 5; k++) {
-                        double df = (double)keep[m].a[k] - (double)PX[k * NP + il];
-                        if (stage == 0) u1[m][k] = u0[m][k] - lambda * df;
-                        else if (row_ssum<CPT, NFIX>()) u1[m][k] = .5 * (SS[k * NP + i] - lambda * df);
-                        else u1[m][k] = .5 * (u1[m][k] + u0[m][k] - lambda * df);
-                    }
-                }
-            }
-        }
-    }
-    }
-#pragma unroll
-    for (int m = 0; m < CPT; m++) {
-        int i = threadIdx.x + m * blockDim.x;
-        if (act[m]) {
-#pragma unroll
-            for (int k = 0; k < 5; k++) q[(int64_t)slot_of<METHOD, 1>(k) * S + i] = u1[m][k];
-        }
-    }
-}
 
 // ------------------------------------------------------------------------------------------
 // TMA-fed pencil pipeline: a persistent CTA walks pencil blocks b = blockIdx.x, +gridDim.x, ...

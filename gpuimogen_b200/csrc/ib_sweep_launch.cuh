@@ -3,6 +3,7 @@
 
 #include "ib_internal.cuh"
 #include "ib_sweep.cuh"
+#include "ib_duo_launch.cuh"
 
 #include <cstdlib>
 #include <type_traits>
@@ -173,33 +174,6 @@ int launch_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, co
     return check_launch();
 }
 
-// Radial rows (cylindrical x sweeps) of at most 512 cells: the row kernel with the radial update,
-// one CTA per row.  Returns IB_ERROR_NOIMPLEMENT (caller falls back) for longer rows.
-template <int METHOD, int SLOPE>
-int launch_row_radial(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<double> &c,
-                      cudaStream_t st, const CylPencil &cyl)
-{
-    const int nx = grid[0];
-    if (nx > 512) return IB_ERROR_NOIMPLEMENT;
-    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, cyl.rin, cyl.dr};
-    const int64_t rows = (int64_t)grid[1] * grid[2];
-    const int nt = ((nx + 31) / 32) * 32;
-    const size_t shm = (size_t)10 * nx * sizeof(double) + (size_t)40 * nx;  // two planes, the SSPRK sum
-    if (nx == 256) {  // the length at compile time (constant plane offsets, fewer spills); 30 KB
-        sweep_row_kernel<METHOD, SLOPE, double, 1, 256, 1, CYL_RADIAL><<<(unsigned)rows, nt, shm, st>>>(a, c);
-        return check_launch();
-    }
-    auto kern = sweep_row_kernel<METHOD, SLOPE, double, 1, 0, 1, CYL_RADIAL>;
-    static int attr_bytes = 0;
-    if ((int)shm > attr_bytes) {
-        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes = (int)shm;
-    }
-    kern<<<(unsigned)rows, nt, shm, st>>>(a, c);
-    return check_launch();
-}
-
 // Chunked TMA pipeline (sweep_chunk_kernel) for pencils of more than 512 cells: W = 1, R = 256
 // (x rows) or W = 4, R = 128 (y/z pencils), after chunk_halo_kernel has copied the rows around the
 // chunk boundaries to scratch memory.  Returns IB_ERROR_NOIMPLEMENT (caller falls back) when the
@@ -303,13 +277,18 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScala
         const char *e = getenv("IMOGEN_B200_PIPE");  // 0 = the non-TMA kernels only
         return !(e && e[0] == '0');
     }();
-    // x rows load contiguously and the row kernel below is faster for them; y and z pencils
-    // go through the TMA-fed pipeline (IMOGEN_B200_PIPE=x also sends x rows there)
+    // x rows load contiguously and the two-cell row kernel is faster for them; y and z pencils
+    // go through the TMA-fed kernels (IMOGEN_B200_PIPE=x also sends x rows there)
     static const int pipe_x = [] {
         const char *e = getenv("IMOGEN_B200_PIPE");
         return (e && e[0] == 'x') ? 1 : 0;
     }();
-    if (use_pipe && n <= 512 && (dir > 1 || pipe_x)) {
+    // Pencils of 16-63 cells, and z pencils of 64 in x-y planes above 1 MB, take the two-cell kernel: plain
+    // loads of 8 neighbouring pencils (64-byte rows) beat the TMA boxes of 2 or 4 there (HLLC FP64 z of 512 x
+    // 512 x 32 / 512 x 512 x 64 / 192 x 128 x 48: 0.442 / 0.703 / 0.065 -> 0.255 / 0.591 / 0.051 ms; even at 8
+    // cells, 0.106 both).  From 65 cells the boxes win (100-cell y of 1000 x 100 x 64: 0.248 against 0.282).
+    const bool short_pencil = dir > 1 && ((n >= 16 && n < 64) || (dir == 3 && n == 64 && (int64_t)nx * ny * 8 > (1 << 20)));
+    if (use_pipe && n <= 512 && ((dir > 1 && !short_pencil) || (dir == 1 && pipe_x))) {
         int rc = IB_ERROR_NOIMPLEMENT;
         // z pencils of large x-y planes: blocks 4 columns wide (32-byte rows), which the memory
         // system serves far better than 16-byte rows at megabyte strides
@@ -423,71 +402,15 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScala
         if (rc != IB_ERROR_NOIMPLEMENT) return rc;
     }
 
-    if (dir == 1 && nx <= 1024) {
-        // one CTA per row, one or two cells per thread
-        SweepArgs a{q, slab, nx, ny, nz, lambda};
-        const int64_t rows = (int64_t)ny * nz;
-        static const int xcpt = [] {
-            const char *e = getenv("IMOGEN_B200_XCPT");  // 2 = two cells per thread for all rows
-            return (e && e[0] == '2') ? 2 : 1;
-        }();
-        const int cpt = (nx <= 512 && xcpt == 1) ? 1 : 2;
-        // the planes, plus the SSPRK sum where row_ssum holds (one cell per thread, rows but 512)
-        const size_t shm = (size_t)10 * nx * sizeof(FT) + ((cpt == 1 && nx != 512) ? (size_t)40 * nx : 0);
-        // rows above 384 FP64 cells need more than the default 48 KB of shared memory
-        auto opt_in = [](auto kern, size_t bytes) {
-            return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        };
-        auto launch_rows = [&](auto ns_tag) -> int {
-            constexpr int NS = decltype(ns_tag)::value;
-            if (cpt == 1) {
-                int nt = ((nx + 31) / 32) * 32;
-                const size_t max1 = (size_t)10 * 512 * sizeof(FT) + (size_t)40 * 512;
-                // common row lengths get the length at compile time (cheaper shared-memory indexing)
-                if (nx == 256) {
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 256, NS><<<(unsigned)rows, nt, shm, st>>>(a, c);
-                } else if (nx == 512) {
-                    static const int rc0 = opt_in(sweep_row_kernel<METHOD, SLOPE, FT, 1, 512, NS>, max1);
-                    if (rc0) return rc0;
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 512, NS><<<(unsigned)rows, nt, shm, st>>>(a, c);
-                } else if (nx == 128) {
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 128, NS><<<(unsigned)rows, nt, shm, st>>>(a, c);
-                } else if ((METHOD == IB_METHOD_HLLC || (METHOD == IB_METHOD_HLL && sizeof(FT) == 8)) && nx > 64 &&
-                           nx < 128) {
-                    // planes of a fixed 128- or 256-cell stride: constant offsets in the phases,
-                    // fewer spills (HLLC 96^3 x 0.049 -> 0.046 ms, 160^3 0.204 -> 0.190; HLL 4-5 %)
-                    const size_t shm_p = (size_t)10 * 128 * sizeof(FT) + (size_t)40 * 128;
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS, CYL_NONE, 128><<<(unsigned)rows, nt, shm_p, st>>>(a, c);
-                } else if (METHOD == IB_METHOD_HLLC && nx > 256 && nx < 512) {
-                    // HLLC rows of 257-511 cells: planes of a fixed 512-cell stride (384 cells: x
-                    // 0.209 -> 0.195 ms at 384 x 96 x 96, FP32 flux 0.111 -> 0.106; registers already
-                    // limit these CTAs to two per SM, so the larger planes cost none)
-                    const size_t shm_p = (size_t)10 * 512 * sizeof(FT) + (size_t)40 * 512;
-                    static const int rcp = opt_in(sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS, CYL_NONE, 512>, shm_p);
-                    if (rcp) return rcp;
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS, CYL_NONE, 512><<<(unsigned)rows, nt, shm_p, st>>>(a, c);
-                } else if ((METHOD == IB_METHOD_HLLC || (METHOD == IB_METHOD_HLL && sizeof(FT) == 8)) && nx > 128 &&
-                           nx < 256) {
-                    const size_t shm_p = (size_t)10 * 256 * sizeof(FT) + (size_t)40 * 256;
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS, CYL_NONE, 256><<<(unsigned)rows, nt, shm_p, st>>>(a, c);
-                } else {
-                    static const int rc1 = opt_in(sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS>, max1);
-                    if (rc1) return rc1;
-                    sweep_row_kernel<METHOD, SLOPE, FT, 1, 0, NS><<<(unsigned)rows, nt, shm, st>>>(a, c);
-                }
-            } else {
-                int nt = (((nx + 1) / 2 + 31) / 32) * 32;
-                static const int rc2 =
-                    opt_in(sweep_row_kernel<METHOD, SLOPE, FT, 2, 0, NS>, (size_t)10 * 1024 * sizeof(FT));
-                if (rc2) return rc2;
-                sweep_row_kernel<METHOD, SLOPE, FT, 2, 0, NS><<<(unsigned)rows, nt, shm, st>>>(a, c);
-            }
-            return IB_SUCCESSFUL;
-        };
-        int rc = (nsweep == 2) ? launch_rows(std::integral_constant<int, 2>{})
-                               : launch_rows(std::integral_constant<int, 1>{});
-        if (rc) return rc;
-        return check_launch();
+    // whole rows and pencils with two cells a thread: x rows of up to 1024 cells, short pencils, and pencils of
+    // up to 512 cells that TMA's rules exclude (odd nx; HLL y/z of 121 x 90 x 75: 0.065 / 0.065 ms in the tile
+    // kernel, 0.049 / 0.043 here)
+    {
+        int rc;
+        if (dir == 1) rc = launch_duo_row<METHOD, SLOPE, FT>(q, slab, grid, lambda, c, st, nsweep);
+        else if (dir == 2) rc = launch_duo_pencil<METHOD, SLOPE, FT, 2>(q, slab, grid, lambda, c, st, nsweep);
+        else rc = launch_duo_pencil<METHOD, SLOPE, FT, 3>(q, slab, grid, lambda, c, st, nsweep);
+        if (rc != IB_ERROR_NOIMPLEMENT) return rc;
     }
 
     for (int k = 0; k < nsweep; k++) {
@@ -525,27 +448,33 @@ int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], DevScalar lam
         const char *e = getenv("IMOGEN_B200_CYLFAST");  // 0 = the tile kernel for every cylindrical sweep
         return !(e && e[0] == '0');
     }();
-    // theta pencils shorter than pair_min_cells() take the tile kernel (several pencils a CTA)
-    const bool fast = fast_env && (cs.kind == CYL_RADIAL || grid[1] >= pair_min_cells());
+    const bool fast = fast_env;
+    // theta pencils shorter than pair_min_cells() and odd radial sizes take the two-cell kernel's plain loads
+    const bool pair = grid[1] >= pair_min_cells();
     int rc = IB_ERROR_NOIMPLEMENT;
     switch (cs.kind) {
     case CYL_RADIAL:
-        if (fast) rc = launch_row_radial<METHOD, SLOPE>(q, slab, grid, lambda, c, st, cs.pencil);
+        if (fast)
+            rc = launch_duo_row<METHOD, SLOPE, double, CYL_RADIAL>(q, slab, grid, lambda, c, st, 1, cs.pencil.rin, cs.pencil.dr);
         if (rc != IB_ERROR_NOIMPLEMENT) return rc;
         return launch_tile_dw<METHOD, SLOPE, double, 1, 1, CYL_RADIAL>(q, slab, grid, lambda, c, st, 248, cs.pencil);
     case CYL_THETA_DIV:
         // 256-cell pencils get the length at compile time (fewer registers for indexing, no spills)
-        if (fast && grid[1] == 256)
+        if (fast && pair && grid[1] == 256)
             rc = launch_pair<METHOD, SLOPE, double, 2, 256, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
-        else if (fast)
+        else if (fast && pair)
             rc = launch_pair<METHOD, SLOPE, double, 2, 0, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
+        if (fast && rc == IB_ERROR_NOIMPLEMENT)
+            rc = launch_duo_pencil<METHOD, SLOPE, double, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         if (rc != IB_ERROR_NOIMPLEMENT) return rc;
         return launch_tile_dw<METHOD, SLOPE, double, 2, 4, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 56, cs.pencil);
     case CYL_THETA_LAM:
-        if (fast && grid[1] == 256)
+        if (fast && pair && grid[1] == 256)
             rc = launch_pair<METHOD, SLOPE, double, 2, 256, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
-        else if (fast)
+        else if (fast && pair)
             rc = launch_pair<METHOD, SLOPE, double, 2, 0, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
+        if (fast && rc == IB_ERROR_NOIMPLEMENT)
+            rc = launch_duo_pencil<METHOD, SLOPE, double, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         if (rc != IB_ERROR_NOIMPLEMENT) return rc;
         return launch_tile_dw<METHOD, SLOPE, double, 2, 4, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 56, cs.pencil);
     default: return IB_ERROR_INVALID_ARGS;
