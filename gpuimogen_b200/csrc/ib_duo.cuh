@@ -254,4 +254,120 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT))
     }
 }
 
+// ------------------------------------------------------------------------------------------
+// Chunks of long pencils (ib_sweep.cuh: jobs, side buffer, tiles): R / 2 threads per column, two rows each.
+// ------------------------------------------------------------------------------------------
+template <int METHOD, int SLOPE, typename FT, int DIR, int W, int R>
+__global__ void __launch_bounds__(R *W / 2, 512 / (R * W / 2))
+    sweep_chunk_kernel(const __grid_constant__ CUtensorMap tm, ChunkArgs a, FluidConsts<FT> c)
+{
+    constexpr int L = R - 8;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t full[2];
+    constexpr size_t tb = ((size_t)40 * L * W + 127) / 128 * 128;
+    constexpr size_t hb = ((size_t)320 * W + 127) / 128 * 128;
+    // tile and halo block of buffer b (computed, not indexed arrays, which would live in local memory)
+    auto Ub = [&](int b) { return reinterpret_cast<double *>(smem_raw + b * tb); };
+    auto Hb = [&](int b) { return reinterpret_cast<double *>(smem_raw + 2 * tb + b * hb); };
+    double *SS = reinterpret_cast<double *>(smem_raw + 2 * tb + 2 * hb);
+    FT *planes = reinterpret_cast<FT *>(smem_raw + 2 * tb + 2 * hb + (size_t)40 * R * W);
+    constexpr uint32_t tile_tx = 40u * L * W + 320u * W;
+    constexpr int s0 = slot_of<METHOD, DIR>(0), s1 = slot_of<METHOD, DIR>(1), s2 = slot_of<METHOD, DIR>(2),
+                  s3 = slot_of<METHOD, DIR>(3), s4 = slot_of<METHOD, DIR>(4);
+    const int slots[5] = {s0, s1, s2, s3, s4};
+    constexpr int TT = R * W / 2, T = R / 2;
+    const int col = (W == 1) ? 0 : (int)(threadIdx.x % W);
+    const int t = (int)(threadIdx.x / W);  // this thread's cells: rows 2t and 2t + 1 of the job
+    DuoPos p;
+    p.own = threadIdx.x;
+    p.left = (t > 0) ? p.own - W : p.own;  // the job's edge rows: unused results
+    p.right = (t < T - 1) ? p.own + W : p.own;
+    p.first = p.ghost = false;
+    const int n = a.n, C = a.C;
+    if (a.lambda.off()) return;  // a device timestep of 0: after the end time
+    const double lambda = a.lambda.get();
+    const bool leader = threadIdx.x == 0;
+    const int64_t njobs_all = a.ngroups * C;
+    const int64_t step = gridDim.x;
+
+    if (leader) {
+        prefetch_tmap(&tm);
+        mbar_init(&full[0], 1);
+        mbar_init(&full[1], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    auto issue = [&](int64_t j, int buf) {  // leader only
+        mbar_arrive_expect_tx(&full[buf], tile_tx);
+        chunk_load<DIR>(Ub(buf), &tm, j / C, (int)(j % C) * L, a, W, &full[buf]);
+        bulk_load(Hb(buf), a.side + j * 40 * W, 320u * W, &full[buf]);
+    };
+    // bit b: a load into buffer b is in flight (leader's bookkeeping) / parity to wait for on b
+    uint32_t issued = 0, phase = 0;
+    if (leader) {
+        for (int t = 0; t < 2; t++) {
+            const int64_t jt = blockIdx.x + t * step;
+            if (jt < njobs_all) { issue(jt, t); issued |= 1u << t; }
+        }
+    }
+    int it = 0;
+    for (int64_t j = blockIdx.x; j < njobs_all; j += step, it++) {
+        const int buf = it & 1;
+        const int64_t grp = j / C;
+        const int cc = (int)(j % C);
+        const int c0 = cc * L;                    // first cell of the chunk
+        const int cend = (c0 + L < n) ? c0 + L : n;
+        const bool ok = mbar_wait_cta(&full[buf], (phase >> buf) & 1, a.spin);
+        if (!ok) {
+            if (leader) {
+                atomicOr(a.err, 1u);
+                mbar_wait(&full[buf], (phase >> buf) & 1);  // one more bounded wait for the late tile
+                if ((issued >> (buf ^ 1)) & 1) mbar_wait(&full[buf ^ 1], (phase >> (buf ^ 1)) & 1);
+            }
+            return;
+        }
+        phase ^= 1u << buf;
+        issued &= ~(1u << buf);
+        // row r is cell g = c0 - 4 + r: left halo (side buffer), chunk (tile), right halo (side buffer), or
+        // idle
+        const double *Ut = Ub(buf), *H = Hb(buf);
+        auto fetch = [&](int r, double (&u)[5]) {
+            const int g = c0 - 4 + r;
+            if (g >= c0 && g < cend) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) u[k] = Ut[(slots[k] * L + (g - c0)) * W + col];
+            } else if (g < cend + 4) {
+                const int rr = (g < c0) ? r : 4 + (g - cend);
+#pragma unroll
+                for (int k = 0; k < 5; k++) u[k] = H[(slots[k] * 8 + rr) * W + col];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 5; k++) u[k] = 1.0;
+            }
+        };
+        double ua[5], ub[5];
+        fetch(2 * t, ua);
+        fetch(2 * t + 1, ub);
+        __syncthreads();  // every thread has read tile buf (and is done with the planes)
+        if (leader) {
+            // request the job after next into it
+            const int64_t jn = j + 2 * step;
+            if (jn < njobs_all) {
+                fence_proxy_async_smem();
+                issue(jn, buf);
+                issued |= 1u << buf;
+            }
+        }
+        duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
+        double *base = a.q + chunk_base(a, DIR, W, grp, col);
+        const int g = c0 - 4 + 2 * t;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            double *cell = base + slots[k] * a.slab + (int64_t)g * a.rs;
+            if (g >= c0 && g < cend) cell[0] = ua[k];
+            if (g + 1 >= c0 && g + 1 < cend) cell[a.rs] = ub[k];
+        }
+    }
+}
+
 }  // namespace ib

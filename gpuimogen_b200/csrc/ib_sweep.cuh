@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(512, (CPT == 1) ? 2 : 1)
 // n: pencil length (the box), np: stride of the planes (the pencil length, or PADN)
 __host__ __device__ __forceinline__ size_t pair_smem_bytes(int n, int ftsize, int wc, int np)
 {
-    return pipe_tile_bytes(n, wc) + (size_t)10 * np * ftsize + (size_t)40 * np;
+    return pipe_tile_bytes(n, wc) + (size_t)10 * np * ftsize + (wc == 4 ? 0 : (size_t)40 * np);
 }
 
 // WC: pencils per box (2; 4 for z sweeps of x-y planes above 1 MB, whose 16-byte rows a plane
@@ -568,7 +568,7 @@ __host__ __device__ __forceinline__ size_t pair_smem_bytes(int n, int ftsize, in
 // fewer spills); 0 = the pencil length.
 template <int METHOD, int SLOPE, typename FT, int DIR, int NFIX = 0, int NS = 1, int WC = 2, int GEO = CYL_NONE,
           int PADN = 0>
-__global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : (WC == 4 ? 3 : 4))
+__global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((WC == 4 && sizeof(FT) == 8) ? 3 : 4))
     sweep_pair_kernel(const __grid_constant__ CUtensorMap tm, PipeArgs a, FluidConsts<FT> c, CylPencil cyl)
 {
     static_assert(GEO == CYL_NONE || ((GEO == CYL_THETA_DIV || GEO == CYL_THETA_LAM) && DIR == 2 && NS == 1 &&
@@ -615,7 +615,11 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : (WC
     }
 #pragma unroll 1
     for (int col = 0; col < WC; col++) {
-        auto TI = [&](int k) { return (k * n + i) * WC + col; };
+        // 4-pencil boxes: the tensor map's 32-byte swizzle swaps the 16-byte halves of every other 128 bytes
+        auto TI = [&](int k) {
+            const int x = (k * n + i) * WC + col;
+            return (WC == 4) ? x ^ ((x >> 3) & 2) : x;
+        };
         double u0[5], u1[5];
         V5<FT> keep;
         double rp = 0.0, lam = lambda;  // theta pencils: the pencil's radius and the lambda it takes
@@ -642,7 +646,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : (WC
                     for (int k = 0; k < 5; k++) PX[k * NP + i] = w.a[k];
                     if (stage == 1) {
 #pragma unroll
-                        for (int k = 0; k < 5; k++) SS[k * NP + i] = u1[k] + u0[k];
+                        for (int k = 0; k < 5; k++) (WC == 4 ? T[TI(slots[k])] : SS[k * NP + i]) = u1[k] + u0[k];
                     }
                 }
                 __syncthreads();
@@ -674,12 +678,12 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : (WC
                         if constexpr (GEO == CYL_NONE) {
                             double df = (double)keep.a[k] - (double)PX[k * NP + il];
                             if (stage == 0) u1[k] = u0[k] - lambda * df;
-                            else u1[k] = .5 * (SS[k * NP + i] - lambda * df);
+                            else u1[k] = .5 * ((WC == 4 ? T[TI(slots[k])] : SS[k * NP + i]) - lambda * df);
                         } else {
                             const double d = cyl_dflux<METHOD, GEO>(k, (double)keep.a[k], (double)PX[k * NP + il], lam,
                                                                     0.0, 0.0, rp, 0.0, 0.0, 0.0, c);
                             if (stage == 0) u1[k] = u0[k] - d;
-                            else u1[k] = .5 * (SS[k * NP + i] - d);
+                            else u1[k] = .5 * ((WC == 4 ? T[TI(slots[k])] : SS[k * NP + i]) - d);
                         }
                     }
                 }
@@ -885,9 +889,9 @@ __global__ void __launch_bounds__(512, 1)
 //     and its halo block as one untiled bulk copy, on the same mbarrier; the loads of the next two
 //     jobs are in flight while one is computed (double-buffered, bounded waits).  Outputs are
 //     plain stores from registers.
+// A thread computes two neighbouring cells (ib_duo.cuh, sweep_chunk_kernel).
 // Dynamic shared memory: 2 tiles of 40*L*W bytes and 2 halo blocks of 320*W bytes (each rounded to
-// 128), the SSPRK sum u1 + u0 through the second stage (40*R*W bytes: neither state stays in
-// registers there), then 2 planes of 5*R*W elements of FT.
+// 128), the SSPRK sums (40*R*W bytes), then the two-cell kernels' planes (15 values of FT a thread).
 // ------------------------------------------------------------------------------------------
 struct ChunkArgs {
     double *q;
@@ -904,10 +908,11 @@ struct ChunkArgs {
     uint32_t spin;       // poll limit of the tile waits
 };
 
+// (the planes and the SSPRK sums of R W / 2 threads)
 __host__ __device__ constexpr size_t chunk_smem_bytes(int W, int R, int ftsize)
 {
     return 2 * (((size_t)40 * (R - 8) * W + 127) / 128 * 128) + 2 * (((size_t)320 * W + 127) / 128 * 128) +
-           (size_t)40 * R * W + (size_t)10 * R * W * ftsize;
+           (size_t)40 * R * W + (size_t)15 * R * W / 2 * ftsize;
 }
 
 // First cell of pencil block grp, column col.
@@ -944,153 +949,6 @@ __device__ __forceinline__ void chunk_load(double *dst, const CUtensorMap *tm, i
 {
     if (DIR == 1) tma_load_3d(dst, tm, g0, (int)grp, 0, bar);
     else tma_load_4d(dst, tm, (int)(grp % a.npw) * W, g0, (int)(grp / a.npw), 0, bar);
-}
-
-template <int METHOD, int SLOPE, typename FT, int DIR, int W, int R>
-__global__ void __launch_bounds__(512, 2)
-    sweep_chunk_kernel(const __grid_constant__ CUtensorMap tm, ChunkArgs a, FluidConsts<FT> c)
-{
-    constexpr int L = R - 8;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[2];
-    constexpr size_t tb = ((size_t)40 * L * W + 127) / 128 * 128;
-    constexpr size_t hb = ((size_t)320 * W + 127) / 128 * 128;
-    // tile and halo block of buffer b (computed, not indexed arrays, which would live in local memory)
-    auto Ub = [&](int b) { return reinterpret_cast<double *>(smem_raw + b * tb); };
-    auto Hb = [&](int b) { return reinterpret_cast<double *>(smem_raw + 2 * tb + b * hb); };
-    double *SS = reinterpret_cast<double *>(smem_raw + 2 * tb + 2 * hb);
-    FT *SA = reinterpret_cast<FT *>(smem_raw + 2 * tb + 2 * hb + (size_t)40 * R * W);
-    FT *SB = SA + 5 * R * W;
-    constexpr uint32_t tile_tx = 40u * L * W + 320u * W;
-    constexpr int s0 = slot_of<METHOD, DIR>(0), s1 = slot_of<METHOD, DIR>(1), s2 = slot_of<METHOD, DIR>(2),
-                  s3 = slot_of<METHOD, DIR>(3), s4 = slot_of<METHOD, DIR>(4);
-    const int slots[5] = {s0, s1, s2, s3, s4};
-    const int col = (W == 1) ? 0 : (int)(threadIdx.x % W);
-    const int r = (int)(threadIdx.x / W);  // row of this thread in the job; blockDim.x = W * R
-    const int il = (r > 0) ? r - 1 : 0, ir = (r < R - 1) ? r + 1 : R - 1;  // edge rows: unused results
-    auto SI = [&](int k, int j) { return (k * R + j) * W + col; };
-    const int n = a.n, C = a.C;
-    if (a.lambda.off()) return;  // a device timestep of 0: after the end time
-    const double lambda = a.lambda.get();
-    const bool leader = threadIdx.x == 0;
-    const int64_t njobs_all = a.ngroups * C;
-    const int64_t step = gridDim.x;
-
-    if (leader) {
-        prefetch_tmap(&tm);
-        mbar_init(&full[0], 1);
-        mbar_init(&full[1], 1);
-        fence_mbar_init();
-    }
-    __syncthreads();
-    auto issue = [&](int64_t j, int buf) {  // leader only
-        mbar_arrive_expect_tx(&full[buf], tile_tx);
-        chunk_load<DIR>(Ub(buf), &tm, j / C, (int)(j % C) * L, a, W, &full[buf]);
-        bulk_load(Hb(buf), a.side + j * 40 * W, 320u * W, &full[buf]);
-    };
-    // bit b: a load into buffer b is in flight (leader's bookkeeping) / parity to wait for on b
-    uint32_t issued = 0, phase = 0;
-    if (leader) {
-        for (int t = 0; t < 2; t++) {
-            const int64_t jt = blockIdx.x + t * step;
-            if (jt < njobs_all) { issue(jt, t); issued |= 1u << t; }
-        }
-    }
-    int it = 0;
-    for (int64_t j = blockIdx.x; j < njobs_all; j += step, it++) {
-        const int buf = it & 1;
-        const int64_t grp = j / C;
-        const int cc = (int)(j % C);
-        const int c0 = cc * L;                    // first cell of the chunk
-        const int cend = (c0 + L < n) ? c0 + L : n;
-        const bool ok = mbar_wait_cta(&full[buf], (phase >> buf) & 1, a.spin);
-        if (!ok) {
-            if (leader) {
-                atomicOr(a.err, 1u);
-                mbar_wait(&full[buf], (phase >> buf) & 1);  // one more bounded wait for the late tile
-                if ((issued >> (buf ^ 1)) & 1) mbar_wait(&full[buf ^ 1], (phase >> (buf ^ 1)) & 1);
-            }
-            return;
-        }
-        phase ^= 1u << buf;
-        issued &= ~(1u << buf);
-        // this thread's cell g = c0 - 4 + r: left halo (side buffer, boundary cc), chunk (tile),
-        // right halo (side buffer, boundary cc + 1 mod C), or idle
-        const int g = c0 - 4 + r;
-        const bool act = g < cend + 4;
-        double u0[5], u1[5];
-        if (g >= c0 && g < cend) {
-            const double *Ut = Ub(buf);
-#pragma unroll
-            for (int k = 0; k < 5; k++) u0[k] = Ut[(slots[k] * L + (g - c0)) * W + col];
-        } else if (act) {
-            const int rr = (g < c0) ? r : 4 + (g - cend);
-            const double *H = Hb(buf);
-#pragma unroll
-            for (int k = 0; k < 5; k++) u0[k] = H[(slots[k] * 8 + rr) * W + col];
-        } else {
-#pragma unroll
-            for (int k = 0; k < 5; k++) u0[k] = 1.0;
-        }
-        V5<FT> keep;
-#pragma unroll
-        for (int stage = 0; stage < 2; stage++) {
-            double *u = (stage == 0) ? u0 : u1;
-            {
-                V5<FT> w = stage_prims<METHOD, DIR, FT>(u, c);
-#pragma unroll
-                for (int k = 0; k < 5; k++) SA[SI(k, r)] = w.a[k];
-                if (stage == 1) {  // after the prims: HLL floors u1 in place
-#pragma unroll
-                    for (int k = 0; k < 5; k++) SS[SI(k, r)] = u1[k] + u0[k];
-                }
-            }
-            __syncthreads();
-            if (stage == 0 && leader) {
-                // every thread has read tile buf: request the job after next into it
-                const int64_t jn = j + 2 * step;
-                if (jn < njobs_all) {
-                    fence_proxy_async_smem();
-                    issue(jn, buf);
-                    issued |= 1u << buf;
-                }
-            }
-            {
-                V5<FT> w, dl, dr, Lf;
-#pragma unroll
-                for (int k = 0; k < 5; k++) {
-                    w.a[k] = SA[SI(k, r)];
-                    dl.a[k] = w.a[k] - SA[SI(k, il)];
-                    dr.a[k] = SA[SI(k, ir)] - w.a[k];
-                }
-                stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, Lf, keep);
-#pragma unroll
-                for (int k = 0; k < 5; k++) SB[SI(k, r)] = Lf.a[k];
-            }
-            __syncthreads();
-            {
-                V5<FT> Lr;
-#pragma unroll
-                for (int k = 0; k < 5; k++) Lr.a[k] = SB[SI(k, ir)];
-                keep = stage_flux<METHOD, FT>(c, keep, Lr);
-#pragma unroll
-                for (int k = 0; k < 5; k++) SA[SI(k, r)] = keep.a[k];
-            }
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                double df = (double)keep.a[k] - (double)SA[SI(k, il)];
-                if (stage == 0) u1[k] = u0[k] - lambda * df;
-                else u1[k] = .5 * (SS[SI(k, r)] - lambda * df);
-            }
-            __syncthreads();  // the planes are rewritten next
-        }
-        if (g >= c0 && g < cend) {
-            double *base = a.q + chunk_base(a, DIR, W, grp, col);
-#pragma unroll
-            for (int k = 0; k < 5; k++) base[slots[k] * a.slab + (int64_t)g * a.rs] = u1[k];
-        }
-    }
 }
 
 // The HLL corrector adds (fluid after the floors of the predictor's pressure pass) and

@@ -133,7 +133,7 @@ int launch_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, co
     static_assert(GEO == CYL_NONE || DIR == 2, "theta pencils run along y");
     if (GEO != CYL_NONE && nsweep != 1) return IB_ERROR_NOIMPLEMENT;
     static_assert(DIR != 1, "x rows take the row kernel");
-    static_assert(WC == 2 || (WC == 4 && NFIX != 512), "boxes of 2 pencils, or 4 of at most 256 cells");
+    static_assert(WC == 2 || (WC == 4 && (NFIX != 512 || sizeof(FT) == 4)), "boxes of 2 pencils, or 4 (512 cells: FP32 flux)");
     const int nx = grid[0], ny = grid[1], nz = grid[2];
     const int n = grid[DIR - 1];
     if ((n > 256 && !(NFIX == 512 && n == 512)) || (nx % WC)) return IB_ERROR_NOIMPLEMENT;
@@ -151,7 +151,7 @@ int launch_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, co
     const int64_t nblocks = (int64_t)npw * other;
     if (nblocks >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
     CUtensorMap tm;
-    int rc = encode_tmap_f64(&tm, q, 5, dims, strides, box);
+    int rc = encode_tmap_f64(&tm, q, 5, dims, strides, box, WC == 4);
     if (rc) return rc;
     unsigned int *err = scratch().wait_flag();
     if (!err) return IB_ERROR_NOMEM;
@@ -233,7 +233,7 @@ int launch_chunk(double *q, int64_t slab, const int grid[3], DevScalar lambda, c
         rc = check_launch();
         if (rc) return rc;
     }
-    const int nt = W * R;
+    const int nt = W * R / 2;
     const size_t shm = chunk_smem_bytes(W, R, (int)sizeof(FT));
     auto kern = sweep_chunk_kernel<METHOD, SLOPE, FT, DIR, W, R>;
     static int attr_bytes = 0;

@@ -27,7 +27,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 encoder()
 }
 
 int encode_tmap_f64(CUtensorMap *map, void *base, int rank, const uint64_t *dims, const uint64_t *strides_bytes,
-                    const uint32_t *box)
+                    const uint32_t *box, bool swizzle32)
 {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encoder();
     if (!fn) return IB_ERROR_NOIMPLEMENT;
@@ -46,7 +46,8 @@ int encode_tmap_f64(CUtensorMap *map, void *base, int rank, const uint64_t *dims
         if (gs[i] % 16 != 0) return IB_ERROR_NOIMPLEMENT;
     }
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, (cuuint32_t)rank, base, gd, gs, bx, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    swizzle32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? IB_SUCCESSFUL : IB_ERROR_NOIMPLEMENT;
 }

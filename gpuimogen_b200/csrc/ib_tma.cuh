@@ -169,8 +169,9 @@ __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *map)
 }
 
 // Host: encodes a tiled FP64 tensor map (rank <= 5; dims innermost first, strides in bytes for
-// dims 1..rank-1, box extents <= 256).  Returns 0 on success, else a status.
+// dims 1..rank-1, box extents <= 256).  swizzle32 (rows of 32 bytes, 256-byte aligned box): every other
+// 128 bytes of the box hold their 16-byte halves exchanged.  Returns 0 on success, else a status.
 int encode_tmap_f64(CUtensorMap *map, void *base, int rank, const uint64_t *dims, const uint64_t *strides_bytes,
-                    const uint32_t *box);
+                    const uint32_t *box, bool swizzle32 = false);
 
 }  // namespace ib
