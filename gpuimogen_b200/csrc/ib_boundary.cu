@@ -41,6 +41,31 @@ __global__ void fluid_boundary_kernel(double *q, int64_t S, PencilIdx pi, int64_
     }
 }
 
+// The same fill with one thread per pencil, side and slab (one per side for outflow, whose slabs depend on
+// one another), for pencils long enough that neither side reads what the other writes.  A pencil's fill is
+// a chain of dependent loads and stores: one thread per pencil took 5 us on a single row (a 1-D problem
+// pays that twice an iteration).
+__global__ void __launch_bounds__(128) fluid_boundary_split_kernel(double *q, int64_t S, PencilIdx pi, int64_t npencil,
+                                                                   int mode0, int mode1, int depth)
+{
+    const int64_t id = threadIdx.x + (int64_t)blockIdx.x * blockDim.x;
+    // x rows: a row's ten items next to one another; y and z: neighbouring pencils next to one another
+    const int64_t p = (pi.dir == 1) ? id / 10 : id % npencil;
+    const int item = (int)((pi.dir == 1) ? id % 10 : id / npencil);
+    if (p >= npencil || item >= 10) return;
+    const int side = item / 5, k = item % 5;
+    const int mode = side ? mode1 : mode0;
+    int64_t base, s;
+    int n;
+    pi.get(p, base, s, n);
+    double *v0 = q + base;
+    if (mode == IB_BC_OUTFLOW) {
+        if (k == 0) outflow_x(v0, S, s, n, side, pi.dir, depth);
+    } else if (mode == IB_BC_MIRROR || mode == IB_BC_CONST || mode == IB_BC_LINEAR) {
+        sas_x(v0 + k * S, s, n, mode, side, (k >= 2) && (k - 1 == pi.dir), depth);
+    }
+}
+
 static bool mode_ok(int m)
 {
     return m == IB_BC_CIRCULAR || m == IB_BC_STATIONARY || m == IB_BC_MIRROR || m == IB_BC_CONST ||
@@ -61,6 +86,12 @@ int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int3
     const int64_t N = (int64_t)grid[0] * grid[1] * grid[2];
     const int64_t np = N / n;
     PencilIdx pi{grid[0], grid[1], grid[2], dir};
+    // a side reads at most 2 halo + 1 cells from its own end (linear: 4 from halo on) and writes halo cells
+    if (n >= 3 * halo + 4) {
+        const int64_t items = 10 * np;
+        fluid_boundary_split_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo);
+        return check_launch();
+    }
     fluid_boundary_kernel<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo);
     return check_launch();
 }
