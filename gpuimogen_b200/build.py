@@ -24,23 +24,27 @@ CSRC = os.path.join(HERE, "csrc")
 ROOT = os.path.dirname(HERE)
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 
+# the longest compiles first
 SOURCES = [
-    "ib_capi.cu",
-    "ib_tma.cu",
-    "ib_ensemble.cu",
-    "ib_mlp.cu",
-    "ib_drag_learned.cu",
+    "ib_sweep_cyl.cu",
+    "ib_sweep_hll64.cu",
+    "ib_sweep_hll64_b.cu",
     "ib_sweep_hllc64.cu",
     "ib_sweep_hllc32.cu",
-    "ib_sweep_hll64.cu",
+    "ib_sweep_hllc64_b.cu",
+    "ib_sweep_hllc32_b.cu",
     "ib_xinjin.cu",
+    "ib_ensemble.cu",
+    "ib_drag.cu",
+    "ib_drag_learned.cu",
     "ib_reduce.cu",
     "ib_boundary.cu",
-    "ib_drag.cu",
+    "ib_mlp.cu",
+    "ib_capi.cu",
+    "ib_cylsrc.cu",
+    "ib_tma.cu",
     "ib_tags.cu",
     "ib_time.cu",
-    "ib_sweep_cyl.cu",
-    "ib_cylsrc.cu",
 ]
 HEADERS = ["ib_common.cuh", "ib_internal.cuh", "ib_sweep.cuh", "ib_sweep_launch.cuh", "ib_tma.cuh", "ib_bc.cuh",
            "ib_cfl.cuh", "ib_drag.cuh", "ib_tcgen05.cuh", "ib_cyl.cuh", "ib_fast.cuh", "ib_duo.cuh", "ib_duo_launch.cuh"]
@@ -68,7 +72,7 @@ def _newest_input():
 # Files whose single-precision arithmetic is only the FP32-flux form: FP32 division and square
 # root there use the hardware approximations (FP64 arithmetic is unaffected by these flags).
 FP32_FAST = ["-prec-div=false", "-prec-sqrt=false", "-ftz=true"]
-PER_FILE = {"ib_sweep_hllc32.cu": FP32_FAST, "ib_ensemble.cu": FP32_FAST}
+PER_FILE = {"ib_sweep_hllc32.cu": FP32_FAST, "ib_sweep_hllc32_b.cu": FP32_FAST, "ib_ensemble.cu": FP32_FAST}
 
 
 def _compile(src, obj, extra):
@@ -79,26 +83,39 @@ def _compile(src, obj, extra):
     return obj
 
 
-def build_variant(name, force=False, jobs=None):
-    libname, extra = VARIANTS[name]
-    out = os.path.join(HERE, libname)
-    if not force and os.path.exists(out) and os.path.getmtime(out) >= _newest_input():
-        return out
-    objdir = os.path.join(ROOT, "_build", name)
-    os.makedirs(objdir, exist_ok=True)
-    objs = [os.path.join(objdir, s.replace(".cu", ".o")) for s in SOURCES]
-    jobs = jobs or max(1, min(len(SOURCES), os.cpu_count() or 4))
-    with cf.ThreadPoolExecutor(max_workers=jobs) as ex:
-        futs = [ex.submit(_compile, s, o, extra) for s, o in zip(SOURCES, objs)]
-        for f in futs:
-            f.result()
+def _link(name, objs):
+    out = os.path.join(HERE, VARIANTS[name][0])
     tmp = out + ".tmp"
     cmd = [NVCC, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", tmp] + objs + ["-lcudart_static"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n%s\n%s" % (" ".join(cmd), r.stderr))
     os.replace(tmp, out)
-    return out
+
+
+def build_variants(names, force=False, jobs=None):
+    """Compiles what is out of date of the named variants in one pool, then links them."""
+    outs = [os.path.join(HERE, VARIANTS[n][0]) for n in names]
+    todo = [n for n, out in zip(names, outs)
+            if force or not (os.path.exists(out) and os.path.getmtime(out) >= _newest_input())]
+    objs = {}
+    with cf.ThreadPoolExecutor(max_workers=jobs or max(1, os.cpu_count() or 4)) as ex:
+        futs = []
+        for n in todo:
+            objdir = os.path.join(ROOT, "_build", n)
+            os.makedirs(objdir, exist_ok=True)
+            objs[n] = [os.path.join(objdir, s.replace(".cu", ".o")) for s in SOURCES]
+        for k, s in enumerate(SOURCES):
+            futs += [ex.submit(_compile, s, objs[n][k], VARIANTS[n][1]) for n in todo]
+        for f in futs:
+            f.result()
+    for n in todo:
+        _link(n, objs[n])
+    return outs
+
+
+def build_variant(name, force=False, jobs=None):
+    return build_variants([name], force, jobs)[0]
 
 
 DRIVER_SRC = os.path.join(HERE, "driver", "imogen_run.cpp")
@@ -124,7 +141,7 @@ def build_driver(force=False):
 
 def build(force=False, only=None):
     names = [only] if only else list(VARIANTS)
-    out = [build_variant(n, force=force) for n in names]
+    out = build_variants(names, force=force)
     if only in (None, "product"):
         out.append(build_driver(force=force))
     return out

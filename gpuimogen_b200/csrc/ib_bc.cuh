@@ -82,4 +82,26 @@ __device__ __forceinline__ void outflow_x(double *v0, int64_t S, int64_t s, int 
     }
 }
 
+// Whether the two ends of a pencil of n cells can be filled apart: a side reads at most 2 depth + 1 cells from
+// its own end (linear: 4 from depth on) and writes depth cells.
+__host__ __device__ inline bool row_fill_apart(int n, int depth) { return n >= 3 * depth + 4; }
+__host__ __device__ inline bool row_fill_mode(int m)
+{
+    return m == IB_BC_CIRCULAR || m == IB_BC_STATIONARY || m == IB_BC_MIRROR || m == IB_BC_CONST || m == IB_BC_LINEAR ||
+           m == IB_BC_OUTFLOW;
+}
+
+// One of the ten parts of a pencil's fill: slab item % 5 on side item / 5 (outflow, whose slabs depend on
+// one another: all of them with slab 0).  dir: the pencil's direction, whose momentum mirror reverses.
+__device__ __forceinline__ void fill_item(double *v0, int64_t S, int64_t s, int n, const RowBc &bc, int dir, int item)
+{
+    const int side = item / 5, k = item % 5;
+    const int mode = side ? bc.mode1 : bc.mode0;
+    if (mode == IB_BC_OUTFLOW) {
+        if (k == 0) outflow_x(v0, S, s, n, side, dir, bc.depth);
+    } else if (mode == IB_BC_MIRROR || mode == IB_BC_CONST || mode == IB_BC_LINEAR) {
+        sas_x(v0 + k * S, s, n, mode, side, (k >= 2) && (k - 1 == dir), bc.depth);
+    }
+}
+
 }  // namespace ib

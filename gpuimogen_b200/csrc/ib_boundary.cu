@@ -53,23 +53,10 @@ __global__ void __launch_bounds__(128) fluid_boundary_split_kernel(double *q, in
     const int64_t p = (pi.dir == 1) ? id / 10 : id % npencil;
     const int item = (int)((pi.dir == 1) ? id % 10 : id / npencil);
     if (p >= npencil || item >= 10) return;
-    const int side = item / 5, k = item % 5;
-    const int mode = side ? mode1 : mode0;
     int64_t base, s;
     int n;
     pi.get(p, base, s, n);
-    double *v0 = q + base;
-    if (mode == IB_BC_OUTFLOW) {
-        if (k == 0) outflow_x(v0, S, s, n, side, pi.dir, depth);
-    } else if (mode == IB_BC_MIRROR || mode == IB_BC_CONST || mode == IB_BC_LINEAR) {
-        sas_x(v0 + k * S, s, n, mode, side, (k >= 2) && (k - 1 == pi.dir), depth);
-    }
-}
-
-static bool mode_ok(int m)
-{
-    return m == IB_BC_CIRCULAR || m == IB_BC_STATIONARY || m == IB_BC_MIRROR || m == IB_BC_CONST ||
-           m == IB_BC_LINEAR || m == IB_BC_OUTFLOW;
+    fill_item(q + base, S, s, n, RowBc{mode0, mode1, depth}, pi.dir, item);
 }
 
 int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int32_t bc[6], int halo, int dir,
@@ -78,7 +65,7 @@ int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int3
     const int m0 = bc[2 * (dir - 1)], m1 = bc[2 * (dir - 1) + 1];
     if (m0 == IB_BC_WALL || m1 == IB_BC_WALL || m0 == IB_BC_FREEBALANCE || m1 == IB_BC_FREEBALANCE)
         return IB_ERROR_NOIMPLEMENT;
-    if (!mode_ok(m0) || !mode_ok(m1)) return IB_ERROR_INVALID_ARGS;
+    if (!row_fill_mode(m0) || !row_fill_mode(m1)) return IB_ERROR_INVALID_ARGS;
     const bool any = !((m0 == IB_BC_CIRCULAR || m0 == IB_BC_STATIONARY) && (m1 == IB_BC_CIRCULAR || m1 == IB_BC_STATIONARY));
     if (!any) return IB_SUCCESSFUL;
     const int n = grid[dir - 1];
@@ -86,8 +73,7 @@ int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int3
     const int64_t N = (int64_t)grid[0] * grid[1] * grid[2];
     const int64_t np = N / n;
     PencilIdx pi{grid[0], grid[1], grid[2], dir};
-    // a side reads at most 2 halo + 1 cells from its own end (linear: 4 from halo on) and writes halo cells
-    if (n >= 3 * halo + 4) {
+    if (row_fill_apart(n, halo)) {
         const int64_t items = 10 * np;
         fluid_boundary_split_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo);
         return check_launch();

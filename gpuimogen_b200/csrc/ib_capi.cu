@@ -13,6 +13,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "ib_bc.cuh"
 #include "ib_internal.cuh"
 #include "ib_sweep_launch.cuh"
 
@@ -161,7 +162,7 @@ double *Scratch::bytes(size_t nbytes)
 }
 
 int launch_sweep(int method, int slope, int precision, int dir, double *q, int64_t slab, const int grid[3],
-                 DevScalar lambda, double gamma, double rho_min, double c_iso, cudaStream_t st, int nsweep)
+                 SweepStep lambda, double gamma, double rho_min, double c_iso, cudaStream_t st, int nsweep)
 {
     if (method == IB_METHOD_HLLC) {
         if (precision == IB_PREC_FP32_FLUX)
@@ -271,11 +272,13 @@ struct StepDt {
 // allows it; Xin-Jin: two launches).
 static int fluid_update_1d(ib_fluid *f, const ib_geometry *geo, int method, int dir, const StepDt &dt, double gamma,
                            double rho_min, double c_iso, const Numerics &nm, cudaStream_t st, int nsweep = 1,
-                           int theta_layout = 0)
+                           int theta_layout = 0, RowBc bc = RowBc{0, 0, 0}, bool *filled = nullptr)
 {
     const int grid[3] = {f->grid.nx, f->grid.ny, f->grid.nz};
     if (grid[dir - 1] < 3) return IB_SUCCESSFUL;  // cudaFluidStep.cu:313
-    const DevScalar lambda = dt.lambda(geo->h[dir - 1]);
+    SweepStep lambda(dt.lambda(geo->h[dir - 1]));
+    lambda.bc = bc;
+    lambda.filled = filled;
     const CylSweep cs = cyl_sweep(geo, f->grid, dir, theta_layout, nm);
     if (method == IB_METHOD_XINJIN) {
         for (int k = 0; k < nsweep; k++) {
@@ -326,6 +329,16 @@ static int fluid_boundary(ib_fluid *f, int dir, cudaStream_t st)
     return IB_SUCCESSFUL;
 }
 
+// The fill after an x sweep where a kernel that owns whole rows may do it (fluid_boundary's work without
+// statics, both ends apart: RowBc of depth 0 otherwise).
+static RowBc row_bc(const ib_fluid *f)
+{
+    const int m0 = f->bc[0], m1 = f->bc[1];
+    if (has_statics(f) || !row_fill_apart(f->grid.nx, f->halo) || !row_fill_mode(m0) || !row_fill_mode(m1)) return RowBc{0, 0, 0};
+    const bool any = (m0 != IB_BC_CIRCULAR && m0 != IB_BC_STATIONARY) || (m1 != IB_BC_CIRCULAR && m1 != IB_BC_STATIONARY);
+    return any ? RowBc{m0, m1, f->halo} : RowBc{0, 0, 0};
+}
+
 // The sweep directions of one fluid step (performFluidUpdate_3D, flux.cu:27-165): sweep index
 // (iteration + 3 [direction > 0]) mod 6 selects a row of the ordering table (flux.cu:46-49).  The
 // backward step's order is the forward one's reversed, so the last sweep of the forward step and
@@ -354,9 +367,11 @@ static int sweep_and_fill(ib_fluid *f, const ib_geometry *geo, int method, int d
 {
     const int ext[3] = {f->grid.nx, f->grid.ny, f->grid.nz};
     if (ext[d - 1] <= 3) return IB_SUCCESSFUL;
-    int rc = fluid_update_1d(f, geo, method, d, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st, nsweep, theta_layout);
+    bool filled = false;
+    const RowBc bc = (d == 1 && nsweep == 1) ? row_bc(f) : RowBc{0, 0, 0};
+    int rc = fluid_update_1d(f, geo, method, d, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st, nsweep, theta_layout, bc, &filled);
     if (rc) return rc;
-    return fluid_boundary(f, d, st);
+    return filled ? IB_SUCCESSFUL : fluid_boundary(f, d, st);
 }
 
 // One fluid step (forward or backward) of one fluid, all three sweeps; 1-D grids take the
@@ -366,9 +381,10 @@ static int fluid_step_one(ib_fluid *f, const ib_geometry *geo, int method, const
 {
     const int ext[3] = {f->grid.nx, f->grid.ny, f->grid.nz};
     if (ext[1] == 1 && ext[2] == 1) {
-        int rc = fluid_update_1d(f, geo, method, 1, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st);
+        bool filled = false;
+        int rc = fluid_update_1d(f, geo, method, 1, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st, 1, 0, row_bc(f), &filled);
         if (rc) return rc;
-        return fluid_boundary(f, 1, st);
+        return filled ? IB_SUCCESSFUL : fluid_boundary(f, 1, st);
     }
     int order[3];
     sweep_order(step_number, sweep_dir, order);

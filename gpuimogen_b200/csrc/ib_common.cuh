@@ -34,6 +34,20 @@ struct DevScalar {
     __device__ __forceinline__ bool off() const { return p && *p == 0.0; }
 };
 
+// The fill of the two ends of every row after an x sweep (boundary modes, cells; depth 0: none), for
+// kernels that own whole rows and can do it before they end.
+struct RowBc {
+    int mode0, mode1, depth;
+};
+
+// What one sweep's launch is given: lambda, and the fill that may go with it.  A launcher whose kernel takes
+// the fill along sets *filled; otherwise the caller launches it.
+struct SweepStep : DevScalar {
+    RowBc bc{0, 0, 0};
+    bool *filled = nullptr;
+    SweepStep(const DevScalar &lambda) : DevScalar(lambda) {}
+};
+
 // ------------------------------------------------------------------------------------------
 // Per-sweep thermodynamic constants (cudaFluidStep.cu:289-311), passed by value.
 // ------------------------------------------------------------------------------------------

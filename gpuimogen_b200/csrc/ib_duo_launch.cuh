@@ -16,10 +16,10 @@ int duo_opt_in(K kern, int &have, size_t bytes)
     return rc;
 }
 
-template <int METHOD, int SLOPE, typename FT, int TT, int NS, bool ODD, int GEO>
+template <int METHOD, int SLOPE, typename FT, int TT, int NS, bool ODD, bool FILL, int GEO>
 int launch_duo_row_t(const SweepArgs &a, const FluidConsts<FT> &c, cudaStream_t st)
 {
-    auto kern = duo_row_kernel<METHOD, SLOPE, FT, TT, NS, ODD, GEO>;
+    auto kern = duo_row_kernel<METHOD, SLOPE, FT, TT, NS, ODD, FILL, GEO>;
     constexpr size_t shm = duo_smem_bytes<FT, TT>();
     static int have = 48 * 1024;
     const int rc = duo_opt_in(kern, have, shm);
@@ -37,17 +37,19 @@ int launch_duo_row_t(const SweepArgs &a, const FluidConsts<FT> &c, cudaStream_t 
 // own.  Against one thread per cell (HLLC FP64, x of 160^3 / 256^3 / 320 x 100 x 64 / 512 x 512 x 64 / 1000 x
 // 100 x 64): 0.142 / 0.535 / 0.078 / 0.607 / 0.312 -> 0.137 / 0.469 / 0.067 / 0.548 / 0.282 ms.
 template <int METHOD, int SLOPE, typename FT, int GEO = CYL_NONE>
-int launch_duo_row(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+int launch_duo_row(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                    cudaStream_t st, int nsweep, double crin = 0.0, double cdr = 0.0)
 {
     const int nx = grid[0];
     if (nx > 1024 || (int64_t)grid[1] * grid[2] >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
-    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, crin, cdr};
+    const bool fill = lambda.filled && lambda.bc.depth > 0 && nsweep == 1;
+    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, crin, cdr, fill ? lambda.bc : RowBc{0, 0, 0}};
+    if (fill) *lambda.filled = true;
     const int T = (nx + 1) / 2;
-    auto go = [&](auto ns, auto odd) {
+    auto go = [&](auto ns, auto odd, auto fl) {
         auto t = [&](auto tt) {
-            return launch_duo_row_t<METHOD, SLOPE, FT, decltype(tt)::value, decltype(ns)::value, decltype(odd)::value, GEO>(
-                a, c, st);
+            return launch_duo_row_t<METHOD, SLOPE, FT, decltype(tt)::value, decltype(ns)::value, decltype(odd)::value,
+                                    decltype(fl)::value, GEO>(a, c, st);
         };
         using std::integral_constant;
         if (T <= 64 || (T > 80 && T <= 128)) return t(integral_constant<int, 128>{});
@@ -58,10 +60,11 @@ int launch_duo_row(double *q, int64_t slab, const int grid[3], DevScalar lambda,
     };
     std::integral_constant<int, 1> one;
     if constexpr (GEO == CYL_NONE) {
-        if (nsweep == 2 && !(nx & 1)) return go(std::integral_constant<int, 2>{}, std::false_type{});
+        if (nsweep == 2 && !(nx & 1)) return go(std::integral_constant<int, 2>{}, std::false_type{}, std::false_type{});
     }
+    if (fill) return (nx & 1) ? go(one, std::true_type{}, std::true_type{}) : go(one, std::false_type{}, std::true_type{});
     for (int k = 0; k < nsweep; k++) {
-        const int rc = (nx & 1) ? go(one, std::true_type{}) : go(one, std::false_type{});
+        const int rc = (nx & 1) ? go(one, std::true_type{}, std::false_type{}) : go(one, std::false_type{}, std::false_type{});
         if (rc) return rc;
     }
     return IB_SUCCESSFUL;
@@ -83,12 +86,12 @@ int launch_duo_pencil_t(const SweepArgs &a, const FluidConsts<FT> &c, int n, cud
 // y and z pencils of up to 512 cells, any nx and alignment: as many neighbouring pencils as 256 threads hold,
 // at most 8
 template <int METHOD, int SLOPE, typename FT, int DIR, int GEO = CYL_NONE>
-int launch_duo_pencil(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+int launch_duo_pencil(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                       cudaStream_t st, int nsweep, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
 {
     const int n = grid[DIR - 1];
     if (n > 512 || (int64_t)grid[0] * grid[1] * grid[2] / n >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
-    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, 0.0, 0.0};
+    SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, 0.0, 0.0, RowBc{0, 0, 0}};
     using std::integral_constant;
     auto go = [&](auto odd) {
         auto t = [&](auto tt, auto cols) {

@@ -52,11 +52,11 @@ Scratch &scratch();
 
 // Launchers (return IB_* status)
 int launch_sweep(int method, int slope, int precision, int dir, double *q, int64_t slab, const int grid[3],
-                 DevScalar lambda, double gamma, double rho_min, double c_iso, cudaStream_t st, int nsweep = 1);
-int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+                 SweepStep lambda, double gamma, double rho_min, double c_iso, cudaStream_t st, int nsweep = 1);
+int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                     double rho_min, cudaStream_t st, const CylSweep *cyl = nullptr);
 // cylindrical geometry: HLL/HLLC radial (x) and theta (y) sweeps; the source terms over dt
-int launch_sweep_cyl(int method, int slope, double *q, int64_t slab, const int grid[3], DevScalar lambda,
+int launch_sweep_cyl(int method, int slope, double *q, int64_t slab, const int grid[3], SweepStep lambda,
                      double gamma, double rho_min, double c_iso, cudaStream_t st, const CylSweep &cs);
 int launch_cyl_source(double *q, int64_t slab, const int grid[3], double dr, double r_inner, DevScalar dt,
                       cudaStream_t st);

@@ -305,6 +305,7 @@ struct SweepArgs {
     int nx, ny, nz;
     DevScalar lambda;
     double crin, cdr;  // radial sweeps (GEO == CYL_RADIAL): radius of cell 0's centre, radial cell size
+    RowBc bc;          // x rows: the fill of the rows' ends after the sweep
 };
 
 // ------------------------------------------------------------------------------------------
@@ -313,7 +314,7 @@ struct SweepArgs {
 // in flight (double-buffered U0 tiles, one mbarrier each), so the next block's 5 slabs arrive
 // while this one is computed; results leave through a TMA store from a third tile.  The tile
 // layout is the TMA box's: [memory slab k][cell i][column] with the column fastest.  The
-// arithmetic per cell is the row kernel's.
+// arithmetic per cell is the pencil-pair kernel's.
 // Dynamic shared memory: 3 tiles of 5*W*n doubles (each rounded to 128 B) + 2 planes of
 // 5*W*n elements of FT.
 // ------------------------------------------------------------------------------------------
@@ -540,15 +541,13 @@ __global__ void __launch_bounds__(512, (CPT == 1) ? 2 : 1)
 }
 
 // ------------------------------------------------------------------------------------------
-// Pencil-pair kernel (y and z sweeps, pencils up to 256 cells or of 512, x even): the row kernel's
-// layout applied to a TMA box.  One CTA per block of two adjacent pencils, n threads (one cell
-// each, as the x row kernel), four CTAs per SM (two of 512 threads for 512-cell pencils); thread
-// 0 loads the block's 5-slab box (2 x n x 5
-// doubles, 16-byte rows) with one TMA copy, the CTA sweeps the two pencils one after the other
-// through the row kernel's phases (two shared-memory planes that swap roles between the stages,
-// the SSPRK sum u1 + u0 in a third), writes each pencil's result over its own column of the box
-// and leaves by one TMA store.  No persistent pipeline: the other CTAs on the SM hide a block's
-// load, as they hide the row kernel's.
+// Pencil-pair kernel (y and z sweeps, pencils up to 256 cells or of 512, x even): one CTA per block of two
+// adjacent pencils, n threads (one cell each), four CTAs per SM (two of 512 threads for 512-cell pencils);
+// thread 0 loads the block's 5-slab box (2 x n x 5 doubles, 16-byte rows) with one TMA copy, the CTA sweeps
+// the two pencils one after the other (primitives, limited faces, fluxes and update through two
+// shared-memory planes that swap roles between the stages, the SSPRK sum u1 + u0 in a third), writes each
+// pencil's result over its own column of the box and leaves by one TMA store.  No persistent pipeline: the
+// other CTAs on the SM hide a block's load.
 // Dynamic shared memory: the box (pipe_tile_bytes(n, WC)), 2 planes of 5 NP elements of FT and
 // 5 NP doubles for the SSPRK sum (NP: the pencil length, or PADN).
 // ------------------------------------------------------------------------------------------
@@ -559,7 +558,10 @@ __host__ __device__ __forceinline__ size_t pair_smem_bytes(int n, int ftsize, in
 }
 
 // WC: pencils per box (2; 4 for z sweeps of x-y planes above 1 MB, whose 16-byte rows a plane
-// apart the memory system serves poorly: 32-byte rows, three CTAs per SM)
+// apart the memory system serves poorly: 32-byte rows, three CTAs per SM; and for the FP32 flux's 512-cell
+// pencils).  In a box of 4 a thread's accesses would meet 8-way bank conflicts: its tensor map swaps the 16-byte
+// halves of every other 128 bytes (4-way, as in a box of 2), and the SSPRK sum waits in the pencil's own column
+// of the box, which holds nothing else meanwhile.
 // GEO == CYL_THETA_DIV / CYL_THETA_LAM: the theta sweep of cylindrical geometry (y = theta), the
 // flux difference divided by the pencil's radius or lambda divided by it first (cyl_dflux); the
 // radius of the pencil at radial index x and z index z is theta_radius(cyl, x, z).  FP64, one sweep.
@@ -587,15 +589,19 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                   s3 = slot_of<METHOD, DIR>(3), s4 = slot_of<METHOD, DIR>(4);
     const int slots[5] = {s0, s1, s2, s3, s4};
     const int64_t b = blockIdx.x;
+    // a compile-time length leaves the registers to keep the cell's primitives across the first barrier rather
+    // than read them back (256^3 y: 0.555 -> 0.534 ms; at run-time lengths it spills: 160^3 0.158 -> 0.162)
+    constexpr bool keepw = NFIX != 0;
     const int i = threadIdx.x;
     const bool act = i < n;
     const int il = (i == 0) ? n - 1 : i - 1, ir = (i == n - 1) ? 0 : i + 1;
     if (a.lambda.off()) return;  // a device timestep of 0: after the end time
     const double lambda = a.lambda.get();
     const bool leader = threadIdx.x == 0;
-    // the box's TMA copy needs a 128-byte aligned destination: a CTA whose tile is not aligned
-    // leaves its block undone and sets bit 2 of the wait flag instead of issuing the copy
-    if (smem_u32(T) & 127u) {
+    // the box's TMA copy needs a 128-byte aligned destination (256 for the swizzled 4-pencil boxes): a CTA
+    // whose tile is not aligned leaves its block undone and sets bit 2 of the wait flag instead of issuing
+    // the copy
+    if (smem_u32(T) & (WC == 4 ? 255u : 127u)) {
         if (leader) atomicOr(a.err, 2u);
         return;
     }
@@ -640,8 +646,9 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                 double *u = (stage == 0) ? u0 : u1;
                 FT *PX = (stage == 0) ? SA : SB;  // primitives, then fluxes
                 FT *PY = (stage == 0) ? SB : SA;  // left faces
+                V5<FT> w;
                 if (act) {
-                    V5<FT> w = stage_prims<METHOD, DIR, FT>(u, c);
+                    w = stage_prims<METHOD, DIR, FT>(u, c);
 #pragma unroll
                     for (int k = 0; k < 5; k++) PX[k * NP + i] = w.a[k];
                     if (stage == 1) {
@@ -651,10 +658,10 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                 }
                 __syncthreads();
                 if (act) {
-                    V5<FT> w, dl, dr, L;
+                    V5<FT> dl, dr, L;
 #pragma unroll
                     for (int k = 0; k < 5; k++) {
-                        w.a[k] = PX[k * NP + i];
+                        if (!keepw) w.a[k] = PX[k * NP + i];
                         dl.a[k] = w.a[k] - PX[k * NP + il];
                         dr.a[k] = PX[k * NP + ir] - w.a[k];
                     }

@@ -2,9 +2,11 @@
 #include "ib_sweep_launch.cuh"
 
 namespace ib {
-int launch_hllc64(int slope, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_hllc64(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
               double rho_min, double c_iso, cudaStream_t st, int nsweep)
 {
-    return launch_sweep_slope<IB_METHOD_HLLC, double>(slope, dir, q, slab, grid, lambda, gamma, rho_min, c_iso, st, nsweep);
+    if (slope != IB_SLOPE_OSPRE && slope != IB_SLOPE_MC && slope != IB_SLOPE_VANLEER && slope != IB_SLOPE_ZERO)
+        return launch_hllc64_b(slope, dir, q, slab, grid, lambda, gamma, rho_min, c_iso, st, nsweep);
+    return launch_sweep_slope<IB_METHOD_HLLC, double, 0>(slope, dir, q, slab, grid, lambda, gamma, rho_min, c_iso, st, nsweep);
 }
 }  // namespace ib

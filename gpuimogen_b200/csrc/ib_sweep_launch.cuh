@@ -12,7 +12,7 @@ namespace ib {
 
 // Tile-march launch: W pencils per CTA, chunks of ~TARGET cells, every chunk >= 8 cells.
 template <int METHOD, int SLOPE, typename FT, int DIR, int W, int GEO = CYL_NONE>
-int launch_tile_dw(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+int launch_tile_dw(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                    cudaStream_t st, int target, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
 {
     const int n = grid[DIR - 1];
@@ -51,7 +51,7 @@ int launch_tile_dw(double *q, int64_t slab, const int grid[3], DevScalar lambda,
 // G > 1 selects sweep_pipe_wide_kernel: blocks of W*G columns (one TMA box), computed W at a time,
 // results stored from the input tile; pencils up to 256 cells, y/z sweeps only.
 template <int METHOD, int SLOPE, typename FT, int DIR, int W, int CPT, int NFIX = 0, int G = 1>
-int launch_pipe(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c, cudaStream_t st,
+int launch_pipe(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c, cudaStream_t st,
                 int nsweep)
 {
     const int nx = grid[0], ny = grid[1], nz = grid[2];
@@ -126,13 +126,13 @@ int launch_pipe(double *q, int64_t slab, const int grid[3], DevScalar lambda, co
 // IB_ERROR_NOIMPLEMENT (caller falls back) otherwise.  GEO: cylindrical theta pencils (y, one
 // sweep), with their radius rule in cyl.
 template <int METHOD, int SLOPE, typename FT, int DIR, int NFIX = 0, int WC = 2, int GEO = CYL_NONE, int PADN = 0>
-int launch_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c, cudaStream_t st,
+int launch_pair(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c, cudaStream_t st,
                 int nsweep, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
 {
     static_assert(PADN == 0 || NFIX == 0, "a fixed plane stride for pencils of a run-time length");
     static_assert(GEO == CYL_NONE || DIR == 2, "theta pencils run along y");
     if (GEO != CYL_NONE && nsweep != 1) return IB_ERROR_NOIMPLEMENT;
-    static_assert(DIR != 1, "x rows take the row kernel");
+    static_assert(DIR != 1, "x rows take the two-cell row kernel");
     static_assert(WC == 2 || (WC == 4 && (NFIX != 512 || sizeof(FT) == 4)), "boxes of 2 pencils, or 4 (512 cells: FP32 flux)");
     const int nx = grid[0], ny = grid[1], nz = grid[2];
     const int n = grid[DIR - 1];
@@ -179,7 +179,7 @@ int launch_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, co
 // chunk boundaries to scratch memory.  Returns IB_ERROR_NOIMPLEMENT (caller falls back) when the
 // grid does not meet TMA's rules: x rows of even length; y/z with W dividing nx.
 template <int METHOD, int SLOPE, typename FT, int DIR, int W, int R>
-int launch_chunk(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c, cudaStream_t st)
+int launch_chunk(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c, cudaStream_t st)
 {
     constexpr int L = R - 8;
     const int nx = grid[0], ny = grid[1], nz = grid[2];
@@ -253,7 +253,7 @@ int launch_chunk(double *q, int64_t slab, const int grid[3], DevScalar lambda, c
 }
 
 template <int METHOD, int SLOPE, typename FT>
-int launch_tile_t(int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+int launch_tile_t(int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                   cudaStream_t st)
 {
     if (dir == 1) return launch_tile_dw<METHOD, SLOPE, FT, 1, 1>(q, slab, grid, lambda, c, st, 248);
@@ -265,7 +265,7 @@ int launch_tile_t(int dir, double *q, int64_t slab, const int grid[3], DevScalar
 // sweeps in the middle of an iteration).  The row and pipeline kernels apply both to a block
 // while it is on chip; the chunked pipeline and the tile kernel are launched once per sweep.
 template <int METHOD, int SLOPE, typename FT>
-int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<FT> &c,
+int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                    cudaStream_t st, int nsweep = 1)
 {
     const int nx = grid[0], ny = grid[1], nz = grid[2];
@@ -299,7 +299,6 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScala
         // persistent pipeline, which remains for other lengths when the pair kernel declines
         // (pencils shorter than pair_min_cells() leave most of a pencil-pair CTA idle: pipeline)
         const bool pair = n >= pair_min_cells();
-        constexpr bool pair512 = true;
         // z of x-y planes above 1 MB, FP64: 4-pencil boxes through the pencil-pair kernel (512 x 512
         // x 256: z 3.96 -> 3.58 ms); FP32 flux keeps its 8-column wide blocks (2.43 ms against 2.77
         // for the 4-pencil boxes)
@@ -369,7 +368,14 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScala
             }
             if (rc == IB_ERROR_NOIMPLEMENT) rc = launch_pipe<METHOD, SLOPE, FT, 3, 4, 2>(q, slab, grid, lambda, c, st, nsweep);
         } else if (n == 512) {
-            if (pair512) {
+            // FP32 flux: 4-pencil boxes.  Its sweeps wait for the copies, and a TMA copy costs by the row: 32-byte
+            // rows halve them (512 x 512 x 256 y: 2.07 -> 1.88 ms; 64 x 256 x 512 z: 0.272 -> 0.248).  At 256 and 128
+            // cells the fewer CTAs that fit beside the larger boxes cost as much (256^3 y: 0.387 -> 0.404 ms).
+            if constexpr (sizeof(FT) == 4) {
+                if (dir == 2) rc = launch_pair<METHOD, SLOPE, FT, 2, 512, 4>(q, slab, grid, lambda, c, st, nsweep);
+                else rc = launch_pair<METHOD, SLOPE, FT, 3, 512, 4>(q, slab, grid, lambda, c, st, nsweep);
+            }
+            if (rc == IB_ERROR_NOIMPLEMENT) {
                 if (dir == 2) rc = launch_pair<METHOD, SLOPE, FT, 2, 512>(q, slab, grid, lambda, c, st, nsweep);
                 else rc = launch_pair<METHOD, SLOPE, FT, 3, 512>(q, slab, grid, lambda, c, st, nsweep);
             }
@@ -420,28 +426,45 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], DevScala
     return IB_SUCCESSFUL;
 }
 
-template <int METHOD, typename FT>
-int launch_sweep_slope(int slope, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+// HALF: which limiters a translation unit instantiates (0: Ospre, MC, van Leer and zero; 1: the others), so
+// that the two halves of a method compile side by side
+template <int METHOD, typename FT, int HALF>
+int launch_sweep_slope(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                        double rho_min, double c_iso, cudaStream_t st, int nsweep)
 {
     FluidConsts<FT> c = make_consts<FT>(gamma, rho_min, c_iso);
     switch (slope) {
-    case IB_SLOPE_OSPRE: return launch_sweep_t<METHOD, IB_SLOPE_OSPRE, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_MC: return launch_sweep_t<METHOD, IB_SLOPE_MC, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_VANLEER: return launch_sweep_t<METHOD, IB_SLOPE_VANLEER, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_MINMOD: return launch_sweep_t<METHOD, IB_SLOPE_MINMOD, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_SUPERBEE: return launch_sweep_t<METHOD, IB_SLOPE_SUPERBEE, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_VANALBADA: return launch_sweep_t<METHOD, IB_SLOPE_VANALBADA, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    case IB_SLOPE_ZERO: return launch_sweep_t<METHOD, IB_SLOPE_ZERO, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
-    default: return IB_ERROR_INVALID_ARGS;
+    case IB_SLOPE_OSPRE:
+        if constexpr (HALF == 0) return launch_sweep_t<METHOD, IB_SLOPE_OSPRE, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_MC:
+        if constexpr (HALF == 0) return launch_sweep_t<METHOD, IB_SLOPE_MC, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_VANLEER:
+        if constexpr (HALF == 0) return launch_sweep_t<METHOD, IB_SLOPE_VANLEER, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_MINMOD:
+        if constexpr (HALF == 1) return launch_sweep_t<METHOD, IB_SLOPE_MINMOD, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_SUPERBEE:
+        if constexpr (HALF == 1) return launch_sweep_t<METHOD, IB_SLOPE_SUPERBEE, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_VANALBADA:
+        if constexpr (HALF == 1) return launch_sweep_t<METHOD, IB_SLOPE_VANALBADA, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    case IB_SLOPE_ZERO:
+        if constexpr (HALF == 0) return launch_sweep_t<METHOD, IB_SLOPE_ZERO, FT>(dir, q, slab, grid, lambda, c, st, nsweep);
+        break;
+    default: break;
     }
+    return IB_ERROR_INVALID_ARGS;
 }
 
-// Cylindrical sweeps, FP64: radial x rows of up to 512 cells in the row kernel and theta y pencils
-// of up to 256 cells (x even) in the pencil-pair kernel, each with the geometry's update; other
-// shapes in the tile kernel with the same update
+// Cylindrical sweeps, FP64: radial x rows of up to 1024 cells in the two-cell row kernel, theta y pencils
+// of up to 256 cells (x even) in the pencil-pair kernel and other theta pencils of up to 512 in the two-cell
+// kernel, each with the geometry's update; longer ones in the tile kernel with the same update
 template <int METHOD, int SLOPE>
-int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], DevScalar lambda, const FluidConsts<double> &c,
+int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<double> &c,
                        cudaStream_t st, const CylSweep &cs)
 {
     static const bool fast_env = [] {
@@ -482,7 +505,7 @@ int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], DevScalar lam
 }
 
 template <int METHOD>
-int launch_sweep_cyl_slope(int slope, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_sweep_cyl_slope(int slope, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                            double rho_min, double c_iso, cudaStream_t st, const CylSweep &cs)
 {
     FluidConsts<double> c = make_consts<double>(gamma, rho_min, c_iso);
@@ -498,11 +521,20 @@ int launch_sweep_cyl_slope(int slope, double *q, int64_t slab, const int grid[3]
     }
 }
 
-int launch_hllc64(int slope, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_hllc64(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                   double rho_min, double c_iso, cudaStream_t st, int nsweep);
-int launch_hllc32(int slope, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_hllc32(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                   double rho_min, double c_iso, cudaStream_t st, int nsweep);
-int launch_hll64(int slope, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_hll64(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                  double rho_min, double c_iso, cudaStream_t st, int nsweep);
+
+// the other half of the limiters (ib_sweep_*_b.cu)
+int launch_hllc64_b(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
+                  double rho_min, double c_iso, cudaStream_t st, int nsweep);
+int launch_hllc32_b(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
+                  double rho_min, double c_iso, cudaStream_t st, int nsweep);
+int launch_hll64_b(int slope, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
+                 double rho_min, double c_iso, cudaStream_t st, int nsweep);
+
 
 }  // namespace ib

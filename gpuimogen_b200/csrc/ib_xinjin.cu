@@ -8,6 +8,7 @@
 // and runs both stages, so a sweep is one launch with one read and one write of the state.
 #include <cstdlib>
 
+#include "ib_bc.cuh"
 #include "ib_internal.cuh"
 
 namespace ib {
@@ -109,7 +110,7 @@ __device__ __forceinline__ void flux_limit_pair(double A1, double B1, double A2,
 template <int FLIM, int W, int CPT, bool RELOAD, int GEO = CYL_NONE>
 __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab, int nx, int ny, int nz, int dir,
                                                          DevScalar lam_in, double gamma, double minmass, double mintemp,
-                                                         CylPencil cyl)
+                                                         CylPencil cyl, RowBc bc)
 {
     if (lam_in.off()) return;  // a device timestep of 0: after the end time
     const double lambda = lam_in.get();
@@ -291,6 +292,10 @@ __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab
             for (int k = 0; k < 5; k++) q[k * slab + base + i * stride] = u1[m][k];
         }
     }
+    if (W == 1 && bc.depth > 0) {  // x rows: the row's ends, from the stored row
+        __syncthreads();
+        if (threadIdx.x < 10) fill_item(q + base, slab, 1, n, bc, 1, threadIdx.x);
+    }
 }
 
 // y/z sweeps of pencils of up to 256 cells, or of 512: the pencil-pair kernel's structure.  One TMA
@@ -308,6 +313,7 @@ struct XjPairArgs {
     unsigned int *err;
     uint32_t spin;
     CylPencil cyl;  // cylindrical theta pencils (GEO): the radius rule
+    RowBc bc;       // x rows: the fill of the row's ends after the sweep
 };
 
 __host__ __device__ __forceinline__ size_t xj_box_bytes(int n, int wc) { return ((size_t)40 * n * wc + 127) / 128 * 128; }
@@ -468,6 +474,10 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
             for (int k = 0; k < 5; k++) T[TI(k)] = u1[k];
         }
     }
+    if (DIR == 1 && a.bc.depth > 0) {  // the row's ends, in the box
+        __syncthreads();
+        if (threadIdx.x < 10) fill_item(T, n, 1, n, a.bc, 1, threadIdx.x);
+    }
     fence_proxy_async_smem();
     __syncthreads();
     if (leader) {
@@ -482,7 +492,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 // the kernel's sizes do not hold: nx a multiple of WC, 16-byte aligned base and slab pitch, pencils
 // of up to 256 cells or of 512.
 template <int FLIM, int DIR, int NFIX, int WC, int GEO = CYL_NONE, int PADN = 0>
-static int launch_xj_pair(double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma, double rho_min,
+static int launch_xj_pair(double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma, double rho_min,
                           double mintemp, cudaStream_t st, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
 {
     const int nx = grid[0], ny = grid[1], nz = grid[2];
@@ -531,14 +541,16 @@ static int launch_xj_pair(double *q, int64_t slab, const int grid[3], DevScalar 
         if (rc) return rc;
         attr_bytes = (int)shm;
     }
-    XjPairArgs a{n, npw, lambda, gamma, rho_min, mintemp, err, tile_wait_limit(), cyl};
+    const bool fill = DIR == 1 && lambda.filled && lambda.bc.depth > 0;
+    if (fill) *lambda.filled = true;
+    XjPairArgs a{n, npw, lambda, gamma, rho_min, mintemp, err, tile_wait_limit(), cyl, fill ? lambda.bc : RowBc{0, 0, 0}};
     xj_pair_kernel<FLIM, DIR, NFIX, WC, GEO, PADN><<<(unsigned)nblocks, nt, shm, st>>>(tm, a);
     return check_launch();
 }
 
 // Cylindrical theta pencils (y) of up to 256 cells in the pencil-box kernel
 template <int FLIM>
-static int launch_xj_pair_theta(int geo, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+static int launch_xj_pair_theta(int geo, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                                 double rho_min, double mintemp, cudaStream_t st, const CylPencil &cyl)
 {
     const int n = grid[1];
@@ -553,7 +565,7 @@ static int launch_xj_pair_theta(int geo, double *q, int64_t slab, const int grid
 }
 
 template <int FLIM>
-static int launch_xj_pair_dir(int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+static int launch_xj_pair_dir(int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                               double rho_min, double mintemp, cudaStream_t st)
 {
     const int n = grid[dir - 1];
@@ -585,7 +597,7 @@ static int launch_xj_pair_dir(int dir, double *q, int64_t slab, const int grid[3
     return launch_xj_pair<FLIM, 3, 0, 2>(q, slab, grid, lambda, gamma, rho_min, mintemp, st);
 }
 
-int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3], DevScalar lambda, double gamma,
+int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3], SweepStep lambda, double gamma,
                     double rho_min, cudaStream_t st, const CylSweep *cyl)
 {
     const int geo = cyl ? cyl->kind : CYL_NONE;
@@ -652,6 +664,9 @@ int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3
     const size_t shm_cap = 227 * 1024 - 2048;  // opt-in limit minus the kernel's static shared memory
     if (shm > shm_cap) return IB_ERROR_NOIMPLEMENT;
     const unsigned nblk = (unsigned)(np / W);
+    const bool fill = dir == 1 && lambda.filled && lambda.bc.depth > 0;
+    const RowBc bc = fill ? lambda.bc : RowBc{0, 0, 0};
+    if (fill) *lambda.filled = true;
 #define IB_XJ_G(F, WW, CC, RR, GG)                                                                            \
     do {                                                                                                      \
         static bool attr_set = false;                                                                         \
@@ -662,7 +677,7 @@ int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3
             attr_set = true;                                                                                  \
         }                                                                                                     \
         xj_pencil_kernel<F, WW, CC, RR, GG><<<nblk, nt, shm, st>>>(q, slab, grid[0], grid[1], grid[2], dir,   \
-                                                                   lambda, gamma, rho_min, mintemp, cp);      \
+                                                                   lambda, gamma, rho_min, mintemp, cp, bc);  \
     } while (0)
 #define IB_XJ(F, WW, CC, RR) IB_XJ_G(F, WW, CC, RR, CYL_NONE)
 #define IB_XJ_W(F)                                                                    \
