@@ -27,6 +27,7 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 # the longest compiles first
 SOURCES = [
     "ib_sweep_cyl.cu",
+    "ib_sweep_cyl_hll.cu",
     "ib_sweep_hll64.cu",
     "ib_sweep_hll64_b.cu",
     "ib_sweep_hllc64.cu",
