@@ -260,8 +260,16 @@ struct V5 {
     FT a[5];
 };
 
+// A product that later arithmetic takes rounded (RN): the compiler may otherwise contract it into a sum where both
+// stand in one thread, and not where the product comes from another thread.  Kernels whose results are not to
+// depend on which cell a thread holds ask for it.
+template <bool RN>
+__device__ __forceinline__ double product(double a, double b) { return RN ? __dmul_rn(a, b) : a * b; }
+template <bool RN>
+__device__ __forceinline__ float product(float a, float b) { return RN ? __fmul_rn(a, b) : a * b; }
+
 // Conserved -> HLLC primitives (cudaFluidStep.cu:1200-1237).  u: [rho, E, p_n, p_t1, p_t2].
-template <typename FT>
+template <typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 {
 #ifdef IB_STRICT_ARITH
@@ -270,9 +278,9 @@ __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
     FT F = rcp_fast(A);
 #endif
     B -= (FT).5 * (C * C + D * D + E * E) * F;
-    C *= F;
-    D *= F;
-    E *= F;
+    C = product<RN>(C, F);
+    D = product<RN>(D, F);
+    E = product<RN>(E, F);
     V5<FT> w;
     w.a[0] = A; w.a[1] = B; w.a[2] = C; w.a[3] = D; w.a[4] = E;
     return w;
@@ -300,7 +308,7 @@ __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT
 // HLLC flux through the face between the right face state of the left cell (l) and the left
 // face state of the right cell (r).  (cudaFluidStep.cu:1318-1432)
 #ifdef IB_STRICT_ARITH
-template <typename FT>
+template <typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
     const FT rhoL = l.a[0], PL = l.a[1], vxL = l.a[2], vyL = l.a[3], vzL = l.a[4];
@@ -374,7 +382,7 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
 // The same flux with fewer and shorter dependent chains: reciprocals and roots of ib_fast.cuh, and the
 // star (or outer) state computed once, for the side that the contact speed selects, instead of in
 // divergent branches.
-template <typename FT>
+template <typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
     const FT rhoL = l.a[0], PL = l.a[1], vL = l.a[2];
@@ -391,22 +399,22 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     const FT h = c.govergm1 * P;
     V5<FT> f;
     if (left ? sl > 0 : !(sr > 0)) {  // the outer state: no wave crosses the face
-        const FT m = rho * v;
+        const FT m = product<RN>(rho, v);
         f.a[0] = m;
-        f.a[1] = v * (ke * rho + h);
+        f.a[1] = product<RN>(v, ke * rho + h);
         f.a[2] = m * v + P;
-        f.a[3] = m * t1;
-        f.a[4] = m * t2;
+        f.a[3] = product<RN>(m, t1);
+        f.a[4] = product<RN>(m, t2);
     } else {
         const FT S = left ? sl : sr;
         const FT D = (left ? A : B) * rcp_fast(S - sm);
-        const FT m = D * sm;
+        const FT m = product<RN>(D, sm);
         const FT q = S * (sm - v);
         f.a[0] = m;
-        f.a[1] = m * (h * (left ? irL : irR) + ke + q);
+        f.a[1] = product<RN>(m, h * (left ? irL : irR) + ke + q);
         f.a[2] = P + D * (q + sm * v);
-        f.a[3] = m * t1;
-        f.a[4] = m * t2;
+        f.a[3] = product<RN>(m, t1);
+        f.a[4] = product<RN>(m, t2);
     }
     return f;
 }

@@ -39,7 +39,7 @@ struct DuoGeo {
 // NS sweeps of the cells (ua, ub) of this thread, in place.  planes: 15 TT values of FT; SS: 10 TT
 // doubles, where u1 + u0 of the SSPRK average waits through the second stage.  All threads of the CTA
 // call it.
-template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO>
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO, bool RN = false>
 __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], bool act, const DuoPos &p, FT *planes,
                                            double *SS, double lambda, const FluidConsts<FT> &c, const DuoGeo &g)
 {
@@ -50,8 +50,8 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
         FT *P = planes + (s % 3) * 5 * TT, *Q = planes + ((s + 1) % 3) * 5 * TT, *R = planes + ((s + 2) % 3) * 5 * TT;
         V5<FT> wa, wb;
         if (act) {
-            wa = stage_prims<METHOD, DIR, FT>(second ? va : ua, c);  // HLL floors its argument
-            wb = stage_prims<METHOD, DIR, FT>(second ? vb : ub, c);
+            wa = stage_prims<METHOD, DIR, FT, RN>(second ? va : ua, c);  // HLL floors its argument
+            wb = stage_prims<METHOD, DIR, FT, RN>(second ? vb : ub, c);
 #pragma unroll
             for (int k = 0; k < 5; k++) {
                 P[k * TT + p.own] = wa.a[k];
@@ -80,10 +80,10 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
                 const FT ha = slope_limit<SLOPE, FT>(dl, dm), hb = slope_limit<SLOPE, FT>(dm, dr);
                 FT la;
                 if (METHOD == IB_METHOD_HLLC && k == 1) {  // internal energy to pressure
-                    la = c.gm1 * (wa.a[k] - ha);
-                    ra.a[k] = c.gm1 * (wa.a[k] + ha);
-                    lb.a[k] = c.gm1 * (wb.a[k] - hb);
-                    rb.a[k] = c.gm1 * (wb.a[k] + hb);
+                    la = product<RN>(c.gm1, wa.a[k] - ha);
+                    ra.a[k] = product<RN>(c.gm1, wa.a[k] + ha);
+                    lb.a[k] = product<RN>(c.gm1, wb.a[k] - hb);
+                    rb.a[k] = product<RN>(c.gm1, wb.a[k] + hb);
                     if (GEO == CYL_RADIAL) {
                         pa = (double)la + (double)ra.a[k];
                         pb = (double)lb.a[k] + (double)rb.a[k];
@@ -96,7 +96,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
                 }
                 R[k * TT + p.own] = la;
             }
-            fm = stage_flux<METHOD, FT>(c, ra, lb);
+            fm = stage_flux<METHOD, FT, RN>(c, ra, lb);
         }
         __syncthreads();
         V5<FT> fb;
@@ -104,7 +104,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
             V5<FT> lr;
 #pragma unroll
             for (int k = 0; k < 5; k++) lr.a[k] = R[k * TT + p.right];
-            fb = stage_flux<METHOD, FT>(c, rb, lr);
+            fb = stage_flux<METHOD, FT, RN>(c, rb, lr);
 #pragma unroll
             for (int k = 0; k < 5; k++) P[k * TT + p.own] = (ODD && p.ghost) ? fm.a[k] : fb.a[k];
         }

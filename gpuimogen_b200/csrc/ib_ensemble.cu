@@ -8,13 +8,13 @@
 // (TimeManager.m:270-277).  Here a CTA takes a problem from a device work counter and runs it to
 // its end without leaving the kernel; the problem's cells stay in L2 between sweeps (one
 // problem is at most a few hundred KB), so the launch reads and writes HBM about once per cell.
-// The per-cell arithmetic is the library's sweep arithmetic (stage_prims / stage_faces /
-// stage_flux in ens_sweep), CFL and boundary code, so every problem's result equals running it
-// alone through the library's 1-D entry points.
+// The per-cell arithmetic is the library's sweep arithmetic (stage_prims / stage_faces / stage_flux in
+// ens_sweep, the two-cell stages of ib_duo.cuh in ens_sweep_two), CFL and boundary code, so every problem's
+// result equals running it alone through the library's 1-D entry points.
 #include "ib_bc.cuh"
 #include "ib_cfl.cuh"
 #include "ib_internal.cuh"
-#include "ib_sweep.cuh"
+#include "ib_duo.cuh"
 
 namespace ib {
 
@@ -188,20 +188,83 @@ __device__ __forceinline__ void ens_sweep(double *qb, int64_t S, int n, int nchu
     __syncthreads();
 }
 
-// Three CTAs of 256 threads per SM (80 registers) rather than four: at 64 registers a thread's
-// state of two stages spills; 512-thread CTAs keep two per SM, one would idle half the SM.
-template <int METHOD, int SLOPE, typename FT, int NT>
-__global__ void __launch_bounds__(NT, NT == 512 ? 2 : 768 / NT) ensemble_kernel(EnsArgs a, FluidConsts<FT> c)
+// The same sweep with two rows a thread: thread t computes rows 2t and 2t + 1 of a chunk (ib_duo.cuh; the edge
+// rows' results are not used), TT threads for chunks of up to 2 TT - 8 cells.  Products are rounded (RN), so that
+// a cell's result does not depend on which of the two rows it is, and with it not on the chunk length.
+template <int METHOD, int SLOPE, typename FT, int TT>
+__device__ __forceinline__ void ens_sweep_two(double *qb, int64_t S, int n, int nchunks, double lambda,
+                                          const FluidConsts<FT> &c, FT *planes, double *SS, double *pend, double *first)
+{
+    const int t = threadIdx.x;
+    const bool single = (nchunks == 1);
+    DuoPos p;
+    p.own = t;
+    p.left = (t > 0) ? t - 1 : t;
+    p.right = (t < TT - 1) ? t + 1 : t;
+    p.first = p.ghost = false;
+    for (int ch = 0; ch < nchunks; ch++) {
+        const int cb = (int)((int64_t)ch * n / nchunks);
+        const int len = (int)((int64_t)(ch + 1) * n / nchunks) - cb;
+        const int tr = len + 8;
+        auto fetch = [&](int i, double (&u)[5]) {
+            const int cell = mod_n(cb - 4 + i, n);
+#pragma unroll
+            for (int k = 0; k < 5; k++) u[k] = (i < tr) ? qb[(int64_t)k * S + cell] : 1.0;
+        };
+        double ua[5], ub[5];
+        fetch(2 * t, ua);
+        fetch(2 * t + 1, ub);
+        __syncthreads();  // this chunk has loaded the original state of its halo (and is done with the planes)
+        if (ch > 0 && t < 4) {
+#pragma unroll
+            for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb - 4 + t] = pend[k * 4 + t];
+        }
+        duo_sweeps<METHOD, SLOPE, FT, 1, TT, 1, false, CYL_NONE, true>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
+        auto store = [&](int i, const double (&out)[5]) {
+            const int m = i - 4;  // output cell cb + m
+            if (m < 0 || m >= len) return;
+            if (!single && ch == 0 && m < 4) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) first[k * 4 + m] = out[k];
+            } else if (!single && m >= len - 4) {
+#pragma unroll
+                for (int k = 0; k < 5; k++) pend[k * 4 + m - (len - 4)] = out[k];
+            } else {
+#pragma unroll
+                for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb + m] = out[k];
+            }
+        };
+        store(2 * t, ua);
+        store(2 * t + 1, ub);
+    }
+    __syncthreads();
+    if (!single && t < 4) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            qb[(int64_t)k * S + n - 4 + t] = pend[k * 4 + t];
+            qb[(int64_t)k * S + t] = first[k * 4 + t];
+        }
+    }
+    __syncthreads();
+}
+
+// One row a thread: three CTAs of 256 threads per SM (80 registers) rather than four: at 64 registers a
+// thread's state of two stages spills; 512-thread CTAs keep two per SM, one would idle half the SM.
+// TWO: two rows a thread, CTAs of half the launch shape's `threads`, per SM as for the row kernel
+// (duo_min_blocks): five of 128 threads at 96 registers for the default shape.
+template <int METHOD, int SLOPE, typename FT, int NT, bool TWO>
+__global__ void __launch_bounds__(TWO ? NT / 2 : NT,
+                                  TWO ? (NT == 128 ? 2 * duo_min_blocks<FT>(128) : duo_min_blocks<FT>(NT / 2))
+                                      : (NT == 512 ? 2 : 768 / NT)) ensemble_kernel(EnsArgs a, FluidConsts<FT> c)
 {
     extern __shared__ __align__(16) double tsm[];
     __shared__ int s_prob;
-    __shared__ double s_red[NT / 32];
+    constexpr int TT = TWO ? NT / 2 : NT;
+    __shared__ double s_red[TT / 32];
     __shared__ double s_dt;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     double *pend = tsm;        // [5][4]
     double *first = tsm + 20;  // [5][4]
-    FT *SA = reinterpret_cast<FT *>(tsm + 40);  // [5][lcap]
-    FT *SB = SA + 5 * a.lcap;
     for (;;) {
         if (tid == 0) {
             const unsigned k = atomicAdd(a.counter, 1u);
@@ -229,7 +292,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 768 / NT) ensemble_kernel(
         while (it < a.itermax && t < a.t_end * (1 - 1e-14)) {
             // tau: NaN-ignoring minimum of the signal-crossing times, halved for HLL/HLLC
             double tmin = 1e37;
-            for (int x = tid; x < n; x += NT) {
+            for (int x = tid; x < n; x += TT) {
                 const double rho = qb[x], px = qb[x + 2 * a.S];
                 const double cs = soundspeed_cell(rho, qb[x + a.S], px, qb[x + 3 * a.S], qb[x + 4 * a.S], a.gg1);
                 tmin = min_keep(tmin, cfl_cell<1, false>(rho, px, 0.0, 0.0, cs, h, h, h, h));
@@ -240,7 +303,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 768 / NT) ensemble_kernel(
             __syncthreads();
             if (tid == 0) {
                 double r = 1e38;
-                for (int w = 0; w < NT / 32; w++) r = (s_red[w] < r) ? s_red[w] : r;
+                for (int w = 0; w < TT / 32; w++) r = (s_red[w] < r) ? s_red[w] : r;
                 if (a.halve) r = r / 2;
                 double dt = __dmul_rn(a.cfl, r);
                 if (__dadd_rn(t, __dmul_rn(2.0, dt)) > a.t_end) dt = __dmul_rn(.5, __dadd_rn(a.t_end, -t));
@@ -250,7 +313,14 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 768 / NT) ensemble_kernel(
             const double dt = s_dt;
             const double lambda = dt / h;
             for (int half = 0; half < 2; half++) {
-                ens_sweep<METHOD, SLOPE, FT, NT>(qb, a.S, n, nc, lambda, c, SA, SB, a.lcap, pend, first);
+                if constexpr (TWO) {
+                    double *SS = tsm + 40;  // the SSPRK sums, then the planes
+                    ens_sweep_two<METHOD, SLOPE, FT, TT>(qb, a.S, n, nc, lambda, c,
+                                                         reinterpret_cast<FT *>(SS + 10 * TT), SS, pend, first);
+                } else {
+                    FT *SA = reinterpret_cast<FT *>(tsm + 40);  // [5][lcap]
+                    ens_sweep<METHOD, SLOPE, FT, NT>(qb, a.S, n, nc, lambda, c, SA, SA + 5 * a.lcap, a.lcap, pend, first);
+                }
                 if (tid == 0) ens_boundary(qb, a.S, n, a.bc0, a.bc1);
                 __syncthreads();
             }
@@ -268,20 +338,21 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 768 / NT) ensemble_kernel(
     }
 }
 
-// Shared memory of one CTA: the pending and first outputs, two planes of a chunk of up to lcap
-// tile rows.
-template <typename FT>
+// Shared memory of one CTA: the pending and first outputs, and two planes of a chunk of up to lcap tile
+// rows, or the sums and planes of two rows a thread.
+template <typename FT, int NT, bool TWO>
 static size_t ens_smem(int lcap)
 {
-    return sizeof(double) * 40 + sizeof(FT) * 10 * (size_t)lcap;
+    return sizeof(double) * 40 + (TWO ? duo_smem_bytes<FT, NT / 2>() : sizeof(FT) * 10 * (size_t)lcap);
 }
 
-template <int METHOD, int SLOPE, typename FT, int NT>
+template <int METHOD, int SLOPE, typename FT, int NT, bool TWO>
 static int launch_ens_nt(const EnsArgs &a0, const FluidConsts<FT> &c, int ctas_per_sm, cudaStream_t st)
 {
     EnsArgs a = a0;
-    auto kern = ensemble_kernel<METHOD, SLOPE, FT, NT>;
-    const size_t shm = ens_smem<FT>(a.lcap);
+    auto kern = ensemble_kernel<METHOD, SLOPE, FT, NT, TWO>;
+    constexpr int TT = TWO ? NT / 2 : NT;
+    const size_t shm = ens_smem<FT, NT, TWO>(a.lcap);
     static int attr_bytes = 0;
     int rc;
     if ((int)shm > attr_bytes) {
@@ -290,22 +361,40 @@ static int launch_ens_nt(const EnsArgs &a0, const FluidConsts<FT> &c, int ctas_p
         attr_bytes = (int)shm;
     }
     int per_sm = 0;
-    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, shm)))) return rc;
+    if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TT, shm)))) return rc;
     if (per_sm < 1 || a.lcap > NT) return IB_ERROR_INVALID_ARGS;
-    if (ctas_per_sm > 0 && ctas_per_sm < per_sm) per_sm = ctas_per_sm;
+    // a CTA of two rows a thread counts as half a CTA of the launch shape's `threads`, so that a limit keeps
+    // the rows in flight that it was chosen for
+    const int limit = TWO ? 2 * ctas_per_sm : ctas_per_sm;
+    if (limit > 0 && limit < per_sm) per_sm = limit;
     const int64_t grid = std::min<int64_t>((int64_t)per_sm * num_sms(), a.np);
     if ((rc = check_cuda(cudaMemsetAsync(a.counter, 0, sizeof(unsigned int), st)))) return rc;
-    kern<<<(unsigned)grid, NT, shm, st>>>(a, c);
+    kern<<<(unsigned)grid, TT, shm, st>>>(a, c);
     return check_launch();
+}
+
+// Two rows a thread where the problems fill the chip twice at the default launch shape (five CTAs per SM for
+// FP64, six for the FP32 flux): half the shared-memory traffic, 1500 / 4096 problems of 256-4096 cells 2.96 /
+// 6.30 -> 2.53 / 5.23 ms (FP64, 10 / 8 iterations), 5.05 -> 4.01 (FP32 flux, 4096).  With fewer, a problem's own
+// time counts, and a CTA of half the threads takes longer for it: 170 problems 1.19 -> 1.33, 800 1.71 -> 2.28.
+// The rule is by the number of problems alone, so that results do not depend on the launch shape.
+template <typename FT>
+static bool ens_two_rows(int np) { return np >= 2 * duo_min_blocks<FT>(128) * num_sms(); }
+
+template <int METHOD, int SLOPE, typename FT, int NT>
+static int launch_ens_form(const EnsArgs &a, const FluidConsts<FT> &c, int ctas_per_sm, cudaStream_t st)
+{
+    return ens_two_rows<FT>(a.np) ? launch_ens_nt<METHOD, SLOPE, FT, NT, true>(a, c, ctas_per_sm, st)
+                                  : launch_ens_nt<METHOD, SLOPE, FT, NT, false>(a, c, ctas_per_sm, st);
 }
 
 template <int METHOD, int SLOPE, typename FT>
 static int launch_ens(const EnsArgs &a, const FluidConsts<FT> &c, int threads, int ctas_per_sm, cudaStream_t st)
 {
     switch (threads) {
-    case 128: return launch_ens_nt<METHOD, SLOPE, FT, 128>(a, c, ctas_per_sm, st);
-    case 256: return launch_ens_nt<METHOD, SLOPE, FT, 256>(a, c, ctas_per_sm, st);
-    case 512: return launch_ens_nt<METHOD, SLOPE, FT, 512>(a, c, ctas_per_sm, st);
+    case 128: return launch_ens_form<METHOD, SLOPE, FT, 128>(a, c, ctas_per_sm, st);
+    case 256: return launch_ens_form<METHOD, SLOPE, FT, 256>(a, c, ctas_per_sm, st);
+    case 512: return launch_ens_form<METHOD, SLOPE, FT, 512>(a, c, ctas_per_sm, st);
     default: return IB_ERROR_INVALID_ARGS;
     }
 }

@@ -39,7 +39,7 @@ __device__ __forceinline__ V5<FT> v5_sub(const V5<FT> &a, const V5<FT> &b)
 // HLL primitives: [rho, v_n, P, v_t1, v_t2] with P taken from the floored pressure
 // (cudaFluidStep.cu:1864-1888).  irho: 1 / rho, product build (one reciprocal for the five quotients of
 // the pressure solver and the velocities; the strict build divides as the reference does)
-template <typename FT>
+template <typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2, FT irho)
 {
     V5<FT> w;
@@ -50,9 +50,9 @@ __device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2,
     w.a[3] = pt1 / rho;
     w.a[4] = pt2 / rho;
 #else
-    w.a[1] = pn * irho;
-    w.a[3] = pt1 * irho;
-    w.a[4] = pt2 * irho;
+    w.a[1] = product<RN>(pn, irho);
+    w.a[3] = product<RN>(pt1, irho);
+    w.a[4] = product<RN>(pt2, irho);
 #endif
     return w;
 }
@@ -71,7 +71,7 @@ __device__ __forceinline__ void hll_faces(const V5<FT> &w, const V5<FT> &dl, con
 
 // HLL flux (cudaFluidStep.cu:2057-2198).  le = right face of the left cell, re = left face of
 // the right cell, both [rho, v_n, P, v_t1, v_t2].  Output [rho, E, p_n, p_t1, p_t2].
-template <typename FT>
+template <typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT> &le, const V5<FT> &re)
 {
     const FT Ale = le.a[0], Ble = le.a[1], Cle = le.a[2], Dle = le.a[3], Ele = le.a[4];
@@ -92,8 +92,8 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
 #else
     FT Atilde = rcp_fast(Sright - Sleft);
 #endif
-    FT Fa = Ale * Ble;
-    FT Fb = Are * Bre;
+    FT Fa = product<RN>(Ale, Ble);
+    FT Fb = product<RN>(Are, Bre);
     V5<FT> f;
     int mode = 1;
     if (Sleft >= 0) mode = 0;
@@ -101,24 +101,24 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
     if (mode == 0) {
         f.a[0] = Fa;
         if (!iso) {
-            f.a[1] = Ble * (c.govergm1 * Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele));
+            f.a[1] = product<RN>(Ble, (c.govergm1 * Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele)));
             f.a[2] = Fa * Ble + Cle;
         } else {
-            f.a[1] = Ble * (Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele));
+            f.a[1] = product<RN>(Ble, (Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele)));
             f.a[2] = Fa * Ble + c.isotempsq * Ale;
         }
-        f.a[3] = Fa * Dle;
-        f.a[4] = Fa * Ele;
+        f.a[3] = product<RN>(Fa, Dle);
+        f.a[4] = product<RN>(Fa, Ele);
     } else if (mode == 1) {
-        f.a[0] = (Sright * (Ble - Sleft) * Ale - Sleft * (Bre - Sright) * Are) * Atilde;
+        f.a[0] = product<RN>((Sright * (Ble - Sleft) * Ale - Sleft * (Bre - Sright) * Are), Atilde);
         if (!iso) {
-            f.a[2] = (Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb + Sright * Cle - Sleft * Cre) * Atilde;
+            f.a[2] = product<RN>((Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb + Sright * Cle - Sleft * Cre), Atilde);
         } else {
-            f.a[2] = (Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb +
-                      c.isotempsq * (Sright * Ale - Sleft * Are)) * Atilde;
+            f.a[2] = product<RN>((Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb +
+                      c.isotempsq * (Sright * Ale - Sleft * Are)), Atilde);
         }
-        f.a[3] = (Sright * (Ble - Sleft) * Ale * Dle - Sleft * (Bre - Sright) * Are * Dre) * Atilde;
-        f.a[4] = (Sright * (Ble - Sleft) * Ale * Ele - Sleft * (Bre - Sright) * Are * Ere) * Atilde;
+        f.a[3] = product<RN>((Sright * (Ble - Sleft) * Ale * Dle - Sleft * (Bre - Sright) * Are * Dre), Atilde);
+        f.a[4] = product<RN>((Sright * (Ble - Sleft) * Ale * Ele - Sleft * (Bre - Sright) * Are * Ere), Atilde);
         if (!iso) {
             Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele);
             Fb = (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere);
@@ -128,7 +128,7 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
 #else
             const FT dp = Sleft * Sright * (Cre - Cle) * c.rgm1;
 #endif
-            f.a[1] = (e + (c.govergm1 * (Sright * Cle * Ble - Sleft * Cre * Bre) + dp)) * Atilde;
+            f.a[1] = product<RN>((e + (c.govergm1 * (Sright * Cle * Ble - Sleft * Cre * Bre) + dp)), Atilde);
         } else {
             // isothermal energy flux lacks the 1/(S_R-S_L) factor (cudaFluidStep.cu:2178-2182)
             Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele) + Cle;
@@ -138,14 +138,14 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
     } else {
         f.a[0] = Fb;
         if (!iso) {
-            f.a[1] = Bre * (c.govergm1 * Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere));
+            f.a[1] = product<RN>(Bre, (c.govergm1 * Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere)));
             f.a[2] = Fb * Bre + Cre;
         } else {
-            f.a[1] = Bre * (Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere));
+            f.a[1] = product<RN>(Bre, (Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere)));
             f.a[2] = Fb * Bre + c.isotemp * Are;  // c_iso, not c_iso^2 (cudaFluidStep.cu:2191)
         }
-        f.a[3] = Fb * Dre;
-        f.a[4] = Fb * Ere;
+        f.a[3] = product<RN>(Fb, Dre);
+        f.a[4] = product<RN>(Fb, Ere);
     }
     return f;
 }
@@ -212,15 +212,15 @@ __device__ __forceinline__ constexpr int slot_of(int k)
 }
 
 // Per-cell stage "prims" for either method.  For HLL the floors are applied to u first.
-template <int METHOD, int DIR, typename FT>
+template <int METHOD, int DIR, typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> stage_prims(double u[5], const FluidConsts<FT> &c)
 {
     if constexpr (METHOD == IB_METHOD_HLLC) {
-        return hllc_prims<FT>((FT)u[0], (FT)u[1], (FT)u[2], (FT)u[3], (FT)u[4]);
+        return hllc_prims<FT, RN>((FT)u[0], (FT)u[1], (FT)u[2], (FT)u[3], (FT)u[4]);
     } else {
         double irho;
         double P = hll_pressure<DIR>(u, c.minmass, c.mintemp, (double)c.gm1, irho);
-        return hll_prims<FT>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4], (FT)irho);
+        return hll_prims<FT, RN>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4], (FT)irho);
     }
 }
 
@@ -232,11 +232,11 @@ __device__ __forceinline__ void stage_faces(const FluidConsts<FT> &c, const V5<F
     else hll_faces<SLOPE, FT>(w, dl, dr, L, R);
 }
 
-template <int METHOD, typename FT>
+template <int METHOD, typename FT, bool RN = false>
 __device__ __forceinline__ V5<FT> stage_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
-    if constexpr (METHOD == IB_METHOD_HLLC) return hllc_flux<FT>(c, l, r);
-    else return hll_flux<FT>(c, l, r);
+    if constexpr (METHOD == IB_METHOD_HLLC) return hllc_flux<FT, RN>(c, l, r);
+    else return hll_flux<FT, RN>(c, l, r);
 }
 
 // lambda times the flux difference of one cell in cylindrical geometry, component by component
