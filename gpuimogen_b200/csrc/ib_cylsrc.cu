@@ -11,7 +11,8 @@
 // become non-positive, where E is reset to the new kinetic energy plus 1e-5 rho.
 //
 // One thread per cell: a grid-stride loop over the arrays in XYZ order, 5 loads and at most 3
-// stores of 8 bytes per cell (HBM-bound; it runs once per source step).
+// stores of 8 bytes per cell.  The cell's 14 divisions bound it, not memory, so the product build
+// forms the reciprocals of r and rho once each and the quotients from them, to the division's error.
 #include "ib_internal.cuh"
 
 namespace ib {
@@ -30,32 +31,44 @@ __global__ void __launch_bounds__(256) cyl_source_kernel(double *__restrict__ q,
     const double dt = dts.get();
     for (int64_t x = threadIdx.x + (int64_t)blockIdx.x * blockDim.x; x < n; x += (int64_t)blockDim.x * gridDim.x) {
         double *base = q + x;
-        const double r = rin + (int)(x % nx) * dr;
+        const double r = rin + column_of(x, nx) * dr;
         const double rho = base[0];
+#ifdef IB_STRICT_ARITH
+        auto over_r = [&](double a) { return a / r; };
         double u = base[2 * slab] / rho;  // v_r
         double v = base[3 * slab] / rho;  // v_theta
-        double diffmom = dt * v / r;
+#else
+        const double ir = rcp_fast(r), irho = rcp_fast(rho);
+        auto over_r = [&](double a) { return quotient_fast(a, r, ir); };
+        double u = quotient_fast(base[2 * slab], rho, irho);
+        double v = quotient_fast(base[3 * slab], rho, irho);
+#endif
+        double diffmom = over_r(dt * v);
         double vrA = u + kGL11 * v * diffmom;
         double vphiA = v - kGL11 * u * diffmom;
         double vrB = u + kGL12 * v * diffmom;
         double vphiB = v - kGL12 * u * diffmom;
 #pragma unroll
         for (int it = 0; it < 2; it++) {
-            diffmom = dt * vphiA / r;
-            const double diffmomB = dt * vphiB / r;
+            diffmom = over_r(dt * vphiA);
+            const double diffmomB = over_r(dt * vphiB);
             double scratch = vrA;
             vrA = u + kGL11 * vphiA * diffmom + kGL12 * vphiB * diffmomB;
             vphiA = v - kGL11 * scratch * diffmom + kGL12 * vrB * diffmomB;
-            diffmom = dt * vphiA / r;
+            diffmom = over_r(dt * vphiA);
             scratch = vrB;
             vrB = u + kGL21 * vphiA * diffmom + kGL22 * vphiB * diffmomB;
             vphiB = v - kGL21 * scratch * diffmom + kGL22 * scratch * diffmomB;
         }
-        u = rho * (u + .5 * dt * (vphiA * vphiA + vphiB * vphiB) / r);
-        v = rho * (v - .5 * dt * (vphiA * vrA + vphiB * vrB) / r);
+        u = rho * (u + over_r(.5 * dt * (vphiA * vphiA + vphiB * vphiB)));
+        v = rho * (v - over_r(.5 * dt * (vphiA * vrA + vphiB * vrB)));
         const double E = base[slab];
         const double w = base[4 * slab];
+#ifdef IB_STRICT_ARITH
         const double newP = E - .5 * (u * u + v * v + w * w) / rho;
+#else
+        const double newP = E - quotient_fast(.5 * (u * u + v * v + w * w), rho, irho);
+#endif
         if (newP <= 0.0) base[slab] = .5 * (u * u + v * v + w * w) / rho + .00001 * rho;
         base[2 * slab] = u;
         base[3 * slab] = v;

@@ -38,6 +38,13 @@ __device__ __forceinline__ double rcp_fast_pos(double x)
     return fma(y, fma(e, e, e), y);
 }
 
+// a / x from ix, the rounded reciprocal: one correction by the remainder, whose error is that of the division
+__device__ __forceinline__ double quotient_fast(double a, double x, double ix)
+{
+    const double q = a * ix;
+    return fma(fma(-q, x, a), ix, q);
+}
+
 // sqrt(x); the seed's operand is at least the smallest normal number (unsigned: negative ones pass)
 __device__ __forceinline__ double sqrt_fast(double x)
 {

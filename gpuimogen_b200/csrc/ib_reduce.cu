@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(256) cfl_kernel(const double *__restrict__ q, 
             const double vy = (SIM > 1 || XJ) ? py[u] : 0.0, vz = (SIM > 2 || XJ) ? pz[u] : 0.0;
             if constexpr (CYL)
                 tmin = min_keep(tmin, cfl_cell_cyl<SIM, XJ>(rho[u], px[u], vy, vz, cs[u], hmin, hx, hy, hz, rin,
-                                                            (int)(x % nx)));
+                                                            column_of(x, nx)));
             else
                 tmin = min_keep(tmin, cfl_cell<SIM, XJ>(rho[u], px[u], vy, vz, cs[u], hmin, hx, hy, hz));
         }
