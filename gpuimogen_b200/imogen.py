@@ -390,33 +390,37 @@ def fluidstep(fluids, geometry, params, num=None):
     _check("ib_fluidstep", _lib().ib_fluidstep(fs, th, len(fluids), ctypes.byref(g), p, n, nm, _stream()))
 
 
-def completeTimestep(fluids, geometry, params, num=None, drag=None):
-    """performCompleteTimestep(fluids, [dt, purehydro, iteration, method]): source half step,
-    forward fluid step, source step, backward fluid step, source half step.  drag = (thermo_gas,
-    thermo_dust, method) makes fluids [gas, dust] exchange momentum by the two-fluid drag; without
-    it there is no source and the two same-axis sweeps mid-step run as one launch where they can."""
-    if isinstance(fluids, Fluid):
-        fluids = [fluids]
-    fs = (IbFluid * len(fluids))(*[f.c_struct() for f in fluids])
-    th = (IbFluidThermo * len(fluids))(*[f.thermo() for f in fluids])
-    g = geometry.c_struct()
-    p, n = _dvec(params)
-    nm = ctypes.byref(num) if num is not None else None
-    ds = None
-    if drag is not None:
-        tg, td, method = drag
-        ds = ctypes.byref(IbDragSource(thermo_struct(tg), thermo_struct(td),
-                                       DRAG[method] if isinstance(method, str) else int(method), 0))
-    _check("ib_completeTimestep", _lib().ib_completeTimestep(fs, th, len(fluids), ctypes.byref(g), p, n, nm, ds,
-                                                             _stream()))
-
-
 def _drag_struct(drag):
     if drag is None:
         return None
     tg, td, method = drag
     return IbDragSource(thermo_struct(tg), thermo_struct(td), DRAG[method] if isinstance(method, str) else int(method),
                         0)
+
+
+def _complete_args(fluids, geometry, num=None, drag=None):
+    """The C arguments of a complete timestep other than its parameter vector."""
+    if isinstance(fluids, Fluid):
+        fluids = [fluids]
+    fs = (IbFluid * len(fluids))(*[f.c_struct() for f in fluids])
+    th = (IbFluidThermo * len(fluids))(*[f.thermo() for f in fluids])
+    return fs, th, geometry.c_struct(), num, _drag_struct(drag)
+
+
+def _complete(args, params):
+    fs, th, g, num, ds = args
+    p, n = _dvec(params)
+    _check("ib_completeTimestep", _lib().ib_completeTimestep(
+        fs, th, len(fs), ctypes.byref(g), p, n, ctypes.byref(num) if num is not None else None,
+        ctypes.byref(ds) if ds is not None else None, _stream()))
+
+
+def completeTimestep(fluids, geometry, params, num=None, drag=None):
+    """performCompleteTimestep(fluids, [dt, purehydro, iteration, method]): source half step,
+    forward fluid step, source step, backward fluid step, source half step.  drag = (thermo_gas,
+    thermo_dust, method) makes fluids [gas, dust] exchange momentum by the two-fluid drag; without
+    it there is no source and the two same-axis sweeps mid-step run as one launch where they can."""
+    _complete(_complete_args(fluids, geometry, num, drag), params)
 
 
 def completeTimestepDeviceDt(fluids, geometry, dt_device, params, num=None, drag=None):

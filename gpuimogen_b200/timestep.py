@@ -42,23 +42,44 @@ class TimeManager:
         return self.time < self.TIMEMAX * (1 - 1e-14) if math.isfinite(self.TIMEMAX) else True
 
 
-def cfl_tau(fluids, geometry, method):
-    """Minimum over fluids of the CFL time (TimeManager.update loop)."""
+def _launch_cfl(fluids, geometry, method):
+    """Queues the CFL reduction of every fluid; each writes its time straight into page-locked host memory."""
+    taus = torch.empty(len(fluids), dtype=torch.float64, pin_memory=True)
+    try:
+        for k, f in enumerate(fluids):
+            ib.cflTimestepFused(f, f.gamma, geometry, method, tau_device=taus[k:k + 1])
+    except Exception:
+        torch.cuda.current_stream().synchronize()  # the memory goes back only when nothing writes it
+        raise
+    return taus
+
+
+def _wait_tau(taus):
+    torch.cuda.current_stream().synchronize()
     tau = 1e38
-    for f in fluids:
-        t = ib.cflTimestepFused(f, f.gamma, geometry, method)
+    for t in taus.tolist():
         if not math.isfinite(t):
             raise ib.ImogenError("cflTimestep: non-finite timestep", -101)
         tau = min(tau, t)
     return tau
 
 
+def cfl_tau(fluids, geometry, method):
+    """Minimum over fluids of the CFL time (TimeManager.update loop)."""
+    return _wait_tau(_launch_cfl(fluids, geometry, method))
+
+
 def run_iteration(fluids, geometry, tm, method, num=None, source=None, drag=None):
     """One main-loop iteration; `source(fluids, dt_fraction)` applies the sources if given
     (forward and backward fluid steps through fluidstep, as the Matlab loop calls them);
     otherwise the complete timestep runs through completeTimestep (performCompleteTimestep), with
-    the two-fluid drag between the steps when drag = (thermo_gas, thermo_dust, method)."""
-    tau = cfl_tau(fluids, geometry, method)
+    the two-fluid drag between the steps when drag = (thermo_gas, thermo_dust, method).  The host prepares
+    the step's arguments while the reductions run and waits once for all fluids."""
+    taus = _launch_cfl(fluids, geometry, method)
+    try:
+        args = ib._complete_args(fluids, geometry, num, drag) if source is None else None
+    finally:
+        tau = _wait_tau(taus)
     dt = tm.update(tau)
     if source is not None:
         source(fluids, 0.5 * dt)
@@ -67,7 +88,7 @@ def run_iteration(fluids, geometry, tm, method, num=None, source=None, drag=None
         ib.fluidstep(fluids, geometry, [dt, 1, -1, tm.iteration, method], num)
         source(fluids, 0.5 * dt)
     else:
-        ib.completeTimestep(fluids, geometry, [dt, 1, tm.iteration, method], num, drag=drag)
+        ib._complete(args, [dt, 1, tm.iteration, method])
     tm.step()
     return dt
 
