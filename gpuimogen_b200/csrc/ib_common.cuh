@@ -92,15 +92,6 @@ __device__ __forceinline__ FT flux_minmod(FT A, FT B)
     return A;
 }
 
-__device__ __forceinline__ bool signs_differ(double a, double b)
-{
-    return (__double2hiint(a) ^ __double2hiint(b)) < 0;
-}
-__device__ __forceinline__ bool signs_differ(float a, float b)
-{
-    return (__float_as_int(a) ^ __float_as_int(b)) < 0;
-}
-
 template <int SLOPE, typename FT>
 __device__ __forceinline__ FT slope_limit(FT A, FT B)
 {
@@ -127,12 +118,12 @@ __device__ __forceinline__ FT slope_limit(FT A, FT B)
         return S * A;
 #else
         // min(.25(1+R), R, 1) * A with R = B/A, without the division: for A and B of one sign it is
-        // the smallest in magnitude of .25(A+B), B and A (of opposite sign: 0; by their sign bits,
-        // so that slopes below 1e-162, whose product underflows to zero, are limited like any other)
+        // the smallest in magnitude of .25(A+B), B and A.  A is kept where B or the sum is NaN, as in the
+        // form with the quotient
         const FT S = (FT).25 * (A + B);
-        const FT m = (fabs(A) < fabs(B)) ? A : B;
-        const FT r = (fabs(m) <= fabs(S)) ? m : S;
-        return signs_differ(A, B) ? (FT)0 : r;
+        const FT m = (fabs(B) < fabs(A)) ? B : A;
+        const FT r = (fabs(S) < fabs(m)) ? S : m;
+        return (A * B <= 0) ? (FT)0 : r;
 #endif
     } else if constexpr (SLOPE == IB_SLOPE_VANLEER) {  // limiter_functions.h:54-61
         FT r = A * B;
