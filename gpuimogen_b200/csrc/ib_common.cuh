@@ -92,22 +92,45 @@ __device__ __forceinline__ FT flux_minmod(FT A, FT B)
     return A;
 }
 
-template <int SLOPE, typename FT>
+// Sums of products.  Product build: written with fma, so that every kernel, and every instantiation of one, rounds
+// them alike (the compiler can contract a b + c d in two ways).  Strict build: the plain operations.
+#ifdef IB_STRICT_ARITH
+template <typename FT> __device__ __forceinline__ FT add_product(FT s, FT a, FT b) { return s + a * b; }
+template <typename FT> __device__ __forceinline__ FT sub_product(FT s, FT a, FT b) { return s - a * b; }
+template <typename FT> __device__ __forceinline__ FT sum_products(FT a, FT b, FT c, FT d) { return a * b + c * d; }
+template <typename FT> __device__ __forceinline__ FT diff_products(FT a, FT b, FT c, FT d) { return a * b - c * d; }
+#else
+template <typename FT> __device__ __forceinline__ FT add_product(FT s, FT a, FT b) { return fma(a, b, s); }
+template <typename FT> __device__ __forceinline__ FT sub_product(FT s, FT a, FT b) { return fma(-a, b, s); }
+template <typename FT> __device__ __forceinline__ FT sum_products(FT a, FT b, FT c, FT d) { return fma(a, b, c * d); }
+template <typename FT> __device__ __forceinline__ FT diff_products(FT a, FT b, FT c, FT d) { return fma(a, b, -(c * d)); }
+#endif
+template <typename FT>
+__device__ __forceinline__ FT square_sum(FT a, FT b, FT c) { return add_product(add_product(a * a, b, b), c, c); }
+
+#ifdef IB_STRICT_ARITH
+template <typename OPS> constexpr bool kDivide = true;
+#else
+template <typename OPS> constexpr bool kDivide = std::is_same<OPS, IeeeOps>::value;
+#endif
+
+template <int SLOPE, typename FT, typename OPS = FastOps>
 __device__ __forceinline__ FT slope_limit(FT A, FT B)
 {
     if constexpr (SLOPE == IB_SLOPE_OSPRE) {  // limiter_functions.h:87-95
         FT R = A * B;
-#ifdef IB_STRICT_ARITH
-        if (R > 0) {
-            FT S = A + B;
-            return (FT).75 * R * S / (S * S - R);
+        if constexpr (kDivide<OPS>) {
+            if (R > 0) {
+                FT S = A + B;
+                return (FT).75 * R * S / (S * S - R);
+            }
+            return (FT)0.0;
         }
-        return (FT)0.0;
-#else
-        const FT S = A + B;  // the denominator is A^2 + A B + B^2 > 0 where R > 0
-        const FT s = (FT).75 * R * S * rcp_fast_pos(S * S - R);
-        return (R > 0) ? s : (FT)0;
-#endif
+        // the denominator is A^2 + A B + B^2 > 0 where R > 0; from 2^1022 on (slopes above 6e153) the slope is 0,
+        // as the division gives it where the denominator overflows
+        const FT S = A + B, D = sub_product(S * S, A, B);
+        const FT s = (FT).75 * R * S * rcp_fast_pos(D);
+        return (R > 0 && !(D >= (FT)kRcpTop)) ? s : (FT)0;
     } else if constexpr (SLOPE == IB_SLOPE_MC) {  // limiter_functions.h:105-115
 #ifdef IB_STRICT_ARITH
         if (A * B <= 0) return (FT)0;
@@ -127,13 +150,12 @@ __device__ __forceinline__ FT slope_limit(FT A, FT B)
 #endif
     } else if constexpr (SLOPE == IB_SLOPE_VANLEER) {  // limiter_functions.h:54-61
         FT r = A * B;
-#ifdef IB_STRICT_ARITH
-        if (r > (FT)0.0) return r / (A + B);
-        return (FT)0;
-#else
+        if constexpr (kDivide<OPS>) {
+            if (r > (FT)0.0) return r / (A + B);
+            return (FT)0;
+        }
         const FT s = r * rcp_fast(A + B);
         return (r > (FT)0.0) ? s : (FT)0;
-#endif
     } else if constexpr (SLOPE == IB_SLOPE_MINMOD) {  // limiter_functions.h:71-77
         // the FP64 reference returns this limiter through a float
         if (A * B < 0) return (FT)0.0;
@@ -146,7 +168,7 @@ __device__ __forceinline__ FT slope_limit(FT A, FT B)
     } else if constexpr (SLOPE == IB_SLOPE_VANALBADA) {  // limiter_functions.h:97-102
         FT R = A * B;
         if (R < 0) return (FT)0;
-        return (FT).5 * R * (A + B) / (A * A + B * B);
+        return (FT).5 * R * (A + B) / sum_products(A, A, B, B);
     } else {
         return (FT)0.0;
     }
@@ -203,43 +225,37 @@ __device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT v
 #else
 // with the Roe weights wl = 1 / (1 + Fa) and wr = Fa wl, Fa = sqrt(rhoR / rhoL); irL, irR: the density
 // reciprocals, which the HLLC star flux takes over
-template <typename FT>
+// With the short forms, sl is NaN where the Roe sound speed is, which the comparisons would drop.
+template <typename OPS, typename FT>
 __device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR, FT vR, FT PR,
                                          FT dvsq, FT &sl, FT &sr, FT &irL, FT &irR)
 {
-    irL = rcp_fast(rhoL);
-    irR = rcp_fast(rhoR);
+    irL = OPS::rcp(rhoL);
+    irR = OPS::rcp(rhoR);
     const FT csql = c.gamma * PL * irL, csqr = c.gamma * PR * irR;
-    const FT Fa = sqrt_fast(rhoR * irL);
-    const FT wl = rcp_fast((FT)1.0 + Fa);
+    const FT Fa = OPS::root(rhoR * irL);
+    const FT wl = OPS::rcp((FT)1.0 + Fa);
     const FT wr = Fa * wl;
-    const FT vroe = wl * vL + wr * vR;
-    const FT croe = sqrt_fast(wl * csql + wr * csqr + c.hgm1 * dvsq * (wl * wr));
-    sl = vL - sqrt_fast(csql);
-    sr = vR + sqrt_fast(csqr);
+    const FT vroe = sum_products(wl, vL, wr, vR);
+    const FT croe = OPS::root(add_product(sum_products(wl, csql, wr, csqr), c.hgm1 * dvsq, wl * wr));
+    sl = vL - OPS::root(csql);
+    sr = vR + OPS::root(csqr);
     const FT s1 = vroe - croe, s2 = vroe + croe;
     sl = (s1 < sl) ? s1 : sl;
     sr = (s2 > sr) ? s2 : sr;
-}
-
-template <typename FT>
-__device__ __forceinline__ void einfeldt(const FluidConsts<FT> &c, FT rhoL, FT vL, FT PL, FT rhoR, FT vR, FT PR,
-                                         FT dvsq, FT &sl, FT &sr)
-{
-    FT irL, irR;
-    einfeldt<FT>(c, rhoL, vL, PL, rhoR, vR, PR, dvsq, sl, sr, irL, irR);
+    if constexpr (kPoison<OPS, FT>) sl = fma(croe, 0.0, sl);
 }
 #endif
 
-template <typename FT>
+template <typename OPS, typename FT>
 __device__ __forceinline__ void einfeldt_iso(FT rhoL, FT vL, FT rhoR, FT vR, FT cs, FT &sl, FT &sr)
 {
 #ifdef IB_STRICT_ARITH
     FT Fa = dsqrt<FT>(rhoR / rhoL);
     FT Fb = (FT)1.0 / ((FT)1.0 + Fa);
 #else
-    FT Fa = sqrt_fast(rhoR * rcp_fast(rhoL));
-    FT Fb = rcp_fast((FT)1.0 + Fa);
+    FT Fa = OPS::root(rhoR * OPS::rcp(rhoL));
+    FT Fb = OPS::rcp((FT)1.0 + Fa);
 #endif
     FT Vroe = (vL + Fa * vR) * Fb;
     cs = Vroe - cs;
@@ -266,15 +282,15 @@ template <bool RN>
 __device__ __forceinline__ float product(float a, float b) { return RN ? __fmul_rn(a, b) : a * b; }
 
 // Conserved -> HLLC primitives (cudaFluidStep.cu:1200-1237).  u: [rho, E, p_n, p_t1, p_t2].
-template <typename FT, bool RN = false>
+template <typename FT, bool RN = false, typename OPS = GuardedOps>
 __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 {
 #ifdef IB_STRICT_ARITH
     FT F = (FT)1.0 / A;
 #else
-    FT F = rcp_fast(A);
+    FT F = OPS::rcp(A);
 #endif
-    B -= (FT).5 * (C * C + D * D + E * E) * F;
+    B -= (FT).5 * square_sum(C, D, E) * F;
     C = product<RN>(C, F);
     D = product<RN>(D, F);
     E = product<RN>(E, F);
@@ -285,13 +301,13 @@ __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 
 // Limited faces of one cell from its primitive value and its two backward differences.
 // L/R faces: rho, P = gm1*(e -/+ s), v.  (cudaFluidStep.cu:1287-1310)
-template <int SLOPE, typename FT>
+template <int SLOPE, typename FT, typename OPS = FastOps>
 __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT> &w,
                                            const V5<FT> &dl, const V5<FT> &dr, V5<FT> &L, V5<FT> &R)
 {
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        FT s = slope_limit<SLOPE, FT>(dl.a[k], dr.a[k]);
+        FT s = slope_limit<SLOPE, FT, OPS>(dl.a[k], dr.a[k]);
         if (k == 1) {
             L.a[1] = c.gm1 * (w.a[1] - s);
             R.a[1] = c.gm1 * (w.a[1] + s);
@@ -305,7 +321,7 @@ __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT
 // HLLC flux through the face between the right face state of the left cell (l) and the left
 // face state of the right cell (r).  (cudaFluidStep.cu:1318-1432)
 #ifdef IB_STRICT_ARITH
-template <typename FT, bool RN = false>
+template <typename FT, bool RN = false, typename OPS = IeeeOps>
 __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
     const FT rhoL = l.a[0], PL = l.a[1], vxL = l.a[2], vyL = l.a[3], vzL = l.a[4];
@@ -378,38 +394,39 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
 #else
 // The same flux with fewer and shorter dependent chains: reciprocals and roots of ib_fast.cuh, and the
 // star (or outer) state computed once, for the side that the contact speed selects, instead of in
-// divergent branches.
-template <typename FT, bool RN = false>
+// divergent branches.  With the short forms the mass flux is NaN wherever one of them is: a NaN among the
+// waves makes sm NaN, which then takes the star state.
+template <typename FT, bool RN = false, typename OPS = IeeeOps>
 __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
     const FT rhoL = l.a[0], PL = l.a[1], vL = l.a[2];
     const FT rhoR = r.a[0], PR = r.a[1], vR = r.a[2];
     const FT dn = vL - vR, d1 = l.a[3] - r.a[3], d2 = l.a[4] - r.a[4];
     FT sl, sr, irL, irR;
-    einfeldt<FT>(c, rhoL, vL, PL, rhoR, vR, PR, dn * dn + d1 * d1 + d2 * d2, sl, sr, irL, irR);
+    einfeldt<OPS, FT>(c, rhoL, vL, PL, rhoR, vR, PR, square_sum(dn, d1, d2), sl, sr, irL, irR);
     const FT A = rhoL * (sl - vL), B = rhoR * (sr - vR);
-    const FT sm = (B * vR - PR - A * vL + PL) * rcp_fast(B - A);  // Batten et al. eq. 34
+    const FT sm = (sub_product(add_product(-PR, B, vR), A, vL) + PL) * OPS::rcp(B - A);  // Batten et al. eq. 34
     const bool left = sm > 0;
     const FT rho = left ? rhoL : rhoR, P = left ? PL : PR, v = left ? vL : vR;
     const FT t1 = left ? l.a[3] : r.a[3], t2 = left ? l.a[4] : r.a[4];
-    const FT ke = (FT).5 * (v * v + t1 * t1 + t2 * t2);
+    const FT ke = (FT).5 * square_sum(v, t1, t2);
     const FT h = c.govergm1 * P;
     V5<FT> f;
-    if (left ? sl > 0 : !(sr > 0)) {  // the outer state: no wave crosses the face
+    if (left ? sl > 0 : ((!kPoison<OPS, FT> || sm <= 0) && !(sr > 0))) {  // the outer state: no wave crosses the face
         const FT m = product<RN>(rho, v);
         f.a[0] = m;
-        f.a[1] = product<RN>(v, ke * rho + h);
-        f.a[2] = m * v + P;
+        f.a[1] = product<RN>(v, add_product(h, ke, rho));
+        f.a[2] = add_product(P, m, v);
         f.a[3] = product<RN>(m, t1);
         f.a[4] = product<RN>(m, t2);
     } else {
         const FT S = left ? sl : sr;
-        const FT D = (left ? A : B) * rcp_fast(S - sm);
+        const FT D = (left ? A : B) * OPS::rcp(S - sm);
         const FT m = product<RN>(D, sm);
         const FT q = S * (sm - v);
         f.a[0] = m;
-        f.a[1] = product<RN>(m, h * (left ? irL : irR) + ke + q);
-        f.a[2] = P + D * (q + sm * v);
+        f.a[1] = product<RN>(m, add_product(ke, h, left ? irL : irR) + q);
+        f.a[2] = add_product(P, D, add_product(q, sm, v));
         f.a[3] = product<RN>(m, t1);
         f.a[4] = product<RN>(m, t2);
     }

@@ -35,45 +35,44 @@ __global__ void __launch_bounds__(256) cyl_source_kernel(double *__restrict__ q,
         double *base = q + x;
         const double r = rin + column_of(x, nx) * dr;
         const double rho = base[0];
+        const auto step = [&](auto over_r, auto over_rho) {
+            double u = over_rho(base[2 * slab]);  // v_r
+            double v = over_rho(base[3 * slab]);  // v_theta
+            double diffmom = over_r(dt * v);
+            double vrA = u + kGL11 * v * diffmom;
+            double vphiA = v - kGL11 * u * diffmom;
+            double vrB = u + kGL12 * v * diffmom;
+            double vphiB = v - kGL12 * u * diffmom;
+#pragma unroll
+            for (int it = 0; it < 2; it++) {
+                diffmom = over_r(dt * vphiA);
+                const double diffmomB = over_r(dt * vphiB);
+                double scratch = vrA;
+                vrA = u + kGL11 * vphiA * diffmom + kGL12 * vphiB * diffmomB;
+                vphiA = v - kGL11 * scratch * diffmom + kGL12 * vrB * diffmomB;
+                diffmom = over_r(dt * vphiA);
+                scratch = vrB;
+                vrB = u + kGL21 * vphiA * diffmom + kGL22 * vphiB * diffmomB;
+                vphiB = v - kGL21 * scratch * diffmom + kGL22 * scratch * diffmomB;
+            }
+            u = rho * (u + over_r(.5 * dt * (vphiA * vphiA + vphiB * vphiB)));
+            v = rho * (v - over_r(.5 * dt * (vphiA * vrA + vphiB * vrB)));
+            const double E = base[slab];
+            const double w = base[4 * slab];
+            const double newP = E - over_rho(.5 * (u * u + v * v + w * w));
+            if (newP <= 0.0) base[slab] = .5 * (u * u + v * v + w * w) / rho + .00001 * rho;
+            base[2 * slab] = u;
+            base[3 * slab] = v;
+        };
+        const auto over_r = [&](double a) { return a / r; };
+        const auto over_rho = [&](double a) { return a / rho; };
 #ifdef IB_STRICT_ARITH
-        auto over_r = [&](double a) { return a / r; };
-        double u = base[2 * slab] / rho;  // v_r
-        double v = base[3 * slab] / rho;  // v_theta
+        step(over_r, over_rho);
 #else
         const double ir = rcp_fast(r), irho = rcp_fast(rho);
-        auto over_r = [&](double a) { return quotient_fast(a, r, ir); };
-        double u = quotient_fast(base[2 * slab], rho, irho);
-        double v = quotient_fast(base[3 * slab], rho, irho);
+        if (rcp_outside(r) || rcp_outside(rho)) step(over_r, over_rho);
+        else step([&](double a) { return quotient_fast(a, r, ir); }, [&](double a) { return quotient_fast(a, rho, irho); });
 #endif
-        double diffmom = over_r(dt * v);
-        double vrA = u + kGL11 * v * diffmom;
-        double vphiA = v - kGL11 * u * diffmom;
-        double vrB = u + kGL12 * v * diffmom;
-        double vphiB = v - kGL12 * u * diffmom;
-#pragma unroll
-        for (int it = 0; it < 2; it++) {
-            diffmom = over_r(dt * vphiA);
-            const double diffmomB = over_r(dt * vphiB);
-            double scratch = vrA;
-            vrA = u + kGL11 * vphiA * diffmom + kGL12 * vphiB * diffmomB;
-            vphiA = v - kGL11 * scratch * diffmom + kGL12 * vrB * diffmomB;
-            diffmom = over_r(dt * vphiA);
-            scratch = vrB;
-            vrB = u + kGL21 * vphiA * diffmom + kGL22 * vphiB * diffmomB;
-            vphiB = v - kGL21 * scratch * diffmom + kGL22 * scratch * diffmomB;
-        }
-        u = rho * (u + over_r(.5 * dt * (vphiA * vphiA + vphiB * vphiB)));
-        v = rho * (v - over_r(.5 * dt * (vphiA * vrA + vphiB * vrB)));
-        const double E = base[slab];
-        const double w = base[4 * slab];
-#ifdef IB_STRICT_ARITH
-        const double newP = E - .5 * (u * u + v * v + w * w) / rho;
-#else
-        const double newP = E - quotient_fast(.5 * (u * u + v * v + w * w), rho, irho);
-#endif
-        if (newP <= 0.0) base[slab] = .5 * (u * u + v * v + w * w) / rho + .00001 * rho;
-        base[2 * slab] = u;
-        base[3 * slab] = v;
     }
 }
 

@@ -39,10 +39,10 @@ __device__ __forceinline__ double allregime_cdrag(double Re, double Kn)
 #ifdef IB_STRICT_ARITH
     double cunningham = 1 + Kn * (1.142 + 1 * 0.558 * exp(-0.999 / Kn));
     double C_drag = (3 / Re + .45 * pow_of(pow_base(Re), -.319) + .0509 * Re / (8710 + Re)) / cunningham;
-#else  // the reciprocals of ib_fast.cuh (Kn is zero in gas without internal energy)
-    double cunningham = 1 + Kn * (1.142 + 1 * 0.558 * exp(-0.999 * rcp_fast_pos(Kn)));
-    double C_drag = (3 * rcp_fast_pos(Re) + .45 * pow_of(pow_base(Re), -.319) + .0509 * Re * rcp_fast(8710 + Re)) *
-                    rcp_fast(cunningham);
+#else
+    double cunningham = 1 + Kn * (1.142 + 1 * 0.558 * exp(-0.999 * rcp_full(Kn)));
+    double C_drag = (3 * rcp_full(Re) + .45 * pow_of(pow_base(Re), -.319) + .0509 * Re * rcp_full(8710 + Re)) *
+                    rcp_full(cunningham);
 #endif
     return C_drag;
 }
@@ -58,7 +58,7 @@ __device__ __forceinline__ double drag_k(const DragParams &d, double rhoA, doubl
 #ifdef IB_STRICT_ARITH
     double Kn = d.beta * pow_of(bT, d.lampow) / rhoA;
 #else
-    double Kn = d.beta * pow_of(bT, d.lampow) * rcp_fast(rhoA);
+    double Kn = d.beta * pow_of(bT, d.lampow) * rcp_full(rhoA);
 #endif
     double Cd_hat = allregime_cdrag(Re, Kn);
     return Cd_hat * magdv * (rhoA + rhoB) * d.epsilon;
@@ -75,7 +75,7 @@ __device__ __forceinline__ double logtrap_keff(const DragParams &d, double g0, d
 #ifdef IB_STRICT_ARITH
     mu = d0 / (g0 + d0);
 #else
-    mu = d0 * rcp_fast(g0 + d0);
+    mu = d0 * rcp_full(g0 + d0);
 #endif
     k = drag_k(d, g0, d0, t0, t1, skip);
     t2 = skip ? 0 : k;
@@ -126,7 +126,7 @@ __device__ __forceinline__ void drag_features(double g0, double gE, double g2, d
     magdv = sqrt(dvsq);
     u = press / g0;
 #else  // the two density reciprocals once instead of eight divisions
-    const double ig = rcp_fast(g0), id = rcp_fast(d0);
+    const double ig = rcp_full(g0), id = rcp_full(d0);
     dv = g2 * ig - d2 * id;
     dvsq = dv * dv;
     dv = g3 * ig - d3 * id;
@@ -134,7 +134,7 @@ __device__ __forceinline__ void drag_features(double g0, double gE, double g2, d
     dv = g4 * ig - d4 * id;
     dvsq += dv * dv;
     press = (gE - .5 * (g2 * g2 + g3 * g3 + g4 * g4) * ig);
-    magdv = sqrt_fast(dvsq);
+    magdv = sqrt_full(dvsq);
     u = press * ig;
 #endif
 }
@@ -154,10 +154,10 @@ __device__ __forceinline__ void drag_apply(double *g, double *ds, int64_t S, dou
     auto over_sum = [&](double x) { return x / (g0 + d0); };
     auto over_d0 = [&](double x) { return x / d0; };
 #else  // three reciprocals instead of nine divisions
-    const double isum = rcp_fast(g0 + d0), rhodinv = rcp_fast(d0);
+    const double isum = rcp_full(g0 + d0), rhodinv = rcp_full(d0);
     mu = d0 * isum;
     mu = mu * g0;
-    rhoginv = rcp_fast(g0);
+    rhoginv = rcp_full(g0);
     auto over_sum = [&](double x) { return x * isum; };
     auto over_d0 = [&](double x) { return x * rhodinv; };
 #endif

@@ -165,7 +165,7 @@ __device__ __forceinline__ void drag_apply_learned(double *g, double *ds, int64_
                                                    const double gm[3], double d0, const double dm[3],
                                                    const double dvv[3], double rdi, double decay)
 {
-    const double rsum = rcp_fast(g0 + d0);
+    const double rsum = rcp_full(g0 + d0);
     const double mu = g0 * d0 * rsum;
     double pd = 0;
 #pragma unroll
@@ -251,8 +251,8 @@ __global__ void __launch_bounds__(LT, 5) mlp_tc_kernel(LearnedArgs a)
             // the next tile's values stream in behind this tile's MMAs and update
             const int64_t inext = i + (int64_t)gridDim.x * LT;
             if (inext < a.n) stage_cell(s, a, inext);
-            const double rgi = rcp_fast(g0);
-            rdi = rcp_fast(d0);
+            const double rgi = rcp_full(g0);
+            rdi = rcp_full(d0);
             double dvsq = 0, momsq = 0;
 #pragma unroll
             for (int k = 0; k < 3; k++) {
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(LT, 5) mlp_tc_kernel(LearnedArgs a)
                 dvsq += dvv[k] * dvv[k];
                 momsq += gm[k] * gm[k];
             }
-            magdv = sqrt_fast(dvsq);
+            magdv = sqrt_full(dvsq);
             const double u = (gE - .5 * momsq * rgi) * rgi;
             const float raw[5] = {logf((float)g0), logf((float)d0), logf((float)magdv), logf((float)u),
                                   logf((float)a.dt)};

@@ -38,8 +38,9 @@ struct DuoGeo {
 
 // NS sweeps of the cells (ua, ub) of this thread, in place.  planes: 15 TT values of FT; SS: 10 TT
 // doubles, where u1 + u0 of the SSPRK average waits through the second stage.  All threads of the CTA
-// call it.
-template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO, bool RN = false>
+// call it.  OPS: FastOps (the caller tests the resulting densities, density_suspect) or IeeeOps.
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO, bool RN = false,
+          typename OPS = FastOps>
 __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], bool act, const DuoPos &p, FT *planes,
                                            double *SS, double lambda, const FluidConsts<FT> &c, const DuoGeo &g)
 {
@@ -50,8 +51,8 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
         FT *P = planes + (s % 3) * 5 * TT, *Q = planes + ((s + 1) % 3) * 5 * TT, *R = planes + ((s + 2) % 3) * 5 * TT;
         V5<FT> wa, wb;
         if (act) {
-            wa = stage_prims<METHOD, DIR, FT, RN>(second ? va : ua, c);  // HLL floors its argument
-            wb = stage_prims<METHOD, DIR, FT, RN>(second ? vb : ub, c);
+            wa = stage_prims<METHOD, DIR, FT, RN, OPS>(second ? va : ua, c);  // HLL floors its argument
+            wb = stage_prims<METHOD, DIR, FT, RN, OPS>(second ? vb : ub, c);
 #pragma unroll
             for (int k = 0; k < 5; k++) {
                 P[k * TT + p.own] = wa.a[k];
@@ -77,7 +78,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
                 const FT wl = (ODD && p.first) ? P[k * TT + p.left] : Q[k * TT + p.left];
                 const FT wr = (ODD && p.ghost) ? Q[k * TT + p.right] : P[k * TT + p.right];
                 const FT dl = wa.a[k] - wl, dm = wb.a[k] - wa.a[k], dr = wr - wb.a[k];
-                const FT ha = slope_limit<SLOPE, FT>(dl, dm), hb = slope_limit<SLOPE, FT>(dm, dr);
+                const FT ha = slope_limit<SLOPE, FT, OPS>(dl, dm), hb = slope_limit<SLOPE, FT, OPS>(dm, dr);
                 FT la;
                 if (METHOD == IB_METHOD_HLLC && k == 1) {  // internal energy to pressure
                     la = product<RN>(c.gm1, wa.a[k] - ha);
@@ -96,7 +97,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
                 }
                 R[k * TT + p.own] = la;
             }
-            fm = stage_flux<METHOD, FT, RN>(c, ra, lb);
+            fm = stage_flux<METHOD, FT, RN, OPS>(c, ra, lb);
         }
         __syncthreads();
         V5<FT> fb;
@@ -104,7 +105,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
             V5<FT> lr;
 #pragma unroll
             for (int k = 0; k < 5; k++) lr.a[k] = R[k * TT + p.right];
-            fb = stage_flux<METHOD, FT, RN>(c, rb, lr);
+            fb = stage_flux<METHOD, FT, RN, OPS>(c, rb, lr);
 #pragma unroll
             for (int k = 0; k < 5; k++) P[k * TT + p.own] = (ODD && p.ghost) ? fm.a[k] : fb.a[k];
         }
@@ -138,6 +139,14 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
             }
         }
     }
+}
+
+// The same with the IEEE operations, out of line: its registers are not the caller's.
+template <int METHOD, int SLOPE, typename FT, int DIR, int TT, bool RN>
+__device__ __noinline__ void duo_sweep_ieee(double (&ua)[5], double (&ub)[5], DuoPos p, FT *planes, double *SS, double lambda,
+                                            FluidConsts<FT> c)
+{
+    duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE, RN, IeeeOps>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
 }
 
 // Dynamic shared memory of a CTA of TT threads: the planes and the SSPRK sums.
@@ -179,6 +188,7 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT)) duo_row_kernel(Swe
     p.ghost = ODD && t == T - 1;
     double ua[5], ub[5];
     double *q = a.q + row * n + 2 * t;
+    bool suspect = false;
 #pragma unroll
     for (int k = 0; k < 5; k++) ua[k] = ub[k] = 1.0;
     if (act) {
@@ -200,7 +210,15 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT)) duo_row_kernel(Swe
     DuoGeo g;
     if (GEO == CYL_RADIAL) { g.ra = a.crin + (2 * t) * a.cdr; g.rb = a.crin + (2 * t + 1) * a.cdr; g.dr = a.cdr; }
     duo_sweeps<METHOD, SLOPE, FT, 1, TT, NS, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
-    if (act) {
+    if constexpr (kPoison<FastOps, FT>) {
+        if (act) suspect = density_suspect(ua[0]) || (density_suspect(ub[0]) && !p.ghost);
+        suspect = __syncthreads_or(suspect);
+    }
+    if (suspect) {
+        if constexpr (kPoison<FastOps, FT>)
+            ieee_pencils<METHOD, SLOPE, 1, GEO>(
+                IeeePencils{a.q, a.slab, a.nx, a.ny, a.nz, (int64_t)blockIdx.x * rp, rp, NS, lambda, CylPencil{a.crin, a.cdr, 0, 0}}, c, SS);
+    } else if (act) {
         if (!ODD && vec) {
 #pragma unroll
             for (int k = 0; k < 5; k++)
@@ -255,8 +273,17 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT))
     }
     DuoGeo g;
     if (GEO != CYL_NONE) g.rpen = theta_radius(cyl, (int)(pencil % a.nx), (int)(pencil / a.nx));
+    bool suspect = false;
     duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
-    if (act) {
+    if constexpr (kPoison<FastOps, FT>) {
+        if (act) suspect = density_suspect(ua[0]) || (density_suspect(ub[0]) && !p.ghost);
+        suspect = __syncthreads_or(suspect);
+    }
+    if (suspect) {
+        if constexpr (kPoison<FastOps, FT>)
+            ieee_pencils<METHOD, SLOPE, DIR, GEO>(
+                IeeePencils{a.q, a.slab, a.nx, a.ny, a.nz, (int64_t)blockIdx.x * COLS, COLS, 1, lambda, cyl}, c, SS);
+    } else if (act) {
 #pragma unroll
         for (int k = 0; k < 5; k++) {
             q[(int64_t)slot_of<METHOD, DIR>(k) * a.slab] = ua[k];
@@ -359,9 +386,27 @@ __global__ void __launch_bounds__(R *W / 2, 512 / (R * W / 2))
         double ua[5], ub[5];
         fetch(2 * t, ua);
         fetch(2 * t + 1, ub);
-        __syncthreads();  // every thread has read tile buf (and is done with the planes)
+        const int g = c0 - 4 + 2 * t;
+        const bool own_a = g >= c0 && g < cend, own_b = g + 1 >= c0 && g + 1 < cend;
+        bool suspect = false;
+        if constexpr (kPoison<FastOps, FT>) suspect = density_suspect(ua[0]) || density_suspect(ub[0]);
+        duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
+        if constexpr (kPoison<FastOps, FT>) {
+            suspect = suspect || (own_a && density_suspect(ua[0])) || (own_b && density_suspect(ub[0]));
+            if (__syncthreads_or(suspect)) {
+                double xa[5], xb[5];
+                fetch(2 * t, xa);
+                fetch(2 * t + 1, xb);
+                duo_sweep_ieee<METHOD, SLOPE, FT, DIR, TT, false>(xa, xb, p, planes, SS, lambda, c);
+#pragma unroll
+                for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
+                __syncthreads();
+            }
+        } else {
+            __syncthreads();
+        }
+        // every thread is done with tile buf and the planes: request the job after next into the tile
         if (leader) {
-            // request the job after next into it
             const int64_t jn = j + 2 * step;
             if (jn < njobs_all) {
                 fence_proxy_async_smem();
@@ -369,14 +414,12 @@ __global__ void __launch_bounds__(R *W / 2, 512 / (R * W / 2))
                 issued |= 1u << buf;
             }
         }
-        duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
         double *base = a.q + chunk_base(a, DIR, W, grp, col);
-        const int g = c0 - 4 + 2 * t;
 #pragma unroll
         for (int k = 0; k < 5; k++) {
             double *cell = base + slots[k] * a.slab + (int64_t)g * a.rs;
-            if (g >= c0 && g < cend) cell[0] = ua[k];
-            if (g + 1 >= c0 && g + 1 < cend) cell[a.rs] = ub[k];
+            if (own_a) cell[0] = ua[k];
+            if (own_b) cell[a.rs] = ub[k];
         }
     }
 }

@@ -60,14 +60,141 @@ __device__ __forceinline__ int ens_nchunks(int n, int target)
     return nc;
 }
 
+// Stores after a chunk's inputs have been read: the previous chunk's last four outputs, this chunk's output m
+// (the last four, and the first chunk's first four, wait), and at the end those still waiting.  pend: two
+// buffers, so that a chunk's own outputs do not overwrite those of the chunk before.
+__device__ __forceinline__ void ens_store_pending(double *qb, int64_t S, int ch, int cb, int i, const double *pend)
+{
+    if (ch == 0 || i >= 4) return;
+    const double *p = pend + 20 * ((ch - 1) & 1);
+#pragma unroll
+    for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb - 4 + i] = p[k * 4 + i];
+}
+__device__ __forceinline__ void ens_store(double *qb, int64_t S, int ch, int cb, int len, bool single, int m,
+                                          const double (&out)[5], double *pend, double *first)
+{
+    if (!single && ch == 0 && m < 4) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) first[k * 4 + m] = out[k];
+    } else if (!single && m >= len - 4) {
+        double *p = pend + 20 * (ch & 1);
+#pragma unroll
+        for (int k = 0; k < 5; k++) p[k * 4 + m - (len - 4)] = out[k];
+    } else {
+#pragma unroll
+        for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb + m] = out[k];
+    }
+}
+__device__ __forceinline__ void ens_store_ends(double *qb, int64_t S, int n, int nchunks, int i, const double *pend,
+                                               const double *first)
+{
+    __syncthreads();
+    if (nchunks > 1 && i < 4) {
+        const double *p = pend + 20 * ((nchunks - 1) & 1);
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            qb[(int64_t)k * S + n - 4 + i] = p[k * 4 + i];
+            qb[(int64_t)k * S + i] = first[k * 4 + i];
+        }
+    }
+    __syncthreads();
+}
+
+// Both stages of one chunk, row i of its tr rows a thread, which keeps that cell's state u in registers: on
+// return u is the output of rows 4 .. tr - 5.  Two shared-memory planes of FT swap roles between the stages.
+template <int METHOD, int SLOPE, typename FT, typename OPS>
+__device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double lambda, const FluidConsts<FT> &c, FT *SA, FT *SB,
+                                           int TR)
+{
+    double u1[5];
+    V5<FT> keep;
+    // ---- stage A: prims and fluxes in SA, left faces in SB ----
+    if (i < tr) {
+        V5<FT> w = stage_prims<METHOD, 1, FT, false, OPS>(u, c);  // HLL floors u
+#pragma unroll
+        for (int k = 0; k < 5; k++) SA[k * TR + i] = w.a[k];
+    }
+    __syncthreads();
+    if (i >= 1 && i <= tr - 2) {
+        V5<FT> w, dl, dr, L;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            w.a[k] = SA[k * TR + i];
+            dl.a[k] = w.a[k] - SA[k * TR + i - 1];
+            dr.a[k] = SA[k * TR + i + 1] - w.a[k];
+        }
+        stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, keep);
+#pragma unroll
+        for (int k = 0; k < 5; k++) SB[k * TR + i] = L.a[k];
+    }
+    __syncthreads();
+    if (i >= 1 && i <= tr - 3) {
+        V5<FT> Lr;
+#pragma unroll
+        for (int k = 0; k < 5; k++) Lr.a[k] = SB[k * TR + i + 1];
+        keep = stage_flux<METHOD, FT, false, OPS>(c, keep, Lr);
+#pragma unroll
+        for (int k = 0; k < 5; k++) SA[k * TR + i] = keep.a[k];
+    }
+    __syncthreads();
+    if (i >= 2 && i <= tr - 3) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) u1[k] = u[k] - lambda * ((double)keep.a[k] - (double)SA[k * TR + i - 1]);
+    }
+    // ---- stage B: prims and fluxes in SB, left faces in SA (no barrier: stage A's last
+    // phase read SA only) ----
+    if (i >= 2 && i <= tr - 3) {
+        V5<FT> w = stage_prims<METHOD, 1, FT, false, OPS>(u1, c);  // HLL floors u1
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            SB[k * TR + i] = w.a[k];
+            u[k] = u1[k] + u[k];  // the output's (u1 + u0), rounded as it is there first
+        }
+    }
+    __syncthreads();
+    if (i >= 3 && i <= tr - 4) {
+        V5<FT> w, dl, dr, L;
+#pragma unroll
+        for (int k = 0; k < 5; k++) {
+            w.a[k] = SB[k * TR + i];
+            dl.a[k] = w.a[k] - SB[k * TR + i - 1];
+            dr.a[k] = SB[k * TR + i + 1] - w.a[k];
+        }
+        stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, keep);
+#pragma unroll
+        for (int k = 0; k < 5; k++) SA[k * TR + i] = L.a[k];
+    }
+    __syncthreads();
+    if (i >= 3 && i <= tr - 5) {
+        V5<FT> Lr;
+#pragma unroll
+        for (int k = 0; k < 5; k++) Lr.a[k] = SA[k * TR + i + 1];
+        keep = stage_flux<METHOD, FT, false, OPS>(c, keep, Lr);
+#pragma unroll
+        for (int k = 0; k < 5; k++) SB[k * TR + i] = keep.a[k];
+    }
+    __syncthreads();
+    if (i >= 4 && i <= tr - 5) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) u[k] = .5 * (u[k] - lambda * ((double)keep.a[k] - (double)SB[k * TR + i - 1]));
+    }
+}
+
+// The same with the IEEE operations, out of line: its registers are not the caller's
+template <int METHOD, int SLOPE, typename FT>
+__device__ __noinline__ void ens_stages_ieee(double (&u)[5], int i, int tr, double lambda, FluidConsts<FT> c, FT *SA, FT *SB,
+                                             int TR)
+{
+    ens_stages<METHOD, SLOPE, FT, IeeeOps>(u, i, tr, lambda, c, SA, SB, TR);
+}
+
 // One x sweep of a problem of n cells in nc chunks (ens_nchunks; the longest chunk + 8 <= lcap <= NT):
 // the tile sweep's in-place rules (each chunk loads its cells and 4 halo cells a side of the original
-// state; the last four outputs of a chunk wait in `pend` until the next chunk has loaded them, the
+// state; the last four outputs of a chunk wait in `pend` until the next chunk has been computed, the
 // first chunk's first four in `first` until the last chunk has read them through the periodic
-// wrap) with the row kernel's phases: tile row i of a chunk is thread i, which keeps that cell's
-// state in registers through both stages; two shared-memory planes of FT swap roles between the
-// stages, so a chunk takes seven barriers.  The arithmetic is the library's sweep arithmetic
-// (stage_prims / stage_faces / stage_flux), so the results are those of the tile sweep.
+// wrap).  A chunk's inputs stay in memory until its outputs have been tested (density_suspect), so that it can be
+// computed again with the IEEE operations.  The arithmetic is the library's sweep arithmetic (stage_prims /
+// stage_faces / stage_flux), so the results are those of the tile sweep.
 template <int METHOD, int SLOPE, typename FT, int NT>
 __device__ __forceinline__ void ens_sweep(double *qb, int64_t S, int n, int nchunks, double lambda,
                                           const FluidConsts<FT> &c, FT *SA, FT *SB, int TR, double *pend,
@@ -79,113 +206,37 @@ __device__ __forceinline__ void ens_sweep(double *qb, int64_t S, int n, int nchu
         const int cb = (int)((int64_t)ch * n / nchunks);
         const int len = (int)((int64_t)(ch + 1) * n / nchunks) - cb;
         const int tr = len + 8;
-        double u0[5], u1[5];
-        V5<FT> keep;
-        if (i < tr) {
-            const int cell = mod_n(cb - 4 + i, n);
+        auto fetch = [&](double (&u)[5]) {
+            if (i < tr) {
+                const int cell = mod_n(cb - 4 + i, n);
 #pragma unroll
-            for (int k = 0; k < 5; k++) u0[k] = qb[(int64_t)k * S + cell];
-        }
-        __syncthreads();  // this chunk has loaded the original state of its halo
-        if (ch > 0 && i < 4) {
-#pragma unroll
-            for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb - 4 + i] = pend[k * 4 + i];
-        }
-        // ---- stage A: prims and fluxes in SA, left faces in SB ----
-        if (i < tr) {
-            V5<FT> w = stage_prims<METHOD, 1, FT>(u0, c);  // HLL floors u0
-#pragma unroll
-            for (int k = 0; k < 5; k++) SA[k * TR + i] = w.a[k];
-        }
-        __syncthreads();
-        if (i >= 1 && i <= tr - 2) {
-            V5<FT> w, dl, dr, L;
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                w.a[k] = SA[k * TR + i];
-                dl.a[k] = w.a[k] - SA[k * TR + i - 1];
-                dr.a[k] = SA[k * TR + i + 1] - w.a[k];
+                for (int k = 0; k < 5; k++) u[k] = qb[(int64_t)k * S + cell];
             }
-            stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, keep);
+        };
+        double out[5];
+        fetch(out);
+        const bool mine = i >= 4 && i <= tr - 5;
+        bool suspect = false;
+        if constexpr (kPoison<FastOps, FT>) suspect = i < tr && density_suspect(out[0]);
+        ens_stages<METHOD, SLOPE, FT, FastOps>(out, i, tr, lambda, c, SA, SB, TR);
+        if constexpr (kPoison<FastOps, FT>) {
+            suspect = suspect || (mine && density_suspect(out[0]));
+            if (__syncthreads_or(suspect)) {
+                double x[5];
+                fetch(x);
+                ens_stages_ieee<METHOD, SLOPE, FT>(x, i, tr, lambda, c, SA, SB, TR);
 #pragma unroll
-            for (int k = 0; k < 5; k++) SB[k * TR + i] = L.a[k];
-        }
-        __syncthreads();
-        if (i >= 1 && i <= tr - 3) {
-            V5<FT> Lr;
-#pragma unroll
-            for (int k = 0; k < 5; k++) Lr.a[k] = SB[k * TR + i + 1];
-            keep = stage_flux<METHOD, FT>(c, keep, Lr);
-#pragma unroll
-            for (int k = 0; k < 5; k++) SA[k * TR + i] = keep.a[k];
-        }
-        __syncthreads();
-        if (i >= 2 && i <= tr - 3) {
-#pragma unroll
-            for (int k = 0; k < 5; k++) u1[k] = u0[k] - lambda * ((double)keep.a[k] - (double)SA[k * TR + i - 1]);
-        }
-        // ---- stage B: prims and fluxes in SB, left faces in SA (no barrier: stage A's last
-        // phase read SA only) ----
-        if (i >= 2 && i <= tr - 3) {
-            V5<FT> w = stage_prims<METHOD, 1, FT>(u1, c);  // HLL floors u1
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                SB[k * TR + i] = w.a[k];
-                u0[k] = u1[k] + u0[k];  // the output's (u1 + u0), rounded as it is there first
+                for (int k = 0; k < 5; k++) out[k] = x[k];
+                __syncthreads();
             }
+        } else {
+            __syncthreads();
         }
-        __syncthreads();
-        if (i >= 3 && i <= tr - 4) {
-            V5<FT> w, dl, dr, L;
-#pragma unroll
-            for (int k = 0; k < 5; k++) {
-                w.a[k] = SB[k * TR + i];
-                dl.a[k] = w.a[k] - SB[k * TR + i - 1];
-                dr.a[k] = SB[k * TR + i + 1] - w.a[k];
-            }
-            stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, keep);
-#pragma unroll
-            for (int k = 0; k < 5; k++) SA[k * TR + i] = L.a[k];
-        }
-        __syncthreads();
-        if (i >= 3 && i <= tr - 5) {
-            V5<FT> Lr;
-#pragma unroll
-            for (int k = 0; k < 5; k++) Lr.a[k] = SA[k * TR + i + 1];
-            keep = stage_flux<METHOD, FT>(c, keep, Lr);
-#pragma unroll
-            for (int k = 0; k < 5; k++) SB[k * TR + i] = keep.a[k];
-        }
-        __syncthreads();
-        if (i >= 4 && i <= tr - 5) {
-            const int m = i - 4;  // output cell cb + m
-            double out[5];
-#pragma unroll
-            for (int k = 0; k < 5; k++)
-                out[k] = .5 * (u0[k] - lambda * ((double)keep.a[k] - (double)SB[k * TR + i - 1]));
-            if (!single && ch == 0 && m < 4) {
-#pragma unroll
-                for (int k = 0; k < 5; k++) first[k * 4 + m] = out[k];
-            } else if (!single && m >= len - 4) {
-#pragma unroll
-                for (int k = 0; k < 5; k++) pend[k * 4 + m - (len - 4)] = out[k];
-            } else {
-#pragma unroll
-                for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb + m] = out[k];
-            }
-        }
-        // the next chunk's first barrier separates these reads of SB and writes of pend from its
-        // stage A
+        // every thread has read this chunk's inputs and is done with the planes
+        ens_store_pending(qb, S, ch, cb, i, pend);
+        if (mine) ens_store(qb, S, ch, cb, len, single, i - 4, out, pend, first);
     }
-    __syncthreads();
-    if (!single && i < 4) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            qb[(int64_t)k * S + n - 4 + i] = pend[k * 4 + i];
-            qb[(int64_t)k * S + i] = first[k * 4 + i];
-        }
-    }
-    __syncthreads();
+    ens_store_ends(qb, S, n, nchunks, i, pend, first);
 }
 
 // The same sweep with two rows a thread: thread t computes rows 2t and 2t + 1 of a chunk (ib_duo.cuh; the edge
@@ -214,38 +265,30 @@ __device__ __forceinline__ void ens_sweep_two(double *qb, int64_t S, int n, int 
         double ua[5], ub[5];
         fetch(2 * t, ua);
         fetch(2 * t + 1, ub);
-        __syncthreads();  // this chunk has loaded the original state of its halo (and is done with the planes)
-        if (ch > 0 && t < 4) {
-#pragma unroll
-            for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb - 4 + t] = pend[k * 4 + t];
-        }
+        const bool own_a = 2 * t >= 4 && 2 * t <= tr - 5, own_b = 2 * t + 1 >= 4 && 2 * t + 1 <= tr - 5;
+        bool suspect = false;
+        if constexpr (kPoison<FastOps, FT>) suspect = density_suspect(ua[0]) || density_suspect(ub[0]);
         duo_sweeps<METHOD, SLOPE, FT, 1, TT, 1, false, CYL_NONE, true>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
-        auto store = [&](int i, const double (&out)[5]) {
-            const int m = i - 4;  // output cell cb + m
-            if (m < 0 || m >= len) return;
-            if (!single && ch == 0 && m < 4) {
+        if constexpr (kPoison<FastOps, FT>) {
+            suspect = suspect || (own_a && density_suspect(ua[0])) || (own_b && density_suspect(ub[0]));
+            if (__syncthreads_or(suspect)) {
+                double xa[5], xb[5];
+                fetch(2 * t, xa);
+                fetch(2 * t + 1, xb);
+                duo_sweep_ieee<METHOD, SLOPE, FT, 1, TT, true>(xa, xb, p, planes, SS, lambda, c);
 #pragma unroll
-                for (int k = 0; k < 5; k++) first[k * 4 + m] = out[k];
-            } else if (!single && m >= len - 4) {
-#pragma unroll
-                for (int k = 0; k < 5; k++) pend[k * 4 + m - (len - 4)] = out[k];
-            } else {
-#pragma unroll
-                for (int k = 0; k < 5; k++) qb[(int64_t)k * S + cb + m] = out[k];
+                for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
+                __syncthreads();
             }
-        };
-        store(2 * t, ua);
-        store(2 * t + 1, ub);
-    }
-    __syncthreads();
-    if (!single && t < 4) {
-#pragma unroll
-        for (int k = 0; k < 5; k++) {
-            qb[(int64_t)k * S + n - 4 + t] = pend[k * 4 + t];
-            qb[(int64_t)k * S + t] = first[k * 4 + t];
+        } else {
+            __syncthreads();
         }
+        // every thread has read this chunk's inputs and is done with the planes
+        ens_store_pending(qb, S, ch, cb, t, pend);
+        if (own_a) ens_store(qb, S, ch, cb, len, single, 2 * t - 4, ua, pend, first);
+        if (own_b) ens_store(qb, S, ch, cb, len, single, 2 * t - 3, ub, pend, first);
     }
-    __syncthreads();
+    ens_store_ends(qb, S, n, nchunks, t, pend, first);
 }
 
 // One row a thread: three CTAs of 256 threads per SM (80 registers) rather than four: at 64 registers a
@@ -263,8 +306,8 @@ __global__ void __launch_bounds__(TWO ? NT / 2 : NT,
     __shared__ double s_red[TT / 32];
     __shared__ double s_dt;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    double *pend = tsm;        // [5][4]
-    double *first = tsm + 20;  // [5][4]
+    double *pend = tsm;        // [2][5][4]
+    double *first = tsm + 40;  // [5][4]
     for (;;) {
         if (tid == 0) {
             const unsigned k = atomicAdd(a.counter, 1u);
@@ -314,11 +357,11 @@ __global__ void __launch_bounds__(TWO ? NT / 2 : NT,
             const double lambda = dt / h;
             for (int half = 0; half < 2; half++) {
                 if constexpr (TWO) {
-                    double *SS = tsm + 40;  // the SSPRK sums, then the planes
+                    double *SS = tsm + 60;  // the SSPRK sums, then the planes
                     ens_sweep_two<METHOD, SLOPE, FT, TT>(qb, a.S, n, nc, lambda, c,
                                                          reinterpret_cast<FT *>(SS + 10 * TT), SS, pend, first);
                 } else {
-                    FT *SA = reinterpret_cast<FT *>(tsm + 40);  // [5][lcap]
+                    FT *SA = reinterpret_cast<FT *>(tsm + 60);  // [5][lcap]
                     ens_sweep<METHOD, SLOPE, FT, NT>(qb, a.S, n, nc, lambda, c, SA, SA + 5 * a.lcap, a.lcap, pend, first);
                 }
                 if (tid == 0) ens_boundary(qb, a.S, n, a.bc0, a.bc1);
@@ -343,7 +386,7 @@ __global__ void __launch_bounds__(TWO ? NT / 2 : NT,
 template <typename FT, int NT, bool TWO>
 static size_t ens_smem(int lcap)
 {
-    return sizeof(double) * 40 + (TWO ? duo_smem_bytes<FT, NT / 2>() : sizeof(FT) * 10 * (size_t)lcap);
+    return sizeof(double) * 60 + (TWO ? duo_smem_bytes<FT, NT / 2>() : sizeof(FT) * 10 * (size_t)lcap);
 }
 
 template <int METHOD, int SLOPE, typename FT, int NT, bool TWO>

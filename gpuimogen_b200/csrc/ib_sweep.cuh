@@ -39,7 +39,7 @@ __device__ __forceinline__ V5<FT> v5_sub(const V5<FT> &a, const V5<FT> &b)
 // HLL primitives: [rho, v_n, P, v_t1, v_t2] with P taken from the floored pressure
 // (cudaFluidStep.cu:1864-1888).  irho: 1 / rho, product build (one reciprocal for the five quotients of
 // the pressure solver and the velocities; the strict build divides as the reference does)
-template <typename FT, bool RN = false>
+template <typename FT, bool RN = false, typename OPS = GuardedOps>
 __device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2, FT irho)
 {
     V5<FT> w;
@@ -53,17 +53,22 @@ __device__ __forceinline__ V5<FT> hll_prims(FT rho, FT pn, FT P, FT pt1, FT pt2,
     w.a[1] = product<RN>(pn, irho);
     w.a[3] = product<RN>(pt1, irho);
     w.a[4] = product<RN>(pt2, irho);
+    if (!std::is_same<OPS, FastOps>::value && rcp_outside(rho)) {
+        w.a[1] = divide_ieee(pn, rho);
+        w.a[3] = divide_ieee(pt1, rho);
+        w.a[4] = divide_ieee(pt2, rho);
+    }
 #endif
     return w;
 }
 
-template <int SLOPE, typename FT>
+template <int SLOPE, typename FT, typename OPS = FastOps>
 __device__ __forceinline__ void hll_faces(const V5<FT> &w, const V5<FT> &dl, const V5<FT> &dr,
                                           V5<FT> &L, V5<FT> &R)
 {
 #pragma unroll
     for (int k = 0; k < 5; k++) {
-        FT s = slope_limit<SLOPE, FT>(dl.a[k], dr.a[k]);
+        FT s = slope_limit<SLOPE, FT, OPS>(dl.a[k], dr.a[k]);
         R.a[k] = w.a[k] + s;
         L.a[k] = w.a[k] - s;
     }
@@ -71,7 +76,8 @@ __device__ __forceinline__ void hll_faces(const V5<FT> &w, const V5<FT> &dl, con
 
 // HLL flux (cudaFluidStep.cu:2057-2198).  le = right face of the left cell, re = left face of
 // the right cell, both [rho, v_n, P, v_t1, v_t2].  Output [rho, E, p_n, p_t1, p_t2].
-template <typename FT, bool RN = false>
+// With the short forms the mass flux is NaN wherever one of them is.
+template <typename FT, bool RN = false, typename OPS = IeeeOps>
 __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT> &le, const V5<FT> &re)
 {
     const FT Ale = le.a[0], Ble = le.a[1], Cle = le.a[2], Dle = le.a[3], Ele = le.a[4];
@@ -80,17 +86,23 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
     FT sl, sr;
     const bool iso = !(c.isotemp == (FT)-1);
     if (!iso) {
-        einfeldt<FT>(c, Ale, Ble, Cle, Are, Bre, Cre, Utilde * Utilde + Sleft * Sleft + Sright * Sright, sl, sr);
+        const FT dvsq = square_sum(Utilde, Sleft, Sright);
+#ifdef IB_STRICT_ARITH
+        einfeldt<FT>(c, Ale, Ble, Cle, Are, Bre, Cre, dvsq, sl, sr);
+#else
+        FT irL, irR;
+        einfeldt<OPS, FT>(c, Ale, Ble, Cle, Are, Bre, Cre, dvsq, sl, sr, irL, irR);
+#endif
     } else {
         // the isothermal bound receives c_iso^2 where a speed is expected (cudaFluidStep.cu:2131)
-        einfeldt_iso<FT>(Ale, Ble, Are, Bre, c.isotempsq, sl, sr);
+        einfeldt_iso<OPS, FT>(Ale, Ble, Are, Bre, c.isotempsq, sl, sr);
     }
     Sleft = sl;
     Sright = sr;
 #ifdef IB_STRICT_ARITH
     FT Atilde = 1 / (Sright - Sleft);
 #else
-    FT Atilde = rcp_fast(Sright - Sleft);
+    FT Atilde = OPS::rcp(Sright - Sleft);
 #endif
     FT Fa = product<RN>(Ale, Ble);
     FT Fb = product<RN>(Are, Bre);
@@ -98,51 +110,53 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
     int mode = 1;
     if (Sleft >= 0) mode = 0;
     if (Sright <= 0) mode = 2;
+    if (kPoison<OPS, FT> && !(Sright >= Sleft)) mode = 1;  // a NaN among the speeds: not dropped
     if (mode == 0) {
         f.a[0] = Fa;
         if (!iso) {
-            f.a[1] = product<RN>(Ble, (c.govergm1 * Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele)));
-            f.a[2] = Fa * Ble + Cle;
+            f.a[1] = product<RN>(Ble, sum_products(c.govergm1, Cle, (FT).5 * Ale, square_sum(Ble, Dle, Ele)));
+            f.a[2] = add_product(Cle, Fa, Ble);
         } else {
-            f.a[1] = product<RN>(Ble, (Cle + (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele)));
-            f.a[2] = Fa * Ble + c.isotempsq * Ale;
+            f.a[1] = product<RN>(Ble, add_product(Cle, (FT).5 * Ale, square_sum(Ble, Dle, Ele)));
+            f.a[2] = sum_products(Fa, Ble, c.isotempsq, Ale);
         }
         f.a[3] = product<RN>(Fa, Dle);
         f.a[4] = product<RN>(Fa, Ele);
     } else if (mode == 1) {
-        f.a[0] = product<RN>((Sright * (Ble - Sleft) * Ale - Sleft * (Bre - Sright) * Are), Atilde);
+        const FT wl = Sright * (Ble - Sleft), wr = Sleft * (Bre - Sright);
+        f.a[0] = product<RN>(diff_products(wl, Ale, wr, Are), Atilde);
         if (!iso) {
-            f.a[2] = product<RN>((Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb + Sright * Cle - Sleft * Cre), Atilde);
+            f.a[2] = product<RN>(sub_product(add_product(diff_products(wl, Fa, wr, Fb), Sright, Cle), Sleft, Cre), Atilde);
         } else {
-            f.a[2] = product<RN>((Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb +
-                      c.isotempsq * (Sright * Ale - Sleft * Are)), Atilde);
+            f.a[2] = product<RN>(add_product(diff_products(wl, Fa, wr, Fb), c.isotempsq, diff_products(Sright, Ale, Sleft, Are)),
+                                 Atilde);
         }
-        f.a[3] = product<RN>((Sright * (Ble - Sleft) * Ale * Dle - Sleft * (Bre - Sright) * Are * Dre), Atilde);
-        f.a[4] = product<RN>((Sright * (Ble - Sleft) * Ale * Ele - Sleft * (Bre - Sright) * Are * Ere), Atilde);
+        f.a[3] = product<RN>(diff_products(wl * Ale, Dle, wr * Are, Dre), Atilde);
+        f.a[4] = product<RN>(diff_products(wl * Ale, Ele, wr * Are, Ere), Atilde);
         if (!iso) {
-            Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele);
-            Fb = (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere);
-            FT e = (Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb);
+            Fa = (FT).5 * Ale * square_sum(Ble, Dle, Ele);
+            Fb = (FT).5 * Are * square_sum(Bre, Dre, Ere);
+            FT e = diff_products(wl, Fa, wr, Fb);
 #ifdef IB_STRICT_ARITH
             const FT dp = Sleft * Sright * (Cre - Cle) / c.gm1;
 #else
             const FT dp = Sleft * Sright * (Cre - Cle) * c.rgm1;
 #endif
-            f.a[1] = product<RN>((e + (c.govergm1 * (Sright * Cle * Ble - Sleft * Cre * Bre) + dp)), Atilde);
+            f.a[1] = product<RN>(e + add_product(dp, c.govergm1, diff_products(Sright * Cle, Ble, Sleft * Cre, Bre)), Atilde);
         } else {
             // isothermal energy flux lacks the 1/(S_R-S_L) factor (cudaFluidStep.cu:2178-2182)
-            Fa = (FT).5 * Ale * (Ble * Ble + Dle * Dle + Ele * Ele) + Cle;
-            Fb = (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere) + Cre;
-            f.a[1] = (Sright * (Ble - Sleft) * Fa - Sleft * (Bre - Sright) * Fb);
+            Fa = add_product(Cle, (FT).5 * Ale, square_sum(Ble, Dle, Ele));
+            Fb = add_product(Cre, (FT).5 * Are, square_sum(Bre, Dre, Ere));
+            f.a[1] = diff_products(wl, Fa, wr, Fb);
         }
     } else {
         f.a[0] = Fb;
         if (!iso) {
-            f.a[1] = product<RN>(Bre, (c.govergm1 * Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere)));
-            f.a[2] = Fb * Bre + Cre;
+            f.a[1] = product<RN>(Bre, sum_products(c.govergm1, Cre, (FT).5 * Are, square_sum(Bre, Dre, Ere)));
+            f.a[2] = add_product(Cre, Fb, Bre);
         } else {
-            f.a[1] = product<RN>(Bre, (Cre + (FT).5 * Are * (Bre * Bre + Dre * Dre + Ere * Ere)));
-            f.a[2] = Fb * Bre + c.isotemp * Are;  // c_iso, not c_iso^2 (cudaFluidStep.cu:2191)
+            f.a[1] = product<RN>(Bre, add_product(Cre, (FT).5 * Are, square_sum(Bre, Dre, Ere)));
+            f.a[2] = sum_products(Fb, Bre, c.isotemp, Are);  // c_iso, not c_iso^2 (cudaFluidStep.cu:2191)
         }
         f.a[3] = product<RN>(Fb, Dre);
         f.a[4] = product<RN>(Fb, Ere);
@@ -153,33 +167,25 @@ __device__ __forceinline__ V5<FT> hll_flux(const FluidConsts<FT> &c, const V5<FT
 // HLL pressure solver with floors (cukern_PressureSolverHydro, cudaFluidStep.cu:2813-2864) on a
 // conserved state in local order u = [rho, E, p_n, p_t1, p_t2]; mom[m] = local index of memory
 // slab 2+m (the reference sums px, py, pz in slab order).  Returns P and 1 / rho, modifies u.
-template <int DIR>
+template <int DIR, typename OPS = GuardedOps>
 __device__ __forceinline__ double hll_pressure(double u[5], double minmass, double mintemp, double gm1, double &irho)
 {
     // local index of memory slabs 2,3,4 under HllSlots<DIR>
     constexpr int m2 = (HllSlots<DIR>::n == 2) ? 2 : ((HllSlots<DIR>::t1 == 2) ? 3 : 4);
     constexpr int m3 = (HllSlots<DIR>::n == 3) ? 2 : ((HllSlots<DIR>::t1 == 3) ? 3 : 4);
     constexpr int m4 = (HllSlots<DIR>::n == 4) ? 2 : ((HllSlots<DIR>::t1 == 4) ? 3 : 4);
-    double rho = u[0], E, z, momsq, P;
+    double rho = u[0], E, momsq, P;
     if (rho < minmass) {
         P = minmass / rho;
         rho = u[0] = minmass;
         E = u[1] = P * u[1];
-        z = u[m2] = P * u[m2];
-        momsq = z * z;
-        z = u[m3] = P * u[m3];
-        momsq += z * z;
-        z = u[m4] = P * u[m4];
-        momsq += z * z;
+        u[m2] = P * u[m2];
+        u[m3] = P * u[m3];
+        u[m4] = P * u[m4];
     } else {
         E = u[1];
-        z = u[m2];
-        momsq = z * z;
-        z = u[m3];
-        momsq += z * z;
-        z = u[m4];
-        momsq += z * z;
     }
+    momsq = square_sum(u[m2], u[m3], u[m4]);
 #ifdef IB_STRICT_ARITH
     irho = 0.0;
     P = E - .5 * momsq / rho;
@@ -189,11 +195,12 @@ __device__ __forceinline__ double hll_pressure(double u[5], double minmass, doub
     }
 #else
     irho = rcp_fast(rho);
-    const double ke = .5 * momsq * irho;
-    P = E - ke;
+    double ke = .5 * momsq, q = irho;
+    if (!std::is_same<OPS, FastOps>::value && rcp_outside(rho)) { ke = divide_ieee(ke, rho); q = 1.0; }
+    P = sub_product(E, ke, q);
     if (P < rho * mintemp) {
         P = mintemp * rho;
-        u[1] = ke + P;
+        u[1] = add_product(P, ke, q);
     }
 #endif
     return P * gm1;
@@ -212,31 +219,51 @@ __device__ __forceinline__ constexpr int slot_of(int k)
 }
 
 // Per-cell stage "prims" for either method.  For HLL the floors are applied to u first.
-template <int METHOD, int DIR, typename FT, bool RN = false>
+template <int METHOD, int DIR, typename FT, bool RN = false, typename OPS = GuardedOps>
 __device__ __forceinline__ V5<FT> stage_prims(double u[5], const FluidConsts<FT> &c)
 {
     if constexpr (METHOD == IB_METHOD_HLLC) {
-        return hllc_prims<FT, RN>((FT)u[0], (FT)u[1], (FT)u[2], (FT)u[3], (FT)u[4]);
+        return hllc_prims<FT, RN, OPS>((FT)u[0], (FT)u[1], (FT)u[2], (FT)u[3], (FT)u[4]);
     } else {
         double irho;
-        double P = hll_pressure<DIR>(u, c.minmass, c.mintemp, (double)c.gm1, irho);
-        return hll_prims<FT, RN>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4], (FT)irho);
+        double P = hll_pressure<DIR, OPS>(u, c.minmass, c.mintemp, (double)c.gm1, irho);
+        return hll_prims<FT, RN, OPS>((FT)u[0], (FT)u[2], (FT)P, (FT)u[3], (FT)u[4], (FT)irho);
     }
 }
 
-template <int METHOD, int SLOPE, typename FT>
+template <int METHOD, int SLOPE, typename FT, typename OPS = GuardedOps>
 __device__ __forceinline__ void stage_faces(const FluidConsts<FT> &c, const V5<FT> &w, const V5<FT> &dl,
                                             const V5<FT> &dr, V5<FT> &L, V5<FT> &R)
 {
-    if constexpr (METHOD == IB_METHOD_HLLC) hllc_faces<SLOPE, FT>(c, w, dl, dr, L, R);
-    else hll_faces<SLOPE, FT>(w, dl, dr, L, R);
+    if constexpr (METHOD == IB_METHOD_HLLC) hllc_faces<SLOPE, FT, OPS>(c, w, dl, dr, L, R);
+    else hll_faces<SLOPE, FT, OPS>(w, dl, dr, L, R);
 }
 
-template <int METHOD, typename FT, bool RN = false>
+template <int METHOD, typename FT, bool RN>
+__device__ __noinline__ V5<FT> stage_flux_ieee(FluidConsts<FT> c, V5<FT> l, V5<FT> r);
+
+template <int METHOD, typename FT, bool RN = false, typename OPS = GuardedOps>
 __device__ __forceinline__ V5<FT> stage_flux(const FluidConsts<FT> &c, const V5<FT> &l, const V5<FT> &r)
 {
-    if constexpr (METHOD == IB_METHOD_HLLC) return hllc_flux<FT, RN>(c, l, r);
-    else return hll_flux<FT, RN>(c, l, r);
+    if constexpr (std::is_same<OPS, GuardedOps>::value) {
+        V5<FT> f = stage_flux<METHOD, FT, RN, FastOps>(c, l, r);
+        if constexpr (kPoison<FastOps, FT>) {
+            if (f.a[0] != f.a[0] || density_suspect(l.a[0]) || density_suspect(r.a[0]))
+                f = stage_flux_ieee<METHOD, FT, RN>(c, l, r);
+        }
+        return f;
+    } else if constexpr (METHOD == IB_METHOD_HLLC) {
+        return hllc_flux<FT, RN, OPS>(c, l, r);
+    } else {
+        return hll_flux<FT, RN, OPS>(c, l, r);
+    }
+}
+
+// (out of line: the guarded kernels seldom come to it)
+template <int METHOD, typename FT, bool RN>
+__device__ __noinline__ V5<FT> stage_flux_ieee(FluidConsts<FT> c, V5<FT> l, V5<FT> r)
+{
+    return stage_flux<METHOD, FT, RN, IeeeOps>(c, l, r);
 }
 
 // lambda times the flux difference of one cell in cylindrical geometry, component by component
@@ -308,6 +335,24 @@ struct SweepArgs {
     RowBc bc;          // x rows: the fill of the rows' ends after the sweep
 };
 
+// Whole periodic pencils in place with the IEEE operations, for the kernels whose CTA owns them and found a
+// density that the short forms did not reach (density_suspect): nothing of the pencils has been stored then.
+// Out of line, in chunks through ieee_pencils_smem() bytes of shared memory (tile_sweep); all threads of the CTA
+// call it.  (Arguments by value: the address of a kernel parameter would move it to local memory for the whole
+// kernel.)
+struct IeeePencils {
+    double *q;
+    int64_t slab;
+    int nx, ny, nz;
+    int64_t first;   // the pencils first .. first + count - 1, those past the grid left out
+    int count, nsweep;
+    double lambda;
+    CylPencil cyl;   // cylindrical sweeps: radial rin, dr or the theta radius rule
+};
+template <int METHOD, int SLOPE, int DIR, int GEO>
+__device__ __noinline__ void ieee_pencils(IeeePencils p, FluidConsts<double> c, double *smem);
+__host__ __device__ constexpr size_t ieee_pencils_smem();
+
 // ------------------------------------------------------------------------------------------
 // TMA-fed pencil pipeline: a persistent CTA walks pencil blocks b = blockIdx.x, +gridDim.x, ...
 // Each block is W adjacent whole pencils (x: one row, W = 1).  Thread 0 keeps two TMA loads
@@ -327,6 +372,9 @@ struct PipeArgs {
     DevScalar lambda;
     unsigned int *err;  // set to 1 when a TMA wait ran out
     uint32_t spin;      // poll limit of the tile waits
+    double *q;
+    int64_t slab;
+    int nx, ny, nz;
 };
 
 __host__ __device__ __forceinline__ size_t pipe_tile_bytes(int n, int W)
@@ -648,7 +696,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                 FT *PY = (stage == 0) ? SB : SA;  // left faces
                 V5<FT> w;
                 if (act) {
-                    w = stage_prims<METHOD, DIR, FT>(u, c);
+                    w = stage_prims<METHOD, DIR, FT, false, FastOps>(u, c);
 #pragma unroll
                     for (int k = 0; k < 5; k++) PX[k * NP + i] = w.a[k];
                     if (stage == 1) {
@@ -665,7 +713,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                         dl.a[k] = w.a[k] - PX[k * NP + il];
                         dr.a[k] = PX[k * NP + ir] - w.a[k];
                     }
-                    stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, keep);
+                    stage_faces<METHOD, SLOPE, FT, FastOps>(c, w, dl, dr, L, keep);
 #pragma unroll
                     for (int k = 0; k < 5; k++) PY[k * NP + i] = L.a[k];
                 }
@@ -674,7 +722,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
                     V5<FT> Lr;
 #pragma unroll
                     for (int k = 0; k < 5; k++) Lr.a[k] = PY[k * NP + ir];
-                    keep = stage_flux<METHOD, FT>(c, keep, Lr);
+                    keep = stage_flux<METHOD, FT, false, FastOps>(c, keep, Lr);
 #pragma unroll
                     for (int k = 0; k < 5; k++) PX[k * NP + i] = keep.a[k];
                 }
@@ -703,7 +751,23 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : ((W
         }
     }
     fence_proxy_async_smem();
-    __syncthreads();
+    if constexpr (kPoison<FastOps, FT>) {
+        bool suspect = false;
+        if (act) {
+#pragma unroll
+            for (int col = 0; col < WC; col++) {
+                const int x = i * WC + col;
+                suspect = suspect || density_suspect(T[(WC == 4) ? x ^ ((x >> 3) & 2) : x]);
+            }
+        }
+        if (__syncthreads_or(suspect)) {  // memory still holds the block's inputs
+            ieee_pencils<METHOD, SLOPE, DIR, GEO>(
+                IeeePencils{a.q, a.slab, a.nx, a.ny, a.nz, b * WC, WC, NS, lambda, cyl}, c, T);
+            return;
+        }
+    } else {
+        __syncthreads();
+    }
     if (leader) {
         pipe_store<DIR>(&tm, T, b, a, WC);
         bulk_commit();
@@ -1000,11 +1064,20 @@ __host__ __device__ __forceinline__ size_t tile_smem_bytes(int Lc, size_t ft)
            (GEO == CYL_RADIAL ? sizeof(double) * TR * W : 0);
 }
 
+// Number of chunks of about `target` cells in which a pencil of n is walked, none shorter than 8 cells
+__host__ __device__ inline int tile_chunks(int n, int target)
+{
+    int nc = (n + target - 1) / target;
+    if (nc < 1) nc = 1;
+    while (nc > 1 && ((n + nc - 1) / nc < 8 || n - (nc - 1) * ((n + nc - 1) / nc) < 8)) nc--;
+    return nc;
+}
+
 // One sweep of W pencils by one CTA.  colbase[c] = offset of pencil c's first cell, colok[c] =
 // whether pencil c exists, stride = distance between consecutive cells of a pencil, n = pencil
 // length, S = slab pitch.  tsm = dynamic shared memory of tile_smem_bytes<W>(Lc).  Must be
 // called by all threads of the CTA.
-template <int METHOD, int SLOPE, typename FT, int DIR, int W, int GEO = CYL_NONE>
+template <int METHOD, int SLOPE, typename FT, int DIR, int W, int GEO = CYL_NONE, typename OPS = GuardedOps>
 __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64_t *colbase, const bool *colok,
                                            int64_t stride, int n, int Lc, double lambda, const FluidConsts<FT> &c,
                                            double *tsm, const double *colr = nullptr, double crin = 0.0,
@@ -1058,7 +1131,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
             double u[5];
 #pragma unroll
             for (int k = 0; k < 5; k++) u[k] = U0t[IDX(k, r, col, TR)];
-            V5<FT> w = stage_prims<METHOD, DIR, FT>(u, c);
+            V5<FT> w = stage_prims<METHOD, DIR, FT, false, OPS>(u, c);
             if (METHOD == IB_METHOD_HLL) {
 #pragma unroll
                 for (int k = 0; k < 5; k++) U0t[IDX(k, r, col, TR)] = u[k];
@@ -1077,7 +1150,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
                 dl.a[k] = w.a[k] - PA[IDX(k, r - 1, col, TR)];
                 dr.a[k] = PA[IDX(k, r + 1, col, TR)] - w.a[k];
             }
-            stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, R);
+            stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, R);
 #pragma unroll
             for (int k = 0; k < 5; k++) { PB[IDX(k, r, col, TR)] = L.a[k]; PC[IDX(k, r, col, TR)] = R.a[k]; }
         }
@@ -1087,7 +1160,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
             V5<FT> Lr, Rl;
 #pragma unroll
             for (int k = 0; k < 5; k++) { Rl.a[k] = PC[IDX(k, r, col, TR)]; Lr.a[k] = PB[IDX(k, r + 1, col, TR)]; }
-            V5<FT> f = stage_flux<METHOD, FT>(c, Rl, Lr);
+            V5<FT> f = stage_flux<METHOD, FT, false, OPS>(c, Rl, Lr);
 #pragma unroll
             for (int k = 0; k < 5; k++) PA[IDX(k, r, col, TR)] = f.a[k];
         }
@@ -1121,7 +1194,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
             double u[5];
 #pragma unroll
             for (int k = 0; k < 5; k++) u[k] = U1t[IDX(k, r1, col, TR1)];
-            V5<FT> w = stage_prims<METHOD, DIR, FT>(u, c);
+            V5<FT> w = stage_prims<METHOD, DIR, FT, false, OPS>(u, c);
             if (METHOD == IB_METHOD_HLL) {
 #pragma unroll
                 for (int k = 0; k < 5; k++) U1t[IDX(k, r1, col, TR1)] = u[k];
@@ -1140,7 +1213,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
                 dl.a[k] = w.a[k] - PA[IDX(k, r - 1, col, TR)];
                 dr.a[k] = PA[IDX(k, r + 1, col, TR)] - w.a[k];
             }
-            stage_faces<METHOD, SLOPE, FT>(c, w, dl, dr, L, R);
+            stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, R);
 #pragma unroll
             for (int k = 0; k < 5; k++) { PB[IDX(k, r, col, TR)] = L.a[k]; PC[IDX(k, r, col, TR)] = R.a[k]; }
         }
@@ -1150,7 +1223,7 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
             V5<FT> Lr, Rl;
 #pragma unroll
             for (int k = 0; k < 5; k++) { Rl.a[k] = PC[IDX(k, r, col, TR)]; Lr.a[k] = PB[IDX(k, r + 1, col, TR)]; }
-            V5<FT> f = stage_flux<METHOD, FT>(c, Rl, Lr);
+            V5<FT> f = stage_flux<METHOD, FT, false, OPS>(c, Rl, Lr);
 #pragma unroll
             for (int k = 0; k < 5; k++) PA[IDX(k, r, col, TR)] = f.a[k];
         }
@@ -1209,6 +1282,27 @@ __device__ __forceinline__ void tile_sweep(double *qbase, int64_t S, const int64
         }
     }
     __syncthreads();
+}
+
+// (chunks of at most 24 cells: one of 8 or more at the end takes up to 30)
+constexpr int kIeeeChunk = 24, kIeeeChunkMax = 30;
+__host__ __device__ constexpr size_t ieee_pencils_smem() { return tile_smem_bytes<1, CYL_RADIAL>(kIeeeChunkMax, sizeof(double)); }
+
+template <int METHOD, int SLOPE, int DIR, int GEO>
+__device__ __noinline__ void ieee_pencils(IeeePencils p, FluidConsts<double> c, double *smem)
+{
+    const PencilMap pm{p.nx, p.ny, p.nz, DIR};
+    const int n = pm.length(), nc = tile_chunks(n, kIeeeChunk);
+    const int64_t npencil = (int64_t)p.nx * p.ny * p.nz / n;
+    const bool ok = true;
+    for (int64_t k = p.first; k < p.first + p.count && k < npencil; k++) {
+        const int64_t base = pm.base(k);
+        const double rpen = (GEO == CYL_THETA_DIV || GEO == CYL_THETA_LAM)
+                                ? theta_radius(p.cyl, (int)(k % p.nx), (int)(k / p.nx)) : 0.0;
+        for (int s = 0; s < p.nsweep; s++)
+            tile_sweep<METHOD, SLOPE, double, DIR, 1, GEO, IeeeOps>(p.q, p.slab, &base, &ok, pm.stride(), n, (n + nc - 1) / nc,
+                                                                   p.lambda, c, smem, &rpen, p.cyl.rin, p.cyl.dr);
+    }
 }
 
 template <int METHOD, int SLOPE, typename FT, int DIR, int W, int GEO = CYL_NONE>

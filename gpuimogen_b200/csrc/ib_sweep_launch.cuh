@@ -20,12 +20,8 @@ int launch_tile_dw(double *q, int64_t slab, const int grid[3], SweepStep lambda,
     // every phase of a chunk must fit in one pass of the CTA's threads: (Lc+8)*W <= 256
     const int lc_max = 256 / W - 8;
     if (target > lc_max) target = lc_max;
-    int nc = std::max(1, (n + target - 1) / target);
-    int Lc = (n + nc - 1) / nc;
-    while (nc > 1 && (Lc < 8 || n - (nc - 1) * Lc < 8)) {
-        nc--;
-        Lc = (n + nc - 1) / nc;
-    }
+    const int nc = tile_chunks(n, target);
+    const int Lc = (n + nc - 1) / nc;
     if (Lc > lc_max) return IB_ERROR_NOIMPLEMENT;  // pencil too short to split into valid chunks
     TileArgs a{q, slab, grid[0], grid[1], grid[2], n, npencil, Lc, lambda, cyl};
     const size_t shm = tile_smem_bytes<W, GEO>(Lc, sizeof(FT));
@@ -116,7 +112,7 @@ int launch_pipe(double *q, int64_t slab, const int grid[3], SweepStep lambda, co
     if (per_sm < 1) return IB_ERROR_NOIMPLEMENT;
     const int64_t want = (int64_t)per_sm * num_sms();
     const unsigned nblk = (unsigned)std::min<int64_t>(want, nblocks);
-    PipeArgs a{n, npw, bh, nh, nblocks, lambda, err, tile_wait_limit()};
+    PipeArgs a{n, npw, bh, nh, nblocks, lambda, err, tile_wait_limit(), q, slab, nx, ny, nz};
     kern<<<nblk, nt, shm, st>>>(tm, a, c);
     return check_launch();
 }
@@ -157,7 +153,7 @@ int launch_pair(double *q, int64_t slab, const int grid[3], SweepStep lambda, co
     if (!err) return IB_ERROR_NOMEM;
     const int nt = (n + 31) / 32 * 32;
     if (PADN && n > PADN) return IB_ERROR_NOIMPLEMENT;
-    const size_t shm = pair_smem_bytes(n, (int)sizeof(FT), WC, NFIX ? NFIX : (PADN ? PADN : n));
+    const size_t shm = std::max(pair_smem_bytes(n, (int)sizeof(FT), WC, NFIX ? NFIX : (PADN ? PADN : n)), ieee_pencils_smem());
     const int ns = (nsweep == 2) ? 2 : 1;
     auto kern = &sweep_pair_kernel<METHOD, SLOPE, FT, DIR, NFIX, 1, WC, GEO, PADN>;
     if constexpr (GEO == CYL_NONE) {
@@ -169,7 +165,7 @@ int launch_pair(double *q, int64_t slab, const int grid[3], SweepStep lambda, co
         if (rc) return rc;
         attr_bytes[ns - 1] = (int)shm;
     }
-    PipeArgs a{n, npw, bh, nh, nblocks, lambda, err, tile_wait_limit()};
+    PipeArgs a{n, npw, bh, nh, nblocks, lambda, err, tile_wait_limit(), q, slab, nx, ny, nz};
     kern<<<(unsigned)nblocks, nt, shm, st>>>(tm, a, c, cyl);
     return check_launch();
 }

@@ -61,25 +61,49 @@ __device__ __forceinline__ double freeze_cell(const double (&X)[5], double invrh
 #ifdef IB_STRICT_ARITH
     return fabs(px) * invrho + sqrt(gamma * P * invrho);
 #else
-    return fabs(px) * invrho + sqrt_fast(gamma * P * invrho);
+    double v = fabs(px) * invrho + sqrt_fast(gamma * P * invrho);
+    if (!(v <= 1.7976931348623157e308)) v = fabs(px) * invrho + sqrt(gamma * P * invrho);
+    return v;
 #endif
 }
+
+#ifndef IB_STRICT_ARITH
+// The same, forming 1 / rho
+__device__ __forceinline__ double freeze_first(const double (&X)[5], double &invrho, double gamma, double gm1)
+{
+    double psq = X[3];
+    double px = X[4];
+    psq = psq * psq + px * px;
+    px = X[2];
+    psq += px * px;
+    invrho = rcp_fast(X[0]);
+    const double arg = gamma * ((X[1] - .5 * psq * invrho) * gm1) * invrho;
+    double v = fabs(px) * invrho + sqrt_fast(arg);
+    if (!(v <= 1.7976931348623157e308)) {
+        invrho = 1.0 / X[0];
+        v = fabs(px) * invrho + sqrt(gamma * ((X[1] - .5 * psq * invrho) * gm1) * invrho);
+    }
+    return v;
+}
+#endif
 
 // The left- and right-going limited fluxes of one component, flux_limit<FLIM>(A1, B1) and
 // flux_limit<FLIM>(A2, B2).  Product build, Ospre and van Leer: selects instead of branches and the
 // reciprocals of ib_fast.cuh.  Ospre's denominator A^2 + A B + B^2 can underflow (momenta near 1e-154):
-// its reciprocal then stays finite and the numerator is zero.  Van Leer's A + B is a normal number
-// wherever 2 A B > 0.
+// its reciprocal then stays finite and the numerator is zero; from 2^1022 on the limiter is 0, as the division
+// gives it where the denominator overflows.  Van Leer's A + B is a normal number wherever 2 A B > 0, and
+// below 2^1022 wherever that product does not overflow by more than a factor 4 in B.
 template <int FLIM>
 __device__ __forceinline__ void flux_limit_pair(double A1, double B1, double A2, double B2, double &o1, double &o2)
 {
 #ifndef IB_STRICT_ARITH
     if constexpr (FLIM == IB_FLUX_OSPRE) {  // 1.5 r (A + B) / (A^2 + r + B^2), 0 where r <= 0
         const double r1 = A1 * B1, r2 = A2 * B2;
-        const double l1 = 1.5 * r1 * (A1 + B1) * rcp_fast_pos(A1 * A1 + r1 + B1 * B1);
-        const double l2 = 1.5 * r2 * (A2 + B2) * rcp_fast_pos(A2 * A2 + r2 + B2 * B2);
-        o1 = (r1 <= 0.0) ? 0.0 : l1;
-        o2 = (r2 <= 0.0) ? 0.0 : l2;
+        const double d1 = A1 * A1 + r1 + B1 * B1, d2 = A2 * A2 + r2 + B2 * B2;
+        const double l1 = 1.5 * r1 * (A1 + B1) * rcp_fast_pos(d1);
+        const double l2 = 1.5 * r2 * (A2 + B2) * rcp_fast_pos(d2);
+        o1 = (r1 <= 0.0 || d1 >= kRcpTop) ? 0.0 : l1;
+        o2 = (r2 <= 0.0 || d2 >= kRcpTop) ? 0.0 : l2;
         return;
     } else if constexpr (FLIM == IB_FLUX_VANLEER) {  // 2AB / (A + B) where 2AB > 0
         const double r1 = 2.0 * A1 * B1, r2 = 2.0 * A2 * B2;
@@ -162,8 +186,7 @@ __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab
 #ifdef IB_STRICT_ARITH
                 const double v = freeze_cell(X, 1.0 / X[0], gamma, gm1);
 #else
-                if (stage == 0) rinv[m] = rcp_fast(X[0]);
-                const double v = freeze_cell(X, rinv[m], gamma, gm1);
+                const double v = (stage == 0) ? freeze_first(X, rinv[m], gamma, gm1) : freeze_cell(X, rinv[m], gamma, gm1);
 #endif
                 cm = (v > cm) ? v : cm;
             }
@@ -276,7 +299,7 @@ __global__ void __launch_bounds__(1024) xj_pencil_kernel(double *q, int64_t slab
 #ifdef IB_STRICT_ARITH
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) / p0;
 #else
-                rinv[m] = rcp_fast(p0);
+                rinv[m] = rcp_full(p0);
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) * rinv[m];
 #endif
                 if ((p1 - w) < p0 * mintemp) p1 = w + p0 * mintemp;
@@ -388,8 +411,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #ifdef IB_STRICT_ARITH
                 const double v = freeze_cell(X, 1.0 / X[0], a.gamma, gm1);
 #else
-                if (stage == 0) rinv = rcp_fast(X[0]);
-                const double v = freeze_cell(X, rinv, a.gamma, gm1);
+                const double v = (stage == 0) ? freeze_first(X, rinv, a.gamma, gm1) : freeze_cell(X, rinv, a.gamma, gm1);
 #endif
                 cm = (v > cm) ? v : cm;
             }
@@ -461,7 +483,7 @@ __global__ void __launch_bounds__(NFIX == 512 ? 512 : 256, NFIX == 512 ? 2 : 4)
 #ifdef IB_STRICT_ARITH
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) / p0;
 #else
-                rinv = rcp_fast(p0);
+                rinv = rcp_full(p0);
                 double w = .5 * (p2 * p2 + p3 * p3 + p4 * p4) * rinv;
 #endif
                 if ((p1 - w) < p0 * a.mintemp) p1 = w + p0 * a.mintemp;
