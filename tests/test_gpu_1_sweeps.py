@@ -13,17 +13,17 @@ from helpers import bits_equal, first_diff, host, product_close, to_fluid
 pytestmark = pytest.mark.gpu
 
 SHAPES = [
-    (37, 11, 9),     # x: row kernel, 1 cell/thread; y,z: tile kernel (odd nx), single chunk
-    (600, 5, 4),     # x: row kernel, 2 cells/thread; y,z: TMA pipeline (pencils below 64 cells)
+    (37, 11, 9),     # odd nx: x in the two-cell row kernel, y and z in the two-cell pencil kernel
+    (600, 5, 4),     # x: two-cell row kernel; y, z: the TMA pipeline (pencils below 16 cells)
     (1100, 3, 4),    # x: chunked TMA pipeline (rows > 1024); y: 3-cell pencils
     (8, 300, 6),     # y: TMA pipeline, pencils of 257-512 cells (two box rows, 2 cells/thread)
     (6, 7, 130),     # z: pencil-pair kernel, 130-cell pencils
-    (5, 4, 3),       # tiny pencils; y,z: tile kernel
+    (5, 4, 3),       # tiny pencils; y, z: two-cell pencil kernel (odd nx)
     (8, 140, 3),     # y: pencil-pair kernels (HLL/HLLC, Xin-Jin) of 129-256 cells
     (4, 3, 200),     # z: the same
-    (160, 3, 2),     # x: HLLC rows of 129-255 cells, planes of a fixed 256-cell stride
-    (96, 100, 90),   # x, y, z: HLLC rows and pencils of 65-127 cells, planes of a 128-cell stride
-    (300, 4, 3),     # x: HLLC rows of 257-511 cells, planes of a 512-cell stride
+    (160, 3, 2),     # x: two-cell rows of 129-160 cells, a CTA of 160 threads
+    (96, 100, 90),   # x: rows that share a CTA; y, z: HLLC pencils of 65-127 cells, planes of a 128-cell stride
+    (300, 4, 3),     # x: two-cell rows of 257-320 cells
 ]
 
 

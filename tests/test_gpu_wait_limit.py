@@ -3,8 +3,9 @@
 Every wait of these kernels for a tile is bounded; one that runs out makes the kernel wait (with
 the full limit) for the copies it has issued, leave, and set the flag ib_device_wait_status reads.
 ib_setTileWaitLimit(0) makes every tile wait give up at once while the copies complete normally,
-so the drain path runs on valid loads.  For each TMA kernel family (pencil-pair kernel with 2- and
-4-pencil boxes, wide-block pipeline, persistent pencil pipeline, chunked pipeline) the test checks
+so the drain path runs on valid loads.  For each TMA kernel family (pencil-pair kernel with 2-pencil boxes;
+4-pencil boxes: test_gpu_19_four_pencil_boxes.py; wide-block pipeline, persistent pencil pipeline, chunked
+pipeline) the test checks
 that the call returns, that the status reports the run-out, that the sweep left the state
 untouched (no tile was computed or stored), and that after the limit is restored and the flag
 cleared the same sweep is correct again.
@@ -19,7 +20,7 @@ pytestmark = pytest.mark.gpu
 
 CASES = [
     ((64, 64, 64), 2, "fp64"),       # y: pencil-pair kernel (2-pencil boxes)
-    ((512, 512, 8), 3, "fp64"),      # z of 2 MB planes: pencil-pair kernel with 4-pencil boxes
+    ((512, 512, 8), 3, "fp64"),      # z of 2 MB planes, 8-cell pencils: persistent pencil pipeline
     ((512, 512, 8), 3, "fp32flux"),  # the same in FP32 flux: wide-block pipeline (8-column boxes)
     ((8, 300, 6), 2, "fp64"),        # y pencils of 257-511 cells: persistent pencil pipeline
     ((8, 600, 4), 2, "fp64"),        # y pencils above 512 cells: chunked pipeline
