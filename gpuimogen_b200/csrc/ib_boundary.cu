@@ -23,8 +23,9 @@ struct PencilIdx {
 };
 
 __global__ void fluid_boundary_kernel(double *q, int64_t S, PencilIdx pi, int64_t npencil, int mode0, int mode1,
-                                      int depth)
+                                      int depth, DevScalar gate)
 {
+    if (gate.off()) return;
     const int64_t p = threadIdx.x + (int64_t)blockIdx.x * blockDim.x;
     if (p >= npencil) return;
     int64_t base, s;
@@ -46,8 +47,9 @@ __global__ void fluid_boundary_kernel(double *q, int64_t S, PencilIdx pi, int64_
 // a chain of dependent loads and stores: one thread per pencil took 5 us on a single row (a 1-D problem
 // pays that twice an iteration).
 __global__ void __launch_bounds__(128) fluid_boundary_split_kernel(double *q, int64_t S, PencilIdx pi, int64_t npencil,
-                                                                   int mode0, int mode1, int depth)
+                                                                   int mode0, int mode1, int depth, DevScalar gate)
 {
+    if (gate.off()) return;
     const int64_t id = threadIdx.x + (int64_t)blockIdx.x * blockDim.x;
     // x rows: a row's ten items next to one another; y and z: neighbouring pencils next to one another
     const int64_t p = (pi.dir == 1) ? id / 10 : id % npencil;
@@ -60,7 +62,7 @@ __global__ void __launch_bounds__(128) fluid_boundary_split_kernel(double *q, in
 }
 
 int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int32_t bc[6], int halo, int dir,
-                          cudaStream_t st)
+                          DevScalar gate, cudaStream_t st)
 {
     const int m0 = bc[2 * (dir - 1)], m1 = bc[2 * (dir - 1) + 1];
     if (m0 == IB_BC_WALL || m1 == IB_BC_WALL || m0 == IB_BC_FREEBALANCE || m1 == IB_BC_FREEBALANCE)
@@ -75,10 +77,10 @@ int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int3
     PencilIdx pi{grid[0], grid[1], grid[2], dir};
     if (row_fill_apart(n, halo)) {
         const int64_t items = 10 * np;
-        fluid_boundary_split_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo);
+        fluid_boundary_split_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
         return check_launch();
     }
-    fluid_boundary_kernel<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo);
+    fluid_boundary_kernel<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
     return check_launch();
 }
 
@@ -139,8 +141,10 @@ int launch_array_boundary(double *phi, const int grid[3], int mode, int dir, int
 }
 
 // cukern_applySpecial_fade (cudaStatics.cu:1240-1266)
-__global__ void statics_kernel(double *phi, const double *statics, int64_t count, int64_t pitch, int64_t numel)
+__global__ void statics_kernel(double *phi, const double *statics, int64_t count, int64_t pitch, int64_t numel,
+                               DevScalar gate)
 {
+    if (gate.off()) return;
     const int64_t i = threadIdx.x + (int64_t)blockIdx.x * blockDim.x;
     if (i >= count) return;
     const double xd = statics[i];
@@ -157,11 +161,11 @@ __global__ void statics_kernel(double *phi, const double *statics, int64_t count
     }
 }
 
-int launch_statics(double *phi, const ib_statics *sl, int64_t numel, cudaStream_t st)
+int launch_statics(double *phi, const ib_statics *sl, int64_t numel, DevScalar gate, cudaStream_t st)
 {
     if (sl == nullptr || sl->data == nullptr || sl->count <= 0) return IB_SUCCESSFUL;
     if (sl->pitch < sl->count) return IB_ERROR_INVALID_ARGS;
-    statics_kernel<<<(unsigned)((sl->count + 127) / 128), 128, 0, st>>>(phi, sl->data, sl->count, sl->pitch, numel);
+    statics_kernel<<<(unsigned)((sl->count + 127) / 128), 128, 0, st>>>(phi, sl->data, sl->count, sl->pitch, numel, gate);
     return check_launch();
 }
 

@@ -310,21 +310,21 @@ static bool has_statics(const ib_fluid *f)
 
 // setFluidBoundary (cudaStatics.cu:112-197): statics of the density array, then per side the
 // statics of every array followed by that side's condition.
-static int fluid_boundary(ib_fluid *f, int dir, cudaStream_t st)
+static int fluid_boundary(ib_fluid *f, int dir, DevScalar gate, cudaStream_t st)
 {
     const int grid[3] = {f->grid.nx, f->grid.ny, f->grid.nz};
     const int64_t S = f->grid.slab_pitch;
     int rc;
-    if (!has_statics(f)) return launch_fluid_boundary(f->q, S, grid, f->bc, f->halo, dir, st);
+    if (!has_statics(f)) return launch_fluid_boundary(f->q, S, grid, f->bc, f->halo, dir, gate, st);
     const int64_t numel = (int64_t)grid[0] * grid[1] * grid[2];
-    if ((rc = launch_statics(f->q, &f->statics[0], numel, st))) return rc;
+    if ((rc = launch_statics(f->q, &f->statics[0], numel, gate, st))) return rc;
     for (int side = 0; side < 2; side++) {
         for (int k = 0; k < 5; k++)
-            if ((rc = launch_statics(f->q + k * S, &f->statics[k], numel, st))) return rc;
+            if ((rc = launch_statics(f->q + k * S, &f->statics[k], numel, gate, st))) return rc;
         int32_t bc1[6];
         memcpy(bc1, f->bc, sizeof(bc1));
         bc1[2 * (dir - 1) + (1 - side)] = IB_BC_CIRCULAR;
-        if ((rc = launch_fluid_boundary(f->q, S, grid, bc1, f->halo, dir, st))) return rc;
+        if ((rc = launch_fluid_boundary(f->q, S, grid, bc1, f->halo, dir, gate, st))) return rc;
     }
     return IB_SUCCESSFUL;
 }
@@ -371,7 +371,7 @@ static int sweep_and_fill(ib_fluid *f, const ib_geometry *geo, int method, int d
     const RowBc bc = (d == 1 && nsweep == 1) ? row_bc(f) : RowBc{0, 0, 0};
     int rc = fluid_update_1d(f, geo, method, d, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st, nsweep, theta_layout, bc, &filled);
     if (rc) return rc;
-    return filled ? IB_SUCCESSFUL : fluid_boundary(f, d, st);
+    return filled ? IB_SUCCESSFUL : fluid_boundary(f, d, dt.part(1.0), st);
 }
 
 // One fluid step (forward or backward) of one fluid, all three sweeps; 1-D grids take the
@@ -384,7 +384,7 @@ static int fluid_step_one(ib_fluid *f, const ib_geometry *geo, int method, const
         bool filled = false;
         int rc = fluid_update_1d(f, geo, method, 1, dt, fp.gamma, fp.rho_min, fp.c_iso, nm, st, 1, 0, row_bc(f), &filled);
         if (rc) return rc;
-        return filled ? IB_SUCCESSFUL : fluid_boundary(f, 1, st);
+        return filled ? IB_SUCCESSFUL : fluid_boundary(f, 1, dt.part(1.0), st);
     }
     int order[3];
     sweep_order(step_number, sweep_dir, order);
@@ -519,7 +519,7 @@ static int complete_timestep(ib_fluid *fluids, const ib_fluid_thermo *thermo, in
         for (int fi = 0; fi < nfluids; fi++)
             for (int d = 1; d <= 3; d++) {
                 if (grid[d - 1] <= 3) continue;
-                int r = fluid_boundary(&fluids[0], d, st);
+                int r = fluid_boundary(&fluids[0], d, dt.part(1.0), st);
                 if (r) return r;
             }
         return IB_SUCCESSFUL;
@@ -746,13 +746,13 @@ int ib_cudaStatics(double *phi, const ib_grid *grid, const int32_t bc[6], int ha
     cudaStream_t st = (cudaStream_t)stream;
     const int g3[3] = {grid->nx, grid->ny, grid->nz};
     for (int side = 0; side < 2; side++) {
-        if ((rc = launch_statics(phi, statics, (int64_t)grid->nx * grid->ny * grid->nz, st))) return rc;
+        if ((rc = launch_statics(phi, statics, (int64_t)grid->nx * grid->ny * grid->nz, DevScalar::of(1.0), st))) return rc;
         const int mode = bc[2 * (direction - 1) + side];
         if (mode == IB_BC_OUTFLOW) {
             int32_t bc1[6] = {IB_BC_CIRCULAR, IB_BC_CIRCULAR, IB_BC_CIRCULAR,
                               IB_BC_CIRCULAR, IB_BC_CIRCULAR, IB_BC_CIRCULAR};
             bc1[2 * (direction - 1) + side] = IB_BC_OUTFLOW;
-            rc = launch_fluid_boundary(phi, grid->slab_pitch, g3, bc1, halo, direction, st);
+            rc = launch_fluid_boundary(phi, grid->slab_pitch, g3, bc1, halo, direction, DevScalar::of(1.0), st);
         } else {
             rc = launch_array_boundary(phi, g3, mode, direction, side, vector_component, halo, st);
         }
@@ -766,7 +766,7 @@ int ib_setFluidBoundary(ib_fluid *fluid, int direction, void *stream)
     int rc;
     if ((rc = validate_fluid(fluid))) return rc;
     if (direction < 1 || direction > 3) return IB_ERROR_INVALID_ARGS;
-    return fluid_boundary(fluid, direction, (cudaStream_t)stream);
+    return fluid_boundary(fluid, direction, DevScalar::of(1.0), (cudaStream_t)stream);
 }
 
 int ib_cudaSource2FluidDrag(ib_fluid *gas, ib_fluid *dust, const ib_thermo *tg, const ib_thermo *td,

@@ -65,11 +65,13 @@ int launch_cfl(const double *q, const double *cs, int64_t slab, const int grid[3
 int launch_soundspeed(const double *q, int64_t slab, int64_t n, double gamma, double *cs, cudaStream_t st);
 int launch_freeze_ptot(double *q, int64_t slab, const int grid[3], double gamma, double cs_min, double *ptot,
                        double *freeze, cudaStream_t st);
+// gate: the timestep of the step that the fill belongs to; a device timestep of 0 (after the end time) leaves
+// the arrays as they are, as it does in the sweeps
 int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int32_t bc[6], int halo, int dir,
-                          cudaStream_t st);
+                          DevScalar gate, cudaStream_t st);
 int launch_array_boundary(double *phi, const int grid[3], int mode, int dir, int side, int vec_component, int halo,
                           cudaStream_t st);
-int launch_statics(double *phi, const ib_statics *st_list, int64_t numel, cudaStream_t st);
+int launch_statics(double *phi, const ib_statics *st_list, int64_t numel, DevScalar gate, cudaStream_t st);
 int launch_drag(double *gas, double *dust, int64_t slab, const int grid[3], const double h[3], const double dp[11],
                 DevScalar dt, int method, cudaStream_t st);
 
