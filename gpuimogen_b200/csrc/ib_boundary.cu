@@ -17,7 +17,12 @@ struct PencilIdx {
     __device__ __forceinline__ void get(int64_t p, int64_t &base, int64_t &stride, int &n) const
     {
         if (dir == 1) { base = p * nx; stride = 1; n = nx; }
-        else if (dir == 2) { base = (p % nx) + (int64_t)nx * ny * (p / nx); stride = nx; n = ny; }
+        else if (dir == 2) {
+            const int64_t x = column_of(p, nx);
+            base = x + (p - x) * ny;  // the line p / nx starts nx ny cells after the one before
+            stride = nx;
+            n = ny;
+        }
         else { base = p; stride = (int64_t)nx * ny; n = nz; }
     }
 };
@@ -42,19 +47,21 @@ __global__ void fluid_boundary_kernel(double *q, int64_t S, PencilIdx pi, int64_
     }
 }
 
-// The same fill with one thread per pencil, side and slab (one per side for outflow, whose slabs depend on
-// one another), for pencils long enough that neither side reads what the other writes.  A pencil's fill is
-// a chain of dependent loads and stores: one thread per pencil took 5 us on a single row (a 1-D problem
-// pays that twice an iteration).
+// The same fill with PER threads per pencil, for pencils long enough that neither side reads what the other
+// writes: one for each side and slab (10), or one for each side where both ends are outflow (2), whose slabs depend
+// on one another.  A pencil's fill is a chain of dependent loads and stores: one thread per pencil took 5 us on a
+// single row (a 1-D problem pays that twice an iteration).
+template <int PER>
 __global__ void __launch_bounds__(128) fluid_boundary_split_kernel(double *q, int64_t S, PencilIdx pi, int64_t npencil,
                                                                    int mode0, int mode1, int depth, DevScalar gate)
 {
     if (gate.off()) return;
     const int64_t id = threadIdx.x + (int64_t)blockIdx.x * blockDim.x;
-    // x rows: a row's ten items next to one another; y and z: neighbouring pencils next to one another
-    const int64_t p = (pi.dir == 1) ? id / 10 : id % npencil;
-    const int item = (int)((pi.dir == 1) ? id % 10 : id / npencil);
-    if (p >= npencil || item >= 10) return;
+    // x rows: a row's items next to one another; y and z: neighbouring pencils next to one another, the items in
+    // the grid's second dimension
+    const int64_t p = (pi.dir == 1) ? id / PER : id;
+    const int item = ((pi.dir == 1) ? (int)(id % PER) : (int)blockIdx.y) * (10 / PER);
+    if (p >= npencil) return;
     int64_t base, s;
     int n;
     pi.get(p, base, s, n);
@@ -75,9 +82,19 @@ int launch_fluid_boundary(double *q, int64_t slab, const int grid[3], const int3
     const int64_t N = (int64_t)grid[0] * grid[1] * grid[2];
     const int64_t np = N / n;
     PencilIdx pi{grid[0], grid[1], grid[2], dir};
-    if (row_fill_apart(n, halo)) {
-        const int64_t items = 10 * np;
-        fluid_boundary_split_kernel<<<(unsigned)((items + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
+    // Split where the chain of a pencil bounds the fill; with very many pencils along y or z, or one outflow end there,
+    // the threads' number does.  us, one thread per pencil and split, const / outflow on both ends: y of 64^3 4.3 / 4.1
+    // and 2.1 / 3.5, of 256^3 6.0 / 5.9 and 5.9 / 5.2, of 512 x 512 x 256 (131072 pencils) 8.8 / 9.3 and 10.2 / 8.6, its z
+    // 21.2 / 21.9 and 21.6 / 21.5; x of 256^3 21.4 / 24.0 and 19.5 / 22.0; outflow on one end of y, 64^3, 3.0 and 3.5.
+    const auto none = [](int m) { return m == IB_BC_CIRCULAR || m == IB_BC_STATIONARY; };
+    const auto by_side = [&](int m) { return m == IB_BC_OUTFLOW || none(m); };
+    const int per = (by_side(m0) && by_side(m1)) ? 2 : 10;
+    const bool one_end = per == 2 && (none(m0) || none(m1));
+    if (row_fill_apart(n, halo) && (dir == 1 || (np < 131072 && !one_end))) {
+        const int64_t threads = dir == 1 ? per * np : np;
+        const dim3 blocks((unsigned)((threads + 127) / 128), dir == 1 ? 1 : per);
+        if (per == 2) fluid_boundary_split_kernel<2><<<blocks, 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
+        else fluid_boundary_split_kernel<10><<<blocks, 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
         return check_launch();
     }
     fluid_boundary_kernel<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(q, slab, pi, np, m0, m1, halo, gate);
