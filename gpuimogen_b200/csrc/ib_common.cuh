@@ -301,7 +301,7 @@ __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 
 // Limited faces of one cell from its primitive value and its two backward differences.
 // L/R faces: rho, P = gm1*(e -/+ s), v.  (cudaFluidStep.cu:1287-1310)
-template <int SLOPE, typename FT, typename OPS = FastOps>
+template <int SLOPE, typename FT, bool RN = false, typename OPS = FastOps>
 __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT> &w,
                                            const V5<FT> &dl, const V5<FT> &dr, V5<FT> &L, V5<FT> &R)
 {
@@ -309,8 +309,8 @@ __device__ __forceinline__ void hllc_faces(const FluidConsts<FT> &c, const V5<FT
     for (int k = 0; k < 5; k++) {
         FT s = slope_limit<SLOPE, FT, OPS>(dl.a[k], dr.a[k]);
         if (k == 1) {
-            L.a[1] = c.gm1 * (w.a[1] - s);
-            R.a[1] = c.gm1 * (w.a[1] + s);
+            L.a[1] = product<RN>(c.gm1, w.a[1] - s);
+            R.a[1] = product<RN>(c.gm1, w.a[1] + s);
         } else {
             L.a[k] = w.a[k] - s;
             R.a[k] = w.a[k] + s;

@@ -121,8 +121,8 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
                 const double ta = second ? SS[k * TT + p.own] : ua[k], tb = second ? SS[(5 + k) * TT + p.own] : ub[k];
                 double na, nb;
                 if constexpr (GEO == CYL_NONE) {
-                    na = ta - lambda * (fc - fl);
-                    nb = tb - lambda * (fr - fc);
+                    na = sub_product(ta, lambda, fc - fl);
+                    nb = sub_product(tb, lambda, fr - fc);
                 } else {
                     na = ta - cyl_dflux<METHOD, GEO>(k, fc, fl, lam, g.ra, g.dr, g.rpen, pa, pa,
                                                      second ? rho_a : (k == 0 ? 0.0 : va[0]), c);

@@ -9,8 +9,10 @@
 // its end without leaving the kernel; the problem's cells stay in L2 between sweeps (one
 // problem is at most a few hundred KB), so the launch reads and writes HBM about once per cell.
 // The per-cell arithmetic is the library's sweep arithmetic (stage_prims / stage_faces / stage_flux in
-// ens_sweep, the two-cell stages of ib_duo.cuh in ens_sweep_two), CFL and boundary code, so every problem's
-// result equals running it alone through the library's 1-D entry points.
+// ens_stages, the two-cell stages of ib_duo.cuh in ens_sweep_two), CFL and boundary code.  A problem's bits
+// depend neither on the launch shape nor on how many problems share the launch.  In the strict build they are those
+// of the problem run alone through the library's 1-D entry points; in the product build, whose other sweeps do not
+// round every product, they agree with them to 1e-12 (relative L1).
 #include "ib_bc.cuh"
 #include "ib_cfl.cuh"
 #include "ib_internal.cuh"
@@ -100,6 +102,9 @@ __device__ __forceinline__ void ens_store_ends(double *qb, int64_t S, int n, int
     __syncthreads();
 }
 
+// Products that leave a cell are rounded (RN), here and in the form with two rows a thread: otherwise the compiler
+// contracts them into the sums of the thread that formed them, and a cell's result would depend on the form.
+//
 // Both stages of one chunk, row i of its tr rows a thread, which keeps that cell's state u in registers: on
 // return u is the output of rows 4 .. tr - 5.  Two shared-memory planes of FT swap roles between the stages.
 template <int METHOD, int SLOPE, typename FT, typename OPS>
@@ -110,7 +115,7 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
     V5<FT> keep;
     // ---- stage A: prims and fluxes in SA, left faces in SB ----
     if (i < tr) {
-        V5<FT> w = stage_prims<METHOD, 1, FT, false, OPS>(u, c);  // HLL floors u
+        V5<FT> w = stage_prims<METHOD, 1, FT, true, OPS>(u, c);  // HLL floors u
 #pragma unroll
         for (int k = 0; k < 5; k++) SA[k * TR + i] = w.a[k];
     }
@@ -123,7 +128,7 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
             dl.a[k] = w.a[k] - SA[k * TR + i - 1];
             dr.a[k] = SA[k * TR + i + 1] - w.a[k];
         }
-        stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, keep);
+        stage_faces<METHOD, SLOPE, FT, OPS, true>(c, w, dl, dr, L, keep);
 #pragma unroll
         for (int k = 0; k < 5; k++) SB[k * TR + i] = L.a[k];
     }
@@ -132,19 +137,19 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
         V5<FT> Lr;
 #pragma unroll
         for (int k = 0; k < 5; k++) Lr.a[k] = SB[k * TR + i + 1];
-        keep = stage_flux<METHOD, FT, false, OPS>(c, keep, Lr);
+        keep = stage_flux<METHOD, FT, true, OPS>(c, keep, Lr);
 #pragma unroll
         for (int k = 0; k < 5; k++) SA[k * TR + i] = keep.a[k];
     }
     __syncthreads();
     if (i >= 2 && i <= tr - 3) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) u1[k] = u[k] - lambda * ((double)keep.a[k] - (double)SA[k * TR + i - 1]);
+        for (int k = 0; k < 5; k++) u1[k] = sub_product(u[k], lambda, (double)keep.a[k] - (double)SA[k * TR + i - 1]);
     }
     // ---- stage B: prims and fluxes in SB, left faces in SA (no barrier: stage A's last
     // phase read SA only) ----
     if (i >= 2 && i <= tr - 3) {
-        V5<FT> w = stage_prims<METHOD, 1, FT, false, OPS>(u1, c);  // HLL floors u1
+        V5<FT> w = stage_prims<METHOD, 1, FT, true, OPS>(u1, c);  // HLL floors u1
 #pragma unroll
         for (int k = 0; k < 5; k++) {
             SB[k * TR + i] = w.a[k];
@@ -160,7 +165,7 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
             dl.a[k] = w.a[k] - SB[k * TR + i - 1];
             dr.a[k] = SB[k * TR + i + 1] - w.a[k];
         }
-        stage_faces<METHOD, SLOPE, FT, OPS>(c, w, dl, dr, L, keep);
+        stage_faces<METHOD, SLOPE, FT, OPS, true>(c, w, dl, dr, L, keep);
 #pragma unroll
         for (int k = 0; k < 5; k++) SA[k * TR + i] = L.a[k];
     }
@@ -169,14 +174,14 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
         V5<FT> Lr;
 #pragma unroll
         for (int k = 0; k < 5; k++) Lr.a[k] = SA[k * TR + i + 1];
-        keep = stage_flux<METHOD, FT, false, OPS>(c, keep, Lr);
+        keep = stage_flux<METHOD, FT, true, OPS>(c, keep, Lr);
 #pragma unroll
         for (int k = 0; k < 5; k++) SB[k * TR + i] = keep.a[k];
     }
     __syncthreads();
     if (i >= 4 && i <= tr - 5) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) u[k] = .5 * (u[k] - lambda * ((double)keep.a[k] - (double)SB[k * TR + i - 1]));
+        for (int k = 0; k < 5; k++) u[k] = .5 * sub_product(u[k], lambda, (double)keep.a[k] - (double)SB[k * TR + i - 1]);
     }
 }
 
@@ -416,19 +421,24 @@ static int launch_ens_nt(const EnsArgs &a0, const FluidConsts<FT> &c, int ctas_p
     return check_launch();
 }
 
-// Two rows a thread where the problems fill the chip twice at the default launch shape (five CTAs per SM for
-// FP64, six for the FP32 flux): half the shared-memory traffic, 1500 / 4096 problems of 256-4096 cells 2.96 /
-// 6.30 -> 2.53 / 5.23 ms (FP64, 10 / 8 iterations), 5.05 -> 4.01 (FP32 flux, 4096).  With fewer, a problem's own
-// time counts, and a CTA of half the threads takes longer for it: 170 problems 1.19 -> 1.33, 800 1.71 -> 2.28.
-// The rule is by the number of problems alone, so that results do not depend on the launch shape.
-template <typename FT>
-static bool ens_two_rows(int np) { return np >= 2 * duo_min_blocks<FT>(128) * num_sms(); }
+// Two rows a thread from nine problems per SM on: half the shared-memory traffic, but a CTA of half the threads takes
+// longer for a problem, and with fewer problems a problem's own time counts.  Time against one row a thread:
+//   problems                        600    900    1100   1300   1480   2000   3000
+//   FP64, 256-4096 cells            1.31   1.34   1.14   0.97   0.94   0.95   0.95
+//   FP64, 32-512 cells              1.44   1.20   1.07   0.99   0.97   0.97   0.98
+//   FP64, 900-1100 cells            0.98   1.12   1.08   0.98   0.95   0.95   0.99
+//   FP32 flux, 256-4096 cells       1.13   1.38   1.17   1.00   0.90   0.80   0.79
+//   FP32 flux, 32-512 cells         1.23   1.18   1.04   0.96   0.83   0.82   0.80
+//   FP32 flux, 900-1100 cells       0.92   0.85   0.93   0.83   0.84   0.84   0.80
+// (FP64 256-4096 cells, 10 iterations: 1480 problems 3.00 -> 2.81 ms, 3000 5.89 -> 5.59; FP32 flux 2.35 -> 2.11, 4.62 ->
+// 3.62).  By the number of problems and SMs alone: both forms give the same bits.
+static bool ens_two_rows(int np) { return np >= 9 * num_sms(); }
 
 template <int METHOD, int SLOPE, typename FT, int NT>
 static int launch_ens_form(const EnsArgs &a, const FluidConsts<FT> &c, int ctas_per_sm, cudaStream_t st)
 {
-    return ens_two_rows<FT>(a.np) ? launch_ens_nt<METHOD, SLOPE, FT, NT, true>(a, c, ctas_per_sm, st)
-                                  : launch_ens_nt<METHOD, SLOPE, FT, NT, false>(a, c, ctas_per_sm, st);
+    return ens_two_rows(a.np) ? launch_ens_nt<METHOD, SLOPE, FT, NT, true>(a, c, ctas_per_sm, st)
+                              : launch_ens_nt<METHOD, SLOPE, FT, NT, false>(a, c, ctas_per_sm, st);
 }
 
 template <int METHOD, int SLOPE, typename FT>

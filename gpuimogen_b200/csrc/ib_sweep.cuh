@@ -231,11 +231,11 @@ __device__ __forceinline__ V5<FT> stage_prims(double u[5], const FluidConsts<FT>
     }
 }
 
-template <int METHOD, int SLOPE, typename FT, typename OPS = GuardedOps>
+template <int METHOD, int SLOPE, typename FT, typename OPS = GuardedOps, bool RN = false>
 __device__ __forceinline__ void stage_faces(const FluidConsts<FT> &c, const V5<FT> &w, const V5<FT> &dl,
                                             const V5<FT> &dr, V5<FT> &L, V5<FT> &R)
 {
-    if constexpr (METHOD == IB_METHOD_HLLC) hllc_faces<SLOPE, FT, OPS>(c, w, dl, dr, L, R);
+    if constexpr (METHOD == IB_METHOD_HLLC) hllc_faces<SLOPE, FT, RN, OPS>(c, w, dl, dr, L, R);
     else hll_faces<SLOPE, FT, OPS>(w, dl, dr, L, R);
 }
 
