@@ -48,7 +48,8 @@ SOURCES = [
     "ib_time.cu",
 ]
 HEADERS = ["ib_common.cuh", "ib_internal.cuh", "ib_sweep.cuh", "ib_sweep_launch.cuh", "ib_tma.cuh", "ib_bc.cuh",
-           "ib_cfl.cuh", "ib_drag.cuh", "ib_tcgen05.cuh", "ib_cyl.cuh", "ib_fast.cuh", "ib_duo.cuh", "ib_duo_launch.cuh"]
+           "ib_cfl.cuh", "ib_drag.cuh", "ib_tcgen05.cuh", "ib_cyl.cuh", "ib_fast.cuh", "ib_duo.cuh", "ib_duo_launch.cuh",
+           "ib_optin.h"]
 
 BASE_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",

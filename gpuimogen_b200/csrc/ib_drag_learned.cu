@@ -387,15 +387,9 @@ static int launch_mlp_tc(const LearnedArgs &a, cudaStream_t st)
 {
     auto kern = mlp_tc_kernel<MODE>;
     const size_t shm = sizeof(LearnedSmem);
-    static bool attr = false;
+    static SmemOptIn record;
     int rc;
-    if (!attr) {
-        if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm))))
-            return rc;
-        if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100))))
-            return rc;
-        attr = true;
-    }
+    if ((rc = opt_in(record, kern, shm, 100))) return rc;
     // A CTA walks its tiles to the end, so the grid is what fits at once: counted here from the
     // registers and shared memory (the occupancy query reports 1 for this kernel), at most 8
     // (8 x 64 tensor-memory columns are all 512 of an SM).

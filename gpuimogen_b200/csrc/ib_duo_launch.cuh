@@ -6,23 +6,13 @@
 
 namespace ib {
 
-// Opts a kernel in to the dynamic shared memory it needs, when that grows.
-template <typename K>
-int duo_opt_in(K kern, int &have, size_t bytes)
-{
-    if ((int)bytes <= have) return IB_SUCCESSFUL;
-    const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (rc == IB_SUCCESSFUL) have = (int)bytes;
-    return rc;
-}
-
 template <int METHOD, int SLOPE, typename FT, int TT, int NS, bool ODD, bool FILL, int GEO>
 int launch_duo_row_t(const SweepArgs &a, const FluidConsts<FT> &c, cudaStream_t st)
 {
     auto kern = duo_row_kernel<METHOD, SLOPE, FT, TT, NS, ODD, FILL, GEO>;
     constexpr size_t shm = duo_smem_bytes<FT, TT>();
-    static int have = 48 * 1024;
-    const int rc = duo_opt_in(kern, have, shm);
+    static SmemOptIn record;
+    const int rc = opt_in(record, kern, shm);
     if (rc) return rc;
     const int T = (a.nx + 1) / 2, rp = TT / T;
     const int64_t rows = (int64_t)a.ny * a.nz;
@@ -75,8 +65,8 @@ int launch_duo_pencil_t(const SweepArgs &a, const FluidConsts<FT> &c, int n, cud
 {
     auto kern = duo_pencil_kernel<METHOD, SLOPE, FT, DIR, TT, COLS, ODD, GEO>;
     constexpr size_t shm = duo_smem_bytes<FT, TT>();
-    static int have = 48 * 1024;
-    const int rc = duo_opt_in(kern, have, shm);
+    static SmemOptIn record;
+    const int rc = opt_in(record, kern, shm);
     if (rc) return rc;
     const int64_t np = (int64_t)a.nx * a.ny * a.nz / n;
     kern<<<(unsigned)((np + COLS - 1) / COLS), ((n + 1) / 2 * COLS + 31) / 32 * 32, shm, st>>>(a, c, np, cyl);

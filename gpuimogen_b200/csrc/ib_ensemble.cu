@@ -401,13 +401,9 @@ static int launch_ens_nt(const EnsArgs &a0, const FluidConsts<FT> &c, int ctas_p
     auto kern = ensemble_kernel<METHOD, SLOPE, FT, NT, TWO>;
     constexpr int TT = TWO ? NT / 2 : NT;
     const size_t shm = ens_smem<FT, NT, TWO>(a.lcap);
-    static int attr_bytes = 0;
+    static SmemOptIn record;
     int rc;
-    if ((int)shm > attr_bytes) {
-        if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm))))
-            return rc;
-        attr_bytes = (int)shm;
-    }
+    if ((rc = opt_in(record, kern, shm))) return rc;
     int per_sm = 0;
     if ((rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TT, shm)))) return rc;
     if (per_sm < 1 || a.lcap > NT) return IB_ERROR_INVALID_ARGS;

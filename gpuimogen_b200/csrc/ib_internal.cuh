@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include "ib_common.cuh"
+#include "ib_optin.h"
 #include "ib_tma.cuh"
 #include "ib_cyl.cuh"
 
@@ -13,6 +14,21 @@ namespace ib {
 
 // Records the last CUDA error and maps it to the library's status codes.
 int check_cuda(cudaError_t e);
+
+// Opts a kernel in to at least `bytes` of dynamic shared memory on the current device (and to a shared-memory
+// carveout, if one is given).  One record per kernel.
+template <typename K>
+int opt_in(SmemOptIn &record, K kern, size_t bytes, int carveout = -1)
+{
+    int device = 0;
+    const int rc = check_cuda(cudaGetDevice(&device));
+    if (rc) return rc;
+    return record.raise(device, bytes, [&](size_t b) {
+        const int r = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b));
+        if (r || carveout < 0) return r;
+        return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, carveout));
+    });
+}
 int check_launch();
 int num_sms();
 // Poll limit of the TMA-fed kernels' tile waits (IB_TMA_SPIN_LIMIT unless ib_setTileWaitLimit set one).

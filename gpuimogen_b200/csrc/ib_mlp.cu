@@ -409,12 +409,8 @@ __global__ void drag_decay_kernel(const double *__restrict__ f, int64_t n, DragP
 
 static int mlp_smem_attr(const void *fn)
 {
-    static int done_fwd = 0, done_grad = 0;
-    int &done = (fn == (const void *)mlp_forward_kernel) ? done_fwd : done_grad;
-    if (done) return IB_SUCCESSFUL;
-    int rc = check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpSmem)));
-    if (rc == IB_SUCCESSFUL) done = 1;
-    return rc;
+    static SmemOptIn forward, grad;
+    return opt_in(fn == (const void *)mlp_forward_kernel ? forward : grad, fn, sizeof(MlpSmem));
 }
 
 }  // namespace ib

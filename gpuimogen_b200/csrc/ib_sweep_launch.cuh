@@ -25,15 +25,11 @@ int launch_tile_dw(double *q, int64_t slab, const int grid[3], SweepStep lambda,
     if (Lc > lc_max) return IB_ERROR_NOIMPLEMENT;  // pencil too short to split into valid chunks
     TileArgs a{q, slab, grid[0], grid[1], grid[2], n, npencil, Lc, lambda, cyl};
     const size_t shm = tile_smem_bytes<W, GEO>(Lc, sizeof(FT));
-    static int attr_bytes = 0;
-    // opt in whenever the size grows: without it the limit is 48 KB including the static
-    // shared memory and the 1 KB the driver reserves per block (48640 B at 256-cell pencils fails)
-    if ((int)shm > attr_bytes) {
-        int rc = check_cuda(cudaFuncSetAttribute(sweep_tile_kernel<METHOD, SLOPE, FT, DIR, W, GEO>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes = (int)shm;
-    }
+    // opt in whatever the size: without it the limit is 48 KB including the static shared memory and the 1 KB
+    // the driver reserves per block (48640 B at 256-cell pencils fails)
+    static SmemOptIn record;
+    const int rc = opt_in(record, sweep_tile_kernel<METHOD, SLOPE, FT, DIR, W, GEO>, shm);
+    if (rc) return rc;
     const unsigned nblk = (unsigned)((npencil + W - 1) / W);
     sweep_tile_kernel<METHOD, SLOPE, FT, DIR, W, GEO><<<nblk, 256, shm, st>>>(a, c);
     return check_launch();
@@ -100,12 +96,8 @@ int launch_pipe(double *q, int64_t slab, const int grid[3], SweepStep lambda, co
             return ns == 2 ? &sweep_pipe_wide_kernel<METHOD, SLOPE, FT, DIR, W, G, CPT, NFIX, 2>
                            : &sweep_pipe_wide_kernel<METHOD, SLOPE, FT, DIR, W, G, CPT, NFIX, 1>;
     }();
-    static int attr_bytes[2] = {0, 0};
-    if ((int)shm > attr_bytes[ns - 1]) {
-        rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes[ns - 1] = (int)shm;
-    }
+    static SmemOptIn records[2];
+    if ((rc = opt_in(records[ns - 1], kern, shm))) return rc;
     int per_sm = 0;
     rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, shm));
     if (rc) return rc;
@@ -159,12 +151,8 @@ int launch_pair(double *q, int64_t slab, const int grid[3], SweepStep lambda, co
     if constexpr (GEO == CYL_NONE) {
         if (ns == 2) kern = &sweep_pair_kernel<METHOD, SLOPE, FT, DIR, NFIX, 2, WC, CYL_NONE, PADN>;
     }
-    static int attr_bytes[2] = {0, 0};
-    if ((int)shm > attr_bytes[ns - 1]) {
-        rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes[ns - 1] = (int)shm;
-    }
+    static SmemOptIn records[2];
+    if ((rc = opt_in(records[ns - 1], kern, shm))) return rc;
     PipeArgs a{n, npw, bh, nh, nblocks, lambda, err, tile_wait_limit(), q, slab, nx, ny, nz};
     kern<<<(unsigned)nblocks, nt, shm, st>>>(tm, a, c, cyl);
     return check_launch();
@@ -232,12 +220,8 @@ int launch_chunk(double *q, int64_t slab, const int grid[3], SweepStep lambda, c
     const int nt = W * R / 2;
     const size_t shm = chunk_smem_bytes(W, R, (int)sizeof(FT));
     auto kern = sweep_chunk_kernel<METHOD, SLOPE, FT, DIR, W, R>;
-    static int attr_bytes = 0;
-    if ((int)shm > attr_bytes) {
-        rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes = (int)shm;
-    }
+    static SmemOptIn record;
+    if ((rc = opt_in(record, kern, shm))) return rc;
     int per_sm = 0;
     rc = check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, shm));
     if (rc) return rc;

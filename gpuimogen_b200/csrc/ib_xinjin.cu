@@ -556,13 +556,8 @@ static int launch_xj_pair(double *q, int64_t slab, const int grid[3], SweepStep 
     if (!err) return IB_ERROR_NOMEM;
     const int nt = (n + 31) / 32 * 32;
     const size_t shm = xj_box_bytes(n, WC) + (size_t)80 * (NFIX ? NFIX : (PADN ? PADN : n));
-    static int attr_bytes = 0;
-    if ((int)shm > attr_bytes) {
-        rc = check_cuda(cudaFuncSetAttribute(xj_pair_kernel<FLIM, DIR, NFIX, WC, GEO, PADN>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        if (rc) return rc;
-        attr_bytes = (int)shm;
-    }
+    static SmemOptIn record;
+    if ((rc = opt_in(record, xj_pair_kernel<FLIM, DIR, NFIX, WC, GEO, PADN>, shm))) return rc;
     const bool fill = DIR == 1 && lambda.filled && lambda.bc.depth > 0;
     if (fill) *lambda.filled = true;
     XjPairArgs a{n, npw, lambda, gamma, rho_min, mintemp, err, tile_wait_limit(), cyl, fill ? lambda.bc : RowBc{0, 0, 0}};
@@ -691,13 +686,9 @@ int launch_xj_sweep(int flim, int dir, double *q, int64_t slab, const int grid[3
     if (fill) *lambda.filled = true;
 #define IB_XJ_G(F, WW, CC, RR, GG)                                                                            \
     do {                                                                                                      \
-        static bool attr_set = false;                                                                         \
-        if (!attr_set) {                                                                                      \
-            int rc_ = check_cuda(cudaFuncSetAttribute(xj_pencil_kernel<F, WW, CC, RR, GG>,                    \
-                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm_cap)); \
-            if (rc_) return rc_;                                                                              \
-            attr_set = true;                                                                                  \
-        }                                                                                                     \
+        static SmemOptIn record;                                                                              \
+        const int rc_ = opt_in(record, xj_pencil_kernel<F, WW, CC, RR, GG>, shm_cap);                         \
+        if (rc_) return rc_;                                                                                  \
         xj_pencil_kernel<F, WW, CC, RR, GG><<<nblk, nt, shm, st>>>(q, slab, grid[0], grid[1], grid[2], dir,   \
                                                                    lambda, gamma, rho_min, mintemp, cp, bc);  \
     } while (0)
