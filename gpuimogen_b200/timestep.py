@@ -54,18 +54,25 @@ def _launch_cfl(fluids, geometry, method):
     return taus
 
 
-def _wait_tau(taus):
-    torch.cuda.current_stream().synchronize()
+def _least(taus):
     tau = 1e38
-    for t in taus.tolist():
+    for t in taus:
         if not math.isfinite(t):
             raise ib.ImogenError("cflTimestep: non-finite timestep", -101)
         tau = min(tau, t)
     return tau
 
 
+def _wait_tau(taus):
+    torch.cuda.current_stream().synchronize()
+    return _least(taus.tolist())
+
+
 def cfl_tau(fluids, geometry, method):
-    """Minimum over fluids of the CFL time (TimeManager.update loop)."""
+    """Minimum over fluids of the CFL time (TimeManager.update loop).  One fluid: the call that waits on its own
+    (23.4 us for small grids; 26.4 through a page-locked tensor, which pays for itself where it saves a wait)."""
+    if len(fluids) == 1:
+        return _least([ib.cflTimestepFused(fluids[0], fluids[0].gamma, geometry, method)])
     return _wait_tau(_launch_cfl(fluids, geometry, method))
 
 
@@ -75,11 +82,14 @@ def run_iteration(fluids, geometry, tm, method, num=None, source=None, drag=None
     otherwise the complete timestep runs through completeTimestep (performCompleteTimestep), with
     the two-fluid drag between the steps when drag = (thermo_gas, thermo_dust, method).  The host prepares
     the step's arguments while the reductions run and waits once for all fluids."""
-    taus = _launch_cfl(fluids, geometry, method)
-    try:
-        args = ib._complete_args(fluids, geometry, num, drag) if source is None else None
-    finally:
-        tau = _wait_tau(taus)
+    if source is None:
+        taus = _launch_cfl(fluids, geometry, method)
+        try:
+            args = ib._complete_args(fluids, geometry, num, drag)
+        finally:
+            tau = _wait_tau(taus)
+    else:
+        tau = cfl_tau(fluids, geometry, method)
     dt = tm.update(tau)
     if source is not None:
         source(fluids, 0.5 * dt)
