@@ -73,14 +73,18 @@ int launch_duo_pencil_t(const SweepArgs &a, const FluidConsts<FT> &c, int n, cud
     return check_launch();
 }
 
-// y and z pencils of up to 512 cells, any nx and alignment: as many neighbouring pencils as 256 threads hold,
-// at most 8
+// y and z pencils, any nx and alignment: as many neighbouring pencils as 256 threads hold, at most 8.  FP64 up to
+// 512 cells, the FP32 flux up to 256: above, one pencil's CTA reads 8 bytes of every 32-byte sector, which the FP32
+// flux waits for, and four pencils a CTA in the tile kernel are the faster form (us, tile / here: 63 x 257 x 259 y
+// 214 / 251, 64 x 403 x 162 y 210 / 295, 601 x 18 x 384 z 209 / 254, 63 x 130 x 512 z 209 / 243; FP64 there 317 / 314,
+// 277 / 337, 319 / 315, 316 / 285).
 template <int METHOD, int SLOPE, typename FT, int DIR, int GEO = CYL_NONE>
 int launch_duo_pencil(double *q, int64_t slab, const int grid[3], SweepStep lambda, const FluidConsts<FT> &c,
                       cudaStream_t st, int nsweep, CylPencil cyl = CylPencil{0.0, 0.0, 0, 0})
 {
     const int n = grid[DIR - 1];
-    if (n > 512 || (int64_t)grid[0] * grid[1] * grid[2] / n >= (int64_t)1 << 31) return IB_ERROR_NOIMPLEMENT;
+    if (n > (sizeof(FT) == 4 ? 256 : 512) || (int64_t)grid[0] * grid[1] * grid[2] / n >= (int64_t)1 << 31)
+        return IB_ERROR_NOIMPLEMENT;
     SweepArgs a{q, slab, grid[0], grid[1], grid[2], lambda, 0.0, 0.0, RowBc{0, 0, 0}};
     using std::integral_constant;
     auto go = [&](auto odd) {

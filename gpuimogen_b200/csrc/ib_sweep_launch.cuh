@@ -389,7 +389,7 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], SweepSte
     }
 
     // whole rows and pencils with two cells a thread: x rows of up to 1024 cells, short pencils, and pencils of
-    // up to 512 cells that TMA's rules exclude (odd nx; HLL y/z of 121 x 90 x 75: 0.065 / 0.065 ms in the tile
+    // up to 512 cells (FP32 flux 256) that TMA's rules exclude (odd nx; HLL y/z of 121 x 90 x 75: 0.065 / 0.065 ms in the tile
     // kernel, 0.049 / 0.043 here)
     {
         int rc;

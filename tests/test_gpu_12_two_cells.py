@@ -69,7 +69,8 @@ def test_arrays_off_the_16_byte_boundary(cuda, ib, po, direction, shape):
     _check(*_sweep(ib, po, shape, 2, direction, "strict", shift=1), "strict")
 
 
-@pytest.mark.parametrize("direction,shape", [(1, (75, 6, 5)), (1, (256, 6, 5)), (1, (700, 3, 4)), (2, (7, 90, 3)), (3, (7, 3, 201))])
+@pytest.mark.parametrize("direction,shape", [(1, (75, 6, 5)), (1, (256, 6, 5)), (1, (700, 3, 4)), (2, (7, 90, 3)), (3, (7, 3, 201)),
+                                             (2, (7, 257, 3)), (2, (8, 403, 2)), (3, (5, 3, 512))])
 def test_fp32_flux(cuda, ib, po, direction, shape):
     out, ref, n = _sweep(ib, po, shape, 2, direction, "product", precision="fp32flux")
     ok, info = product_close(out, ref, n, l1=1e-5, scale=1e-4)  # the form's stated bound
