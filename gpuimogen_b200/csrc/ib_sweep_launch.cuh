@@ -462,11 +462,9 @@ int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], SweepStep lam
         if (rc != IB_ERROR_NOIMPLEMENT) return rc;
         return launch_tile_dw<METHOD, SLOPE, double, 1, 1, CYL_RADIAL>(q, slab, grid, lambda, c, st, 248, cs.pencil);
     case CYL_THETA_DIV:
-        // 128- and 256-cell pencils get the length at compile time (fewer registers for indexing, no spills)
+        // 256-cell pencils get the length at compile time (fewer registers for indexing, no spills)
         if (fast && pair && grid[1] == 256)
             rc = launch_pair<METHOD, SLOPE, double, 2, 256, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
-        else if (fast && pair && grid[1] == 128)
-            rc = launch_pair<METHOD, SLOPE, double, 2, 128, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         else if (fast && pair)
             rc = launch_pair<METHOD, SLOPE, double, 2, 0, 2, CYL_THETA_DIV>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         if (fast && rc == IB_ERROR_NOIMPLEMENT)
@@ -476,8 +474,6 @@ int launch_sweep_cyl_t(double *q, int64_t slab, const int grid[3], SweepStep lam
     case CYL_THETA_LAM:
         if (fast && pair && grid[1] == 256)
             rc = launch_pair<METHOD, SLOPE, double, 2, 256, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
-        else if (fast && pair && grid[1] == 128)
-            rc = launch_pair<METHOD, SLOPE, double, 2, 128, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         else if (fast && pair)
             rc = launch_pair<METHOD, SLOPE, double, 2, 0, 2, CYL_THETA_LAM>(q, slab, grid, lambda, c, st, 1, cs.pencil);
         if (fast && rc == IB_ERROR_NOIMPLEMENT)
