@@ -105,6 +105,14 @@ template <typename FT> __device__ __forceinline__ FT sub_product(FT s, FT a, FT 
 template <typename FT> __device__ __forceinline__ FT sum_products(FT a, FT b, FT c, FT d) { return fma(a, b, c * d); }
 template <typename FT> __device__ __forceinline__ FT diff_products(FT a, FT b, FT c, FT d) { return fma(a, b, -(c * d)); }
 #endif
+// A product that later arithmetic takes rounded (RN): the compiler may otherwise contract it into a sum where both
+// stand in one thread, and not where the product comes from another thread.  Kernels whose results are not to
+// depend on which cell a thread holds ask for it.
+template <bool RN>
+__device__ __forceinline__ double product(double a, double b) { return RN ? __dmul_rn(a, b) : a * b; }
+template <bool RN>
+__device__ __forceinline__ float product(float a, float b) { return RN ? __fmul_rn(a, b) : a * b; }
+
 template <typename FT>
 __device__ __forceinline__ FT square_sum(FT a, FT b, FT c) { return add_product(add_product(a * a, b, b), c, c); }
 
@@ -257,7 +265,7 @@ __device__ __forceinline__ void einfeldt_iso(FT rhoL, FT vL, FT rhoR, FT vR, FT 
     FT Fa = OPS::root(rhoR * OPS::rcp(rhoL));
     FT Fb = OPS::rcp((FT)1.0 + Fa);
 #endif
-    FT Vroe = (vL + Fa * vR) * Fb;
+    FT Vroe = product<true>(vL + Fa * vR, Fb);  // rounded: its sums below could contract it
     cs = Vroe - cs;
     sl = vL - cs;
     sr = vR + cs;
@@ -273,14 +281,6 @@ struct V5 {
     FT a[5];
 };
 
-// A product that later arithmetic takes rounded (RN): the compiler may otherwise contract it into a sum where both
-// stand in one thread, and not where the product comes from another thread.  Kernels whose results are not to
-// depend on which cell a thread holds ask for it.
-template <bool RN>
-__device__ __forceinline__ double product(double a, double b) { return RN ? __dmul_rn(a, b) : a * b; }
-template <bool RN>
-__device__ __forceinline__ float product(float a, float b) { return RN ? __fmul_rn(a, b) : a * b; }
-
 // Conserved -> HLLC primitives (cudaFluidStep.cu:1200-1237).  u: [rho, E, p_n, p_t1, p_t2].
 template <typename FT, bool RN = false, typename OPS = GuardedOps>
 __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
@@ -290,7 +290,7 @@ __device__ __forceinline__ V5<FT> hllc_prims(FT A, FT B, FT C, FT D, FT E)
 #else
     FT F = OPS::rcp(A);
 #endif
-    B -= (FT).5 * square_sum(C, D, E) * F;
+    B = sub_product(B, (FT).5 * square_sum(C, D, E), F);
     C = product<RN>(C, F);
     D = product<RN>(D, F);
     E = product<RN>(E, F);
@@ -404,8 +404,10 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     const FT dn = vL - vR, d1 = l.a[3] - r.a[3], d2 = l.a[4] - r.a[4];
     FT sl, sr, irL, irR;
     einfeldt<OPS, FT>(c, rhoL, vL, PL, rhoR, vR, PR, square_sum(dn, d1, d2), sl, sr, irL, irR);
-    const FT A = rhoL * (sl - vL), B = rhoR * (sr - vR);
-    const FT sm = (sub_product(add_product(-PR, B, vR), A, vL) + PL) * OPS::rcp(B - A);  // Batten et al. eq. 34
+    const FT wL = sl - vL, wR = sr - vR;
+    const FT A = rhoL * wL, B = rhoR * wR;
+    // Batten et al. eq. 34; rounded, since sums below could contract it
+    const FT sm = product<true>(sub_product(add_product(-PR, B, vR), A, vL) + PL, OPS::rcp(diff_products(rhoR, wR, rhoL, wL)));
     const bool left = sm > 0;
     const FT rho = left ? rhoL : rhoR, P = left ? PL : PR, v = left ? vL : vR;
     const FT t1 = left ? l.a[3] : r.a[3], t2 = left ? l.a[4] : r.a[4];
@@ -413,7 +415,7 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     const FT h = c.govergm1 * P;
     V5<FT> f;
     if (left ? sl > 0 : ((!kPoison<OPS, FT> || sm <= 0) && !(sr > 0))) {  // the outer state: no wave crosses the face
-        const FT m = product<RN>(rho, v);
+        const FT m = product<true>(rho, v);
         f.a[0] = m;
         f.a[1] = product<RN>(v, add_product(h, ke, rho));
         f.a[2] = add_product(P, m, v);
@@ -422,11 +424,11 @@ __device__ __forceinline__ V5<FT> hllc_flux(const FluidConsts<FT> &c, const V5<F
     } else {
         const FT S = left ? sl : sr;
         const FT D = (left ? A : B) * OPS::rcp(S - sm);
-        const FT m = product<RN>(D, sm);
-        const FT q = S * (sm - v);
+        const FT m = product<true>(D, sm);
+        const FT dv = sm - v;
         f.a[0] = m;
-        f.a[1] = product<RN>(m, add_product(ke, h, left ? irL : irR) + q);
-        f.a[2] = add_product(P, D, add_product(q, sm, v));
+        f.a[1] = product<RN>(m, add_product(add_product(ke, h, left ? irL : irR), S, dv));
+        f.a[2] = add_product(P, D, sum_products(sm, v, S, dv));
         f.a[3] = product<RN>(m, t1);
         f.a[4] = product<RN>(m, t2);
     }
