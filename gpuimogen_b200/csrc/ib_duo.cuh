@@ -36,15 +36,27 @@ struct DuoGeo {
     double rpen;        // theta sweeps: the pencil's radius
 };
 
+// What of a thread's two cells is tested for operands that the short forms do not reach, in the last sweep: the
+// primitives of the first stage (in), those of the second (mid), the second stage's mass flux through the cell's
+// right face (face).  A CTA of whole pencils tests the last two of each of its cells.  One that works on part of a
+// pencil tests `face` at the faces of the cells that it returns, `mid` where the second stage's input is theirs to use,
+// and `in` of every cell it loaded: a limiter can drop the NaN of a cell beyond.
+struct DuoTest {
+    bool in_a, in_b, mid_a, mid_b, face_a, face_b;
+};
+
 // NS sweeps of the cells (ua, ub) of this thread, in place.  planes: 15 TT values of FT; SS: 10 TT
 // doubles, where u1 + u0 of the SSPRK average waits through the second stage.  All threads of the CTA
-// call it.  OPS: FastOps (the caller tests the resulting densities, density_suspect) or IeeeOps.
+// call it.  OPS: FastOps (returns to all threads whether a test of theirs asks for the sweep to be done again, with
+// the inputs of old) or IeeeOps.
 template <int METHOD, int SLOPE, typename FT, int DIR, int TT, int NS, bool ODD, int GEO, bool RN = false,
           typename OPS = FastOps>
-__device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], bool act, const DuoPos &p, FT *planes,
-                                           double *SS, double lambda, const FluidConsts<FT> &c, const DuoGeo &g)
+__device__ __forceinline__ bool duo_sweeps(double (&ua)[5], double (&ub)[5], bool act, const DuoPos &p, FT *planes,
+                                           double *SS, double lambda, const FluidConsts<FT> &c, const DuoGeo &g,
+                                           const DuoTest &test = DuoTest{})
 {
     double va[5], vb[5];
+    bool suspect = false;
 #pragma unroll
     for (int s = 0; s < 2 * NS; s++) {
         const bool second = s & 1;
@@ -53,6 +65,11 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
         if (act) {
             wa = stage_prims<METHOD, DIR, FT, RN, OPS>(second ? va : ua, c);  // HLL floors its argument
             wb = stage_prims<METHOD, DIR, FT, RN, OPS>(second ? vb : ub, c);
+            if constexpr (kPoison<OPS, FT>) {
+                if (s == 2 * NS - 2) suspect = (test.in_a && cell_suspect(ua[0], wa.a[3])) || (test.in_b && cell_suspect(ub[0], wb.a[3]));
+                if (s == 2 * NS - 1)
+                    suspect = suspect || (test.mid_a && cell_suspect(va[0], wa.a[3])) || (test.mid_b && cell_suspect(vb[0], wb.a[3]));
+            }
 #pragma unroll
             for (int k = 0; k < 5; k++) {
                 P[k * TT + p.own] = wa.a[k];
@@ -109,7 +126,12 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
 #pragma unroll
             for (int k = 0; k < 5; k++) P[k * TT + p.own] = (ODD && p.ghost) ? fm.a[k] : fb.a[k];
         }
-        __syncthreads();
+        if (kPoison<OPS, FT> && s == 2 * NS - 1) {
+            if (act) suspect = suspect || (test.face_a && fm.a[0] != fm.a[0]) || (test.face_b && fb.a[0] != fb.a[0]);
+            suspect = __syncthreads_or(suspect);
+        } else {
+            __syncthreads();
+        }
         if (act) {
             const double lam = (GEO == CYL_THETA_LAM) ? lambda / g.rpen : lambda;
             // the isothermal HLL radial term's density: the new prediction (first stage), the stage's own
@@ -139,6 +161,7 @@ __device__ __forceinline__ void duo_sweeps(double (&ua)[5], double (&ub)[5], boo
             }
         }
     }
+    return suspect;
 }
 
 // The same with the IEEE operations, out of line: its registers are not the caller's.
@@ -188,7 +211,6 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT)) duo_row_kernel(Swe
     p.ghost = ODD && t == T - 1;
     double ua[5], ub[5];
     double *q = a.q + row * n + 2 * t;
-    bool suspect = false;
 #pragma unroll
     for (int k = 0; k < 5; k++) ua[k] = ub[k] = 1.0;
     if (act) {
@@ -209,12 +231,11 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT)) duo_row_kernel(Swe
     }
     DuoGeo g;
     if (GEO == CYL_RADIAL) { g.ra = a.crin + (2 * t) * a.cdr; g.rb = a.crin + (2 * t + 1) * a.cdr; g.dr = a.cdr; }
-    duo_sweeps<METHOD, SLOPE, FT, 1, TT, NS, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
-    if constexpr (kPoison<FastOps, FT>) {
-        if (act) suspect = density_suspect(ua[0]) || (density_suspect(ub[0]) && !p.ghost);
-        suspect = __syncthreads_or(suspect);
-    }
+    const bool whole = !(ODD && p.ghost);  // the last thread of an odd pencil owns one cell
+    const bool suspect = duo_sweeps<METHOD, SLOPE, FT, 1, TT, NS, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g,
+                                                                           DuoTest{false, false, true, whole, true, whole});
     if (suspect) {
+        __syncthreads();  // every thread is done with the planes
         if constexpr (kPoison<FastOps, FT>)
             ieee_pencils<METHOD, SLOPE, 1, GEO>(
                 IeeePencils{a.q, a.slab, a.nx, a.ny, a.nz, (int64_t)blockIdx.x * rp, rp, NS, lambda, CylPencil{a.crin, a.cdr, 0, 0}}, c, SS);
@@ -273,13 +294,11 @@ __global__ void __launch_bounds__(TT, duo_min_blocks<FT>(TT))
     }
     DuoGeo g;
     if (GEO != CYL_NONE) g.rpen = theta_radius(cyl, (int)(pencil % a.nx), (int)(pencil / a.nx));
-    bool suspect = false;
-    duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g);
-    if constexpr (kPoison<FastOps, FT>) {
-        if (act) suspect = density_suspect(ua[0]) || (density_suspect(ub[0]) && !p.ghost);
-        suspect = __syncthreads_or(suspect);
-    }
+    const bool whole = !(ODD && p.ghost);
+    const bool suspect = duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, ODD, GEO>(ua, ub, act, p, planes, SS, lambda, c, g,
+                                                                            DuoTest{false, false, true, whole, true, whole});
     if (suspect) {
+        __syncthreads();  // every thread is done with the planes
         if constexpr (kPoison<FastOps, FT>)
             ieee_pencils<METHOD, SLOPE, DIR, GEO>(
                 IeeePencils{a.q, a.slab, a.nx, a.ny, a.nz, (int64_t)blockIdx.x * COLS, COLS, 1, lambda, cyl}, c, SS);
@@ -386,26 +405,24 @@ __global__ void __launch_bounds__(R *W / 2, 512 / (R * W / 2))
         double ua[5], ub[5];
         fetch(2 * t, ua);
         fetch(2 * t + 1, ub);
+        __syncthreads();  // every thread is done with the planes
         const int g = c0 - 4 + 2 * t;
         const bool own_a = g >= c0 && g < cend, own_b = g + 1 >= c0 && g + 1 < cend;
-        bool suspect = false;
-        if constexpr (kPoison<FastOps, FT>) suspect = density_suspect(ua[0]) || density_suspect(ub[0]);
-        duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
-        if constexpr (kPoison<FastOps, FT>) {
-            suspect = suspect || (own_a && density_suspect(ua[0])) || (own_b && density_suspect(ub[0]));
-            if (__syncthreads_or(suspect)) {
-                double xa[5], xb[5];
-                fetch(2 * t, xa);
-                fetch(2 * t + 1, xb);
-                duo_sweep_ieee<METHOD, SLOPE, FT, DIR, TT, false>(xa, xb, p, planes, SS, lambda, c);
+        const int last = cend - c0 + 7;  // the last row with a cell
+        const auto among = [&](int r, int skip) { return r >= skip && r <= last - skip; };
+        const DuoTest test{among(2 * t, 0),     among(2 * t + 1, 0),     among(2 * t, 2),
+                           among(2 * t + 1, 2), own_a || g == c0 - 1,    own_b || g + 1 == c0 - 1};
+        if (duo_sweeps<METHOD, SLOPE, FT, DIR, TT, 1, false, CYL_NONE>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{}, test)) {
+            double xa[5], xb[5];
+            fetch(2 * t, xa);
+            fetch(2 * t + 1, xb);
+            __syncthreads();
+            duo_sweep_ieee<METHOD, SLOPE, FT, DIR, TT, false>(xa, xb, p, planes, SS, lambda, c);
 #pragma unroll
-                for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
-                __syncthreads();
-            }
-        } else {
+            for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
             __syncthreads();
         }
-        // every thread is done with tile buf and the planes: request the job after next into the tile
+        // every thread is done with tile buf: request the job after next into it
         if (leader) {
             const int64_t jn = j + 2 * step;
             if (jn < njobs_all) {

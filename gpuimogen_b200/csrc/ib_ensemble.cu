@@ -102,20 +102,23 @@ __device__ __forceinline__ void ens_store_ends(double *qb, int64_t S, int n, int
     __syncthreads();
 }
 
-// Products that leave a cell are rounded (RN), here and in the form with two rows a thread: otherwise the compiler
-// contracts them into the sums of the thread that formed them, and a cell's result would depend on the form.
+// Products that leave a cell are rounded (RN), here and in the form with two rows a thread, and this file is compiled
+// without contraction of the rest: otherwise the compiler takes some of them into the sums of the thread that
+// formed them, and a cell's result would depend on the form.
 //
 // Both stages of one chunk, row i of its tr rows a thread, which keeps that cell's state u in registers: on
 // return u is the output of rows 4 .. tr - 5.  Two shared-memory planes of FT swap roles between the stages.
 template <int METHOD, int SLOPE, typename FT, typename OPS>
-__device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double lambda, const FluidConsts<FT> &c, FT *SA, FT *SB,
+__device__ __forceinline__ bool ens_stages(double (&u)[5], int i, int tr, double lambda, const FluidConsts<FT> &c, FT *SA, FT *SB,
                                            int TR)
 {
     double u1[5];
     V5<FT> keep;
+    bool suspect = false;
     // ---- stage A: prims and fluxes in SA, left faces in SB ----
     if (i < tr) {
         V5<FT> w = stage_prims<METHOD, 1, FT, true, OPS>(u, c);  // HLL floors u
+        if constexpr (kPoison<OPS, FT>) suspect = cell_suspect(u[0], w.a[3]);
 #pragma unroll
         for (int k = 0; k < 5; k++) SA[k * TR + i] = w.a[k];
     }
@@ -150,6 +153,7 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
     // phase read SA only) ----
     if (i >= 2 && i <= tr - 3) {
         V5<FT> w = stage_prims<METHOD, 1, FT, true, OPS>(u1, c);  // HLL floors u1
+        if constexpr (kPoison<OPS, FT>) suspect = suspect || cell_suspect(u1[0], w.a[3]);
 #pragma unroll
         for (int k = 0; k < 5; k++) {
             SB[k * TR + i] = w.a[k];
@@ -177,12 +181,15 @@ __device__ __forceinline__ void ens_stages(double (&u)[5], int i, int tr, double
         keep = stage_flux<METHOD, FT, true, OPS>(c, keep, Lr);
 #pragma unroll
         for (int k = 0; k < 5; k++) SB[k * TR + i] = keep.a[k];
+        if constexpr (kPoison<OPS, FT>) suspect = suspect || keep.a[0] != keep.a[0];
     }
-    __syncthreads();
+    if constexpr (kPoison<OPS, FT>) suspect = __syncthreads_or(suspect);
+    else __syncthreads();
     if (i >= 4 && i <= tr - 5) {
 #pragma unroll
         for (int k = 0; k < 5; k++) u[k] = .5 * sub_product(u[k], lambda, (double)keep.a[k] - (double)SB[k * TR + i - 1]);
     }
+    return suspect;
 }
 
 // The same with the IEEE operations, out of line: its registers are not the caller's
@@ -197,8 +204,8 @@ __device__ __noinline__ void ens_stages_ieee(double (&u)[5], int i, int tr, doub
 // the tile sweep's in-place rules (each chunk loads its cells and 4 halo cells a side of the original
 // state; the last four outputs of a chunk wait in `pend` until the next chunk has been computed, the
 // first chunk's first four in `first` until the last chunk has read them through the periodic
-// wrap).  A chunk's inputs stay in memory until its outputs have been tested (density_suspect), so that it can be
-// computed again with the IEEE operations.  The arithmetic is the library's sweep arithmetic (stage_prims /
+// wrap).  A chunk's inputs stay in memory until its operands have been tested, so that it can be computed again with the
+// IEEE operations.  The arithmetic is the library's sweep arithmetic (stage_prims /
 // stage_faces / stage_flux), so the results are those of the tile sweep.
 template <int METHOD, int SLOPE, typename FT, int NT>
 __device__ __forceinline__ void ens_sweep(double *qb, int64_t S, int n, int nchunks, double lambda,
@@ -220,24 +227,17 @@ __device__ __forceinline__ void ens_sweep(double *qb, int64_t S, int n, int nchu
         };
         double out[5];
         fetch(out);
-        const bool mine = i >= 4 && i <= tr - 5;
-        bool suspect = false;
-        if constexpr (kPoison<FastOps, FT>) suspect = i < tr && density_suspect(out[0]);
-        ens_stages<METHOD, SLOPE, FT, FastOps>(out, i, tr, lambda, c, SA, SB, TR);
-        if constexpr (kPoison<FastOps, FT>) {
-            suspect = suspect || (mine && density_suspect(out[0]));
-            if (__syncthreads_or(suspect)) {
-                double x[5];
-                fetch(x);
-                ens_stages_ieee<METHOD, SLOPE, FT>(x, i, tr, lambda, c, SA, SB, TR);
-#pragma unroll
-                for (int k = 0; k < 5; k++) out[k] = x[k];
-                __syncthreads();
-            }
-        } else {
+        __syncthreads();  // every thread is done with the planes
+        if (ens_stages<METHOD, SLOPE, FT, FastOps>(out, i, tr, lambda, c, SA, SB, TR)) {
+            double x[5];
+            fetch(x);
             __syncthreads();
+            ens_stages_ieee<METHOD, SLOPE, FT>(x, i, tr, lambda, c, SA, SB, TR);
+#pragma unroll
+            for (int k = 0; k < 5; k++) out[k] = x[k];
         }
-        // every thread has read this chunk's inputs and is done with the planes
+        const bool mine = i >= 4 && i <= tr - 5;
+        // every thread has read this chunk's inputs
         ens_store_pending(qb, S, ch, cb, i, pend);
         if (mine) ens_store(qb, S, ch, cb, len, single, i - 4, out, pend, first);
     }
@@ -270,25 +270,22 @@ __device__ __forceinline__ void ens_sweep_two(double *qb, int64_t S, int n, int 
         double ua[5], ub[5];
         fetch(2 * t, ua);
         fetch(2 * t + 1, ub);
-        const bool own_a = 2 * t >= 4 && 2 * t <= tr - 5, own_b = 2 * t + 1 >= 4 && 2 * t + 1 <= tr - 5;
-        bool suspect = false;
-        if constexpr (kPoison<FastOps, FT>) suspect = density_suspect(ua[0]) || density_suspect(ub[0]);
-        duo_sweeps<METHOD, SLOPE, FT, 1, TT, 1, false, CYL_NONE, true>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{});
-        if constexpr (kPoison<FastOps, FT>) {
-            suspect = suspect || (own_a && density_suspect(ua[0])) || (own_b && density_suspect(ub[0]));
-            if (__syncthreads_or(suspect)) {
-                double xa[5], xb[5];
-                fetch(2 * t, xa);
-                fetch(2 * t + 1, xb);
-                duo_sweep_ieee<METHOD, SLOPE, FT, 1, TT, true>(xa, xb, p, planes, SS, lambda, c);
-#pragma unroll
-                for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
-                __syncthreads();
-            }
-        } else {
+        __syncthreads();  // every thread is done with the planes
+        const auto among = [&](int r, int first, int last) { return r >= first && r <= last; };
+        const bool own_a = among(2 * t, 4, tr - 5), own_b = among(2 * t + 1, 4, tr - 5);
+        const DuoTest test{among(2 * t, 0, tr - 1),     among(2 * t + 1, 0, tr - 1), among(2 * t, 2, tr - 3),
+                           among(2 * t + 1, 2, tr - 3), among(2 * t, 3, tr - 5),     among(2 * t + 1, 3, tr - 5)};
+        if (duo_sweeps<METHOD, SLOPE, FT, 1, TT, 1, false, CYL_NONE, true>(ua, ub, true, p, planes, SS, lambda, c, DuoGeo{}, test)) {
+            double xa[5], xb[5];
+            fetch(2 * t, xa);
+            fetch(2 * t + 1, xb);
             __syncthreads();
+            // in line: a call's saved registers cost every chunk more (1500 problems 2.85 against 2.78 ms)
+            duo_sweeps<METHOD, SLOPE, FT, 1, TT, 1, false, CYL_NONE, true, WideOps>(xa, xb, true, p, planes, SS, lambda, c, DuoGeo{});
+#pragma unroll
+            for (int k = 0; k < 5; k++) { ua[k] = xa[k]; ub[k] = xb[k]; }
         }
-        // every thread has read this chunk's inputs and is done with the planes
+        // every thread has read this chunk's inputs
         ens_store_pending(qb, S, ch, cb, t, pend);
         if (own_a) ens_store(qb, S, ch, cb, len, single, 2 * t - 4, ua, pend, first);
         if (own_b) ens_store(qb, S, ch, cb, len, single, 2 * t - 3, ub, pend, first);

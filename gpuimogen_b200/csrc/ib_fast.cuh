@@ -13,11 +13,11 @@
 // there.  A test and a branch at each of the nine operations of a flux was measured and not kept: its registers
 // spill in every kernel (256^3 HLLC y sweep 0.604 ms with the IEEE operation out of line, 0.561 without; one
 // branch per flux, 0.586 against 0.535).  The sweeps let the NaN run instead: a NaN in one operation of a face
-// reaches that face's flux and with it the densities beside it, so one test of each output density, once per
-// sweep, finds every pencil with such an operand, and that pencil is computed again with IeeeOps (ieee_pencils in
-// ib_sweep.cuh; in chunks, the same stages again).  Densities from 2^1000 on are sent there too, so that no
-// flushed reciprocal passes.  (256^3 x/y/z, HLLC 0.469/0.535/0.553 ms without the test, which got such operands
-// wrong, 0.465/0.541/0.552 with it; HLL 0.512/0.551/0.559 and 0.532/0.564/0.572.)
+// reaches that face's mass flux and with it the densities beside it, so one test per cell and sweep finds every
+// pencil with such an operand, and that pencil is computed again with IeeeOps (ieee_pencils in ib_sweep.cuh; in
+// chunks, the same stages again).  Densities from 2^1000 on are sent there too, so that no flushed reciprocal
+// passes.  (256^3 x/y/z, HLLC 0.469/0.535/0.553 ms without the test, which got such operands wrong, 0.465/0.541/
+// 0.552 with it; HLL 0.512/0.551/0.559 and 0.532/0.564/0.572.)
 #pragma once
 
 #include <cuda_runtime.h>
@@ -84,6 +84,24 @@ __device__ __forceinline__ double sqrt_full(double x)
     return y;
 }
 
+// 1/x and sqrt(x) for every x without a call (in Xin-Jin the registers around one spill): the operand is scaled into
+// the short form's range; zeros, infinities and NaN come out as the IEEE operation gives them
+__device__ __forceinline__ double rcp_any(double x)
+{
+    const double s = (fabs(x) < 1.0) ? 0x1p300 : 0x1p-300, t = x * s;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
+    const double e = fma(-t, y, 1.0);
+    const double r = fma(y, fma(e, e, e), y);
+    return ((fabs(x) > 0.0 && fabs(x) <= 1.7976931348623157e308) ? r : y) * s;
+}
+__device__ __forceinline__ double root_any(double x)
+{
+    const bool small = x < 1.0;
+    const double r = sqrt_fast(x * (small ? 0x1p400 : 0x1p-400)) * (small ? 0x1p-200 : 0x1p200);
+    return (x == 0.0 || x > 1.7976931348623157e308) ? x : r;
+}
+
 // a / x from ix = 1/x, both normal numbers: the quotient is corrected by its remainder (Markstein, IBM Journal
 // of Research and Development 34, 1990), whose error is that of the division; an infinite quotient has no
 // remainder
@@ -101,7 +119,8 @@ __device__ __forceinline__ float rcp_fast_pos(float x) { return 1.0f / x; }
 __device__ __forceinline__ float sqrt_fast(float x) { return sqrtf(x); }
 
 // The arithmetic of a sweep.  FastOps: the short forms, NaN where they do not reach; GuardedOps: the same, each
-// group of operations computed again with IeeeOps where the result is NaN; IeeeOps: the IEEE operations.
+// group of operations computed again with IeeeOps where the result is NaN; IeeeOps: the IEEE operations; WideOps: the
+// scaled forms, for code in line that has no registers to spare for a call.
 struct FastOps {
     template <typename FT> static __device__ __forceinline__ FT rcp(FT x) { return rcp_fast(x); }
     template <typename FT> static __device__ __forceinline__ FT root(FT x) { return sqrt_fast(x); }
@@ -115,6 +134,12 @@ struct IeeeOps {
     static __device__ __forceinline__ double root(double x) { return sqrt(x); }
     static __device__ __forceinline__ float root(float x) { return sqrtf(x); }
 };
+struct WideOps {
+    static __device__ __forceinline__ double rcp(double x) { return rcp_any(x); }
+    static __device__ __forceinline__ float rcp(float x) { return 1.0f / x; }
+    static __device__ __forceinline__ double root(double x) { return root_any(x); }
+    static __device__ __forceinline__ float root(float x) { return sqrtf(x); }
+};
 
 #ifdef IB_STRICT_ARITH
 template <typename OPS, typename FT> constexpr bool kPoison = false;
@@ -125,5 +150,7 @@ constexpr bool kPoison = std::is_same<OPS, FastOps>::value && std::is_same<FT, d
 #endif
 // a density that sends its pencil to IeeeOps: NaN, infinite, or so large that a reciprocal may have been flushed
 __device__ __forceinline__ bool density_suspect(double rho) { return !(fabs(rho) < 0x1p1000); }
+// the same of a cell's primitives: a velocity v is NaN where 1 / rho is
+__device__ __forceinline__ bool cell_suspect(double rho, double v) { return !(fma(v, 0.0, fabs(rho)) < 0x1p1000); }
 
 }  // namespace ib

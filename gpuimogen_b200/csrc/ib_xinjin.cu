@@ -62,7 +62,7 @@ __device__ __forceinline__ double freeze_cell(const double (&X)[5], double invrh
     return fabs(px) * invrho + sqrt(gamma * P * invrho);
 #else
     double v = fabs(px) * invrho + sqrt_fast(gamma * P * invrho);
-    if (!(v <= 1.7976931348623157e308)) v = fabs(px) * invrho + sqrt(gamma * P * invrho);
+    if (!(v <= 1.7976931348623157e308)) v = fabs(px) * invrho + root_any(gamma * P * invrho);
     return v;
 #endif
 }
@@ -80,8 +80,8 @@ __device__ __forceinline__ double freeze_first(const double (&X)[5], double &inv
     const double arg = gamma * ((X[1] - .5 * psq * invrho) * gm1) * invrho;
     double v = fabs(px) * invrho + sqrt_fast(arg);
     if (!(v <= 1.7976931348623157e308)) {
-        invrho = 1.0 / X[0];
-        v = fabs(px) * invrho + sqrt(gamma * ((X[1] - .5 * psq * invrho) * gm1) * invrho);
+        invrho = rcp_any(X[0]);
+        v = fabs(px) * invrho + root_any(gamma * ((X[1] - .5 * psq * invrho) * gm1) * invrho);
     }
     return v;
 }

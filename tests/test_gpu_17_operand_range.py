@@ -26,9 +26,10 @@ __global__ void k(const double *a, const double *x, double *o, long n)
     const long i = threadIdx.x + (long)blockIdx.x * blockDim.x;
     if (i >= n) return;
     const double v = x[i];
-    double r[10] = {ib::rcp_fast(v), ib::rcp_full(v), ib::rcp_fast_pos(v), 1.0 / v, ib::sqrt_fast(v), ib::sqrt_full(v),
-                    sqrt(v), ib::quotient_fast(a[i], v, ib::rcp_fast(v)), a[i] / v, ib::rcp_outside(v) ? 1.0 : 0.0};
-    for (int j = 0; j < 10; j++) o[j * n + i] = r[j];
+    double r[12] = {ib::rcp_fast(v), ib::rcp_full(v), ib::rcp_fast_pos(v), 1.0 / v, ib::sqrt_fast(v), ib::sqrt_full(v),
+                    sqrt(v), ib::quotient_fast(a[i], v, ib::rcp_fast(v)), a[i] / v, ib::rcp_outside(v) ? 1.0 : 0.0,
+                    ib::rcp_any(v), ib::root_any(v)};
+    for (int j = 0; j < 12; j++) o[j * n + i] = r[j];
 }
 extern "C" __attribute__((visibility("default"))) int run(const double *a, const double *x, double *o, long n)
 {
@@ -50,10 +51,11 @@ def functions(cuda, tmp_path_factory):
 
     def call(a, x):
         a, x = torch.tensor(a, device="cuda"), torch.tensor(x, device="cuda")
-        o = torch.empty((10, len(x)), dtype=torch.float64, device="cuda")
+        o = torch.empty((12, len(x)), dtype=torch.float64, device="cuda")
         torch.cuda.synchronize()
         assert run(*[ctypes.c_void_p(t.data_ptr()) for t in (a, x, o)], ctypes.c_long(len(x))) == 0
-        names = ["rcp", "rcp_full", "rcp_pos", "ref_rcp", "root", "root_full", "ref_root", "quotient", "ref_quotient", "outside"]
+        names = ["rcp", "rcp_full", "rcp_pos", "ref_rcp", "root", "root_full", "ref_root", "quotient", "ref_quotient", "outside",
+                 "rcp_any", "root_any"]
         return dict(zip(names, o.cpu().numpy()))
 
     return call
@@ -86,6 +88,9 @@ def test_reciprocals(functions):
     assert _ulps(o["rcp"][inside], o["ref_rcp"][inside]).max() <= 1
     assert _ulps(o["rcp_full"][inside], o["ref_rcp"][inside]).max() <= 1
     assert _same(o["rcp_full"][~inside], o["ref_rcp"][~inside]).all()
+    special = ~np.isfinite(o["ref_rcp"]) | (o["ref_rcp"] == 0)
+    assert _same(o["rcp_any"][special], o["ref_rcp"][special]).all()
+    assert _ulps(o["rcp_any"][~special], o["ref_rcp"][~special]).max() <= 1
     # outside: NaN, or 0 for numbers above 2^1022
     low = ~(np.abs(x) >= 2.0 ** -1022) | np.isinf(x)
     assert np.isnan(o["rcp"][low]).all() and (o["rcp"][~inside & ~low & (np.abs(x) > 2.0 ** 1022)] == 0).all()
@@ -103,6 +108,9 @@ def test_roots(functions):
     small = ~inside & (np.abs(x) < 2.0 ** -1022) & (x != 0)
     assert np.isnan(o["root"][~inside & ~small]).all() and np.isinf(o["root"][small]).all()
     assert _same(o["root_full"][~inside], o["ref_root"][~inside]).all()
+    special = ~np.isfinite(o["ref_root"]) | (x == 0)
+    assert _same(o["root_any"][special], o["ref_root"][special]).all()
+    assert _ulps(o["root_any"][~special], o["ref_root"][~special]).max() <= 1
     assert np.array_equal(np.signbit(o["root_full"][x == 0]), np.signbit(x[x == 0]))
 
 
@@ -159,6 +167,31 @@ def test_sweeps(cuda, ib, po, shape, direction, method, slope, kind):
     ib.cudaFluidStep(fl, geo, [dt, 1, 1.4, 5e-324, method, direction], ib.numerics(**kw))
     err = rel_l1(host(fl), ref, n)
     assert np.all(err <= 8e-13), err
+
+
+@pytest.mark.parametrize("shape,direction", [((1030, 4, 2), 1), ((8, 520, 2), 2), ((8, 3, 520), 3)])
+@pytest.mark.parametrize("method", [1, 2])
+def test_operands_beyond_a_chunk(cuda, ib, po, shape, direction, method):
+    """A cell without internal energy (its sound speed is zero: the short root does not reach it)
+    at each distance from a chunk's end, so that in turn it is only among the neighbouring chunk's halo cells."""
+    n = shape[0] * shape[1] * shape[2]
+    L = {1: 248, 2: 120, 3: 120}[direction]
+    stride = {1: 1, 2: shape[0], 3: shape[0] * shape[1]}[direction]
+    geo = ib.Geometry(shape, (0.05, 0.05, 0.05))
+    for d in range(-5, 6):
+        q = problems.random_smooth(shape, gamma=1.4, seed=7, amp=0.1)
+        i = (L + d) * stride + (1 if direction > 1 else 0)
+        rho = q[0, i]
+        q[:, i] = [rho, 0.0, 0.0, 0.0, 0.0]          # at rest, without pressure: P is exactly zero
+        ref = q.copy()
+        po.fluid_sweep(ref, shape, po.step_params(1e-3, geo.h, 1.4, rho_min=1e-5, method=method, slope="mc"), direction)
+        fl = to_fluid(q.copy(), shape)
+        ib.cudaFluidStep(fl, geo, [1e-3, 1, 1.4, 1e-5, method, direction], ib.numerics(slope="mc"))
+        out = host(fl)
+        fin = np.isfinite(ref[:, :n])
+        assert np.array_equal(np.isfinite(out[:, :n]), fin), d
+        out[:, :n][~fin] = ref[:, :n][~fin] = 0.0
+        assert np.all(rel_l1(out, ref, n) <= 1e-13), d
 
 
 @pytest.mark.parametrize("direction", [1, 2])
