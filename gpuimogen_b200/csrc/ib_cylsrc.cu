@@ -12,9 +12,10 @@
 //
 // One thread per cell: a grid-stride loop over the arrays in XYZ order, 5 loads and at most 3
 // stores of 8 bytes per cell.  The cell's 14 divisions bound it, not memory, so the product build
-// forms the reciprocals of r and rho once each and the quotients from them, to the division's error
-// (annulus 192 x 128 x 48, six iterations, 2.35 -> 2.16 ms; products with the reciprocals alone 2.11 ms, with
-// 1.4 times the error).
+// forms the reciprocals of r and rho once each and the quotients from them, to the division's error.
+// (Annulus 192 x 128 x 48, six iterations: this, the CFL kernel's short quotients and a theta form since
+// taken back gave 2.35 -> 2.16 ms together, and products with the reciprocals alone 2.11 ms with 1.4
+// times the error; this change was not timed by itself.)
 #include "ib_internal.cuh"
 
 namespace ib {

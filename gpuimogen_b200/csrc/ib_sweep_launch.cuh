@@ -264,9 +264,11 @@ int launch_sweep_t(int dir, double *q, int64_t slab, const int grid[3], SweepSte
         return (e && e[0] == 'x') ? 1 : 0;
     }();
     // Pencils of 16-63 cells, and z pencils of 64 in x-y planes above 1 MB, take the two-cell kernel: plain
-    // loads of 8 neighbouring pencils (64-byte rows) beat the TMA boxes of 2 or 4 there (HLLC FP64 z of 512 x
-    // 512 x 32 / 512 x 512 x 64 / 192 x 128 x 48: 0.442 / 0.703 / 0.065 -> 0.255 / 0.591 / 0.051 ms; even at 8
-    // cells, 0.106 both).  From 65 cells the boxes win (100-cell y of 1000 x 100 x 64: 0.248 against 0.282).
+    // loads of 8 neighbouring pencils (64-byte rows) beat the TMA boxes of 2 or 4 there, for every method.  us, boxes
+    // and two-cell kernel, HLLC FP64 / HLL / HLLC FP32 flux, 4.2 M cells unless the shape says more: y of 64 x n x ..,
+    // 16 cells 219, 160 / 231, 172 / 154, 110; 32 cells 224, 137 / 235, 148 / 154, 96; 48 cells 217, 177 / 229, 186 /
+    // 154, 102; 63 cells 206, 160 / 217, 167 / 147, 121; z of 512 x 512 x 64 691, 604 / 700, 632 / 472, 424.  (Even at 8
+    // cells, 0.106 ms both.)  From 65 cells the boxes win (100-cell y of 1000 x 100 x 64: 0.248 ms against 0.282).
     const bool short_pencil = dir > 1 && ((n >= 16 && n < 64) || (dir == 3 && n == 64 && (int64_t)nx * ny * 8 > (1 << 20)));
     if (use_pipe && n <= 512 && ((dir > 1 && !short_pencil) || (dir == 1 && pipe_x))) {
         int rc = IB_ERROR_NOIMPLEMENT;
